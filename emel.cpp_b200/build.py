@@ -30,6 +30,7 @@ SOURCES = {
     "gemm_q8_mma.cu": [],
     "gemm_q4k_mma.cu": [],
     "gemm_q6k_mma.cu": [],
+    "gemm_q6k_tc.cu": [],
     "linear.cu": [],
     "gemm_bf16.cu": [],
     "mixer_ops.cu": [],

@@ -1,0 +1,618 @@
+// Q6_K x Q8_K matrix product for many columns (prompt processing) on the Blackwell tensor cores: tcgen05.mma kind::f16,
+// weights as the A operand in TMEM, activations as the B operand in shared memory, f32 accumulators in TMEM that only
+// ever hold exact integers.
+//
+// What is computed is exactly the reference's per-super-block value (src/emel/kernel/x86_64/actions.hpp:1036-1077)
+//   (dx*d) * (float)isum,  isum = sum_g sc_g * dot16_g(q - 32, x)
+// added in ascending block order, so the result equals the mat-vec kernels' (and the x86 AVX2 route's) bit for bit.
+// A weight times its scale is a small integer, and f16 operands with f32 sums are exact as long as every partial sum
+// of a super-block stays below 2^24.  (q - 32) * sc needs 13 bits, f16 holds 11, so sc = 16 * hi + lo with
+// |hi|, |lo| <= 8 and two operands of |.| <= 256 each: |sum| <= 256 * 128 * 256 = 2^23 in any order of addition, and
+// (float)isum = fma(16, D_hi, D_lo), one rounding.
+// The expanded weights pass through neither the shared memory nor its port: a thread owns a weight row = a TMEM lane
+// and writes the operand with tcgen05.st.  Expanding two weights is one mask and one half2 fma: the masked 6-bit
+// quants are f16 subnormals q * 2^-24, times piece * 2^10 plus -32 * piece * 2^-14 is (q - 32) * piece * 2^-14 without a
+// rounding; the factor 2^14 returns in the fma that joins the pieces.  The order of a super-block's 256 weights along
+// the MMA's K is free (the sums are exact), so it follows from the masks; a pre-pass lays the activations out alike.
+//
+// CTA = 128 weight rows (TMEM lanes) x TN columns (32 or 64), one super-block of K per turn, 20 warps:
+//   warps 0-7   producers: two warps per TMEM lane quarter, one for each half (128 weights) of a super-block; what a
+//               half needs of the GGUF blocks of the warp's 32 rows comes by cp.async two turns ahead (ring of three,
+//               no barrier beyond the warp), a thread expands its row's half into TMEM
+//   warps 8-15  epilogue: two warps per TMEM lane quarter, TN/2 columns each, accumulators read in the m16n8 fragment
+//               layout, the float chain on packed f32x2 instructions
+//   warp  16    one elected thread: MMA issue; TMEM allocation
+//   warp  17    one thread: bulk copies of the activations (by half super-blocks) and of their scales
+// TMEM: two turns' accumulators (lo and hi, TN columns each), operands lo and hi of one turn, handed over in halves.
+// Registers are split by setmaxnreg: 640 threads x 96 at launch = 256 x 80 + 256 x 136 + 128 x 48.
+// Every mbarrier wait is bounded; on a timeout the CTA raises the status word, lets its copies land and frees its TMEM.
+//
+// What bounds it: the epilogue (two warps per scheduler) and the producers, each a chain of dependent steps of 2000 to
+// 2800 cycles a turn; the MMAs take 1040 (64 columns).  Measured, B200, kernel alone: 4096 x 11008 by 77 columns 62 us (the
+// mat-vec kernel that took every K before: 20.2 ms), 5 and 16 columns 96 us (1.28 and 4.05 ms).
+// Dispatch: K that gemm_q6k_mma.cu does not take (its copies need rows of a multiple of 16 bytes, K % 2048 == 0).  Where
+// both work they are about equal (14336 x 4096 by 2048 columns 944 + 10 against 1047 us, 4096 x 14336 by 333: 273 + 7
+// against 247, by 32: 124 + 3 against 99), so that kernel keeps its sizes.
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "common.cuh"
+#include "kernels.h"
+
+namespace emelb {
+namespace {
+
+constexpr int BM = 128;
+constexpr int kEpilogueWarp0 = 8, kEpilogueWarps = 8, kMmaWarp = 16, kLoaderWarp = 17;
+constexpr int kThreads = 20 * 32;
+constexpr int kProducerRegs = 80, kEpilogueRegs = 136, kOtherRegs = 48;
+static_assert(8 * 32 * kProducerRegs + 8 * 32 * kEpilogueRegs + 4 * 32 * kOtherRegs <= kThreads * 96, "register split");
+
+// activations in the workspace, and in shared memory: half super-blocks of 128 K, 8-column groups of two K-major
+// 128-byte swizzle atoms (8 columns x 64 values)
+constexpr int kAtomBytes = 1024;
+constexpr int kGroupBytes = 2 * kAtomBytes;             // one 8-column group of a half
+constexpr int kColPad = 128;                            // columns of the workspace past the last one a tile may touch
+
+constexpr int kMaxTN = 64, kHalves = 6;
+// a row's half of a raw block: 17 words of ql, 9 of qh, 3 of scales, the word of d; an odd number: rows on all 32 banks
+constexpr int kRawRow = 124, kRawSlots = 3, kRowMetaSlots = 4, kColMetaSlots = 3;
+constexpr int kHalfBytes = kMaxTN / 8 * kGroupBytes;
+
+// shared memory map
+constexpr int kOffRaw = kHalves * kHalfBytes;
+constexpr int kOffRowMeta = kOffRaw + kRawSlots * 2 * BM * kRawRow;      // [slot][row]: d
+constexpr int kOffColMeta = kOffRowMeta + kRowMetaSlots * BM * 4;        // [slot][column]: dx
+constexpr int kOffBars = kOffColMeta + kColMetaSlots * kMaxTN * 4;
+constexpr int kSmemBytes = kOffBars + 256 + 1024;   // barriers; slack for the base's alignment
+
+constexpr uint32_t kTmemA = 256;   // first operand column
+
+constexpr int kWaitSpins = 1 << 26;
+constexpr unsigned long long kWaitNs = 2000000000ull;  // 2 s
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+
+__device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
+// bounded wait; false when it gave up or another role already raised the abort flag
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  unsigned long long t0 = 0;
+  for (int spins = 0; spins < kWaitSpins; ++spins) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((spins & 63) == 63) {
+      if (*abort_flag) return false;
+      unsigned long long now;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > kWaitNs) break;
+    }
+  }
+  *abort_flag = 1;
+  return false;
+}
+
+// one thread of the warp; the compiler then knows that a single one issues what follows (an MMA loop under lane == 0
+// took 116-133 cycles an instruction, under elect.sync 84)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e != 0;
+}
+
+// B operand: K-major, 128-byte swizzle, 8-column groups kGroupBytes apart (descriptor version 1)
+__device__ __forceinline__ uint64_t operand_desc(uint32_t saddr) {
+  return (uint64_t)((saddr >> 4) & 0x3fffu) | (uint64_t)1 << 16 | (uint64_t)(kGroupBytes >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
+}
+
+// D {128 lanes, N} (+)= A (TMEM, f16) * B (shared memory, f16), f32 accumulators
+__device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+__device__ __forceinline__ void mma_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+// 8 columns of the warp's TMEM lanes
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// 16 TMEM lanes x 16 columns in the m16n8 accumulator-fragment layout: v[0..3] = columns 0-7, v[4..7] = columns
+// 8-15; within a block thread (g, t) gets (row g, col 2t), (row g, col 2t+1), (row g+8, col 2t), (row g+8, col 2t+1)
+__device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
+using f2 = unsigned long long;   // two floats
+__device__ __forceinline__ f2 pack2(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ f2 pack2u(uint32_t a, uint32_t b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint32_t h2_bits(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
+__device__ __forceinline__ __half2 bits_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
+// exact: masked weight bits (f16 subnormals) * s + c
+__device__ __forceinline__ uint32_t expand2(uint32_t bits, __half2 s, __half2 c) { return h2_bits(__hfma2(bits_h2(bits), s, c)); }
+
+struct GemmArgs {
+  const uint8_t* W;
+  int64_t row_bytes;
+  int M, K, N, TN;
+  const uint8_t* x;       // [K/128][npad/8] 8-column groups
+  const float* dx;        // [K/256][npad]
+  int npad;
+  float* y;
+  int64_t ldy;
+  int* status;
+};
+
+// pre-pass: the quantized activation planes of columns col0.. -> operand order.  K position 128 n + 16 w + 8 c + j of
+// a super-block holds element 128 n + 64 c + 32 (j / 4) + 4 w + {0, 2, 1, 3}[j % 4], which is what the producers'
+// masks leave side by side.  grid (K/256, ceil(N/64)), 256 threads; columns past N are zero.
+constexpr int kPreCols = 64, kPreRow = QK_K + 4;   // 65 words: column-wise reads fall on all banks
+
+__global__ void __launch_bounds__(256) tile_activations_f16_kernel(ActPlanes act, int col0, int N, int npad, uint8_t* x, float* dx) {
+  __shared__ __align__(16) uint8_t t8[kPreCols * kPreRow];
+  const int kb = blockIdx.x, c0 = blockIdx.y * kPreCols;
+  for (int q = threadIdx.x; q < kPreCols * 16; q += 256) {
+    const int col = q >> 4, piece = q & 15;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (c0 + col < N) v = *reinterpret_cast<const uint4*>(act.qs + (int64_t)(col0 + c0 + col) * act.col_stride_qs + kb * QK_K + 16 * piece);
+    uint32_t* o = reinterpret_cast<uint32_t*>(t8 + col * kPreRow + 16 * piece);
+    o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+  }
+  __syncthreads();
+  auto halves = [](uint32_t w, uint32_t& even, uint32_t& odd) {   // four int8 -> f16 {0, 2}, {1, 3}
+    const uint32_t u = w ^ 0x80808080u;
+    const __half2 bias = __float2half2_rn(-1152.0f);
+    even = h2_bits(__hadd2(bits_h2((u & 0x00ff00ffu) | 0x64006400u), bias));
+    odd = h2_bits(__hadd2(bits_h2(((u >> 8) & 0x00ff00ffu) | 0x64006400u), bias));
+  };
+  for (int q = threadIdx.x; q < kPreCols * 32; q += 256) {
+    const int col = q & (kPreCols - 1), ch = q >> 6;               // chunk ch of 8 K positions
+    const int n = ch >> 4, w = (ch >> 1) & 7, c = ch & 1;
+    const uint8_t* s = t8 + col * kPreRow + 128 * n + 64 * c + 4 * w;
+    uint4 o;
+    halves(*reinterpret_cast<const uint32_t*>(s), o.x, o.y);
+    halves(*reinterpret_cast<const uint32_t*>(s + 32), o.z, o.w);
+    uint8_t* dst = x + ((size_t)(2 * kb + n) * (npad >> 3) + ((c0 + col) >> 3)) * kGroupBytes + ((ch >> 3) & 1) * kAtomBytes +
+                   (col & 7) * 128 + (((ch ^ col) & 7) << 4);
+    *reinterpret_cast<uint4*>(dst) = o;
+  }
+  if (threadIdx.x < kPreCols) {
+    const int col = c0 + threadIdx.x;
+    dx[(size_t)kb * npad + col] = col < N ? act.d[(int64_t)(col0 + col) * act.col_stride_d + kb] : 0.0f;
+  }
+}
+
+__global__ void __launch_bounds__(kThreads, 1) gemm_q6k_tc_kernel(const GemmArgs p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* raw = smem + kOffRaw;
+  uint8_t* rowmeta = smem + kOffRowMeta;
+  uint8_t* colmeta = smem + kOffColMeta;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kOffBars);
+  uint64_t* a_full = bars;                   // [2 halves] producers -> MMA
+  uint64_t* a_free = a_full + 2;
+  uint64_t* x_full = a_free + 2;             // [kHalves] bulk copies -> MMA
+  uint64_t* x_free = x_full + kHalves;
+  uint64_t* m_full = x_free + kHalves;       // [3] bulk copies -> epilogue: the columns' scales of a super-block
+  uint64_t* m_free = m_full + kColMetaSlots;
+  uint64_t* d_full = m_free + kColMetaSlots;   // [2] MMA -> epilogue: the accumulators hold a finished super-block
+  uint64_t* d_free = d_full + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_free + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int TN = p.TN;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < 2; ++s) { mbar_init(a_full + s, 4); mbar_init(a_free + s, 1); }
+    for (int s = 0; s < kHalves; ++s) { mbar_init(x_full + s, 1); mbar_init(x_free + s, 1); }
+    for (int s = 0; s < kColMetaSlots; ++s) { mbar_init(m_full + s, 1); mbar_init(m_free + s, kEpilogueWarps); }
+    for (int s = 0; s < 2; ++s) { mbar_init(d_full + s, 1); mbar_init(d_free + s, kEpilogueWarps); }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == kMmaWarp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  const int mt = (p.M + BM - 1) / BM, nt = (p.N + TN - 1) / TN, ntiles = mt * nt, nkb = p.K / QK_K;
+  const int my_tiles = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  const int turns = my_tiles * nkb;   // super-blocks this CTA walks
+
+  if (warp < 8) {
+    // ---------------------------------------------------------------- producers
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kProducerRegs));
+    const int quarter = warp & 3, n = warp >> 2;   // TMEM lanes 32 * quarter .., half n of every super-block
+    const uint32_t a_lane = tmem_base + kTmemA + ((uint32_t)(32 * quarter) << 16) + 64u * n;
+    uint8_t* const raw0 = raw + (n * BM + 32 * quarter) * kRawRow;
+    constexpr int kSlotBytes = 2 * BM * kRawRow;
+    int itile = blockIdx.x, ikb = 0, islot = 0;    // the turn staged next
+    auto issue_raw = [&](int it) {
+      if (it < turns) {
+        const int r0 = (itile / nt) * BM + 32 * quarter;
+        uint8_t* dst = raw0 + islot * kSlotBytes;
+        // blocks start at any even byte: a half needs up to 30 of the 53 aligned words that cover its block, one a lane
+        const int word = lane < 17 ? 16 * n + lane : lane < 26 ? 32 + 8 * n + lane - 17 : lane < 29 ? 48 + 2 * n + lane - 26 : 52;
+        if (lane < 30) {
+#pragma unroll 4
+          for (int rr = 0; rr < 32; ++rr) {                      // rows past M repeat the last one; never stored
+            const uintptr_t src = reinterpret_cast<uintptr_t>(p.W) + (size_t)min(r0 + rr, p.M - 1) * p.row_bytes + (size_t)ikb * Q6_K_BYTES;
+            const uint32_t d = smem_u32(dst + rr * kRawRow) + 4 * lane;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"((src & ~uintptr_t(3)) + 4 * word) : "memory");
+          }
+        }
+        if (++ikb == nkb) { ikb = 0; itile += gridDim.x; }
+        if (++islot == kRawSlots) islot = 0;
+      }
+      cp_async_commit();
+    };
+    issue_raw(0);
+    issue_raw(1);
+    int tile = blockIdx.x, kb = 0, slot = 0;
+    bool live = true;
+    for (int it = 0; it < turns; ++it) {
+      issue_raw(it + 2);     // into the slot of turn it - 1
+      cp_async_wait<2>();
+      __syncwarp();
+      const uint8_t* blk = raw0 + slot * kSlotBytes + lane * kRawRow;
+      uint8_t* rm = rowmeta + ((it & (kRowMetaSlots - 1)) * BM + 32 * quarter + lane) * 4;
+      const int row = min((tile / nt) * BM + 32 * quarter + lane, p.M - 1);
+      const uint32_t sh = (uint32_t)((reinterpret_cast<uintptr_t>(p.W) + (size_t)row * p.row_bytes + (size_t)kb * Q6_K_BYTES) & 2) * 8;
+      const uint32_t* bw = reinterpret_cast<const uint32_t*>(blk);
+      auto word = [&](int i) { return __funnelshift_r(bw[i], bw[i + 1], sh); };   // i: 0 ql, 17 qh, 26 scales of the half
+      const uint32_t sw[2] = {word(26), word(27)};   // the half's eight scales
+      live = mbar_wait(a_free + n, (it & 1) ^ 1, abort_flag);
+      live = __all_sync(0xffffffffu, live);
+      if (!live) break;
+      fence_after();
+      // the slot's last readers were done before the MMAs of turn it - 1 could be issued
+      if (n == 0) *reinterpret_cast<uint32_t*>(rm) = sh ? bw[29] >> 16 : bw[29] & 0xffffu;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        // weights 16q .. 16q+15 of each 32: scale 2f + q of the half for form f; sc = 16 hi + lo, both in -8 .. 8
+        __half2 sl[4], cl[4], sh2[4], ch[4];
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+          const int b = 2 * f + q;
+          const int sc = (int)(int8_t)(sw[b >> 2] >> (8 * (b & 3)));
+          const int hi = (sc + 8) >> 4, lo = sc - 16 * hi;
+          const __half2 l2 = __half2half2(__int2half_rn(lo)), h2v = __half2half2(__int2half_rn(hi));
+          sl[f] = __hmul2(l2, __float2half2_rn(1024.0f));
+          cl[f] = __hmul2(l2, __float2half2_rn(-0.001953125f));   // -32 * 2^-14
+          sh2[f] = __hmul2(h2v, __float2half2_rn(1024.0f));
+          ch[f] = __hmul2(h2v, __float2half2_rn(-0.001953125f));
+        }
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          uint32_t ol[8], oh[8];
+          const int i = 4 * q + w;
+          const uint32_t qa = word(i), qb = word(8 + i), qh = word(17 + i);
+          const uint32_t v[4] = {(qa & 0x0f0f0f0fu) | ((qh << 4) & 0x30303030u), (qb & 0x0f0f0f0fu) | ((qh << 2) & 0x30303030u),
+                                 ((qa >> 4) & 0x0f0f0f0fu) | (qh & 0x30303030u), ((qb >> 4) & 0x0f0f0f0fu) | ((qh >> 2) & 0x30303030u)};
+#pragma unroll
+          for (int f = 0; f < 4; ++f) {
+            const uint32_t e = v[f] & 0x00ff00ffu, d = (v[f] >> 8) & 0x00ff00ffu;
+            ol[2 * f] = expand2(e, sl[f], cl[f]);
+            ol[2 * f + 1] = expand2(d, sl[f], cl[f]);
+            oh[2 * f] = expand2(e, sh2[f], ch[f]);
+            oh[2 * f + 1] = expand2(d, sh2[f], ch[f]);
+          }
+          tmem_st8(a_lane + 8u * i, ol);
+          tmem_st8(a_lane + 128u + 8u * i, oh);
+        }
+      }
+      tmem_wait_st();
+      fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(a_full + n);
+      if (++slot == kRawSlots) slot = 0;
+      if (++kb == nkb) { kb = 0; tile += gridDim.x; }
+    }
+    cp_async_wait<0>();
+  } else if (warp >= kMmaWarp) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
+    if (warp == kMmaWarp && elect_one()) {
+      // -------------------------------------------------------------- MMA issue (one thread)
+      // D = f32, A = B = f16, both K-major, M = 128 weight rows, N = TN columns
+      const uint32_t idesc = (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+      const uint64_t x0 = operand_desc(smem_u32(smem));
+      bool live = true, issued = false;
+      int last = 0, xs = 0, xphase = 0;
+      for (int it = 0; live && it < turns; ++it) {
+        const int buf = it & 1;
+        const uint32_t d = tmem_base + (uint32_t)(2 * TN * buf);
+        live = mbar_wait(d_free + buf, ((it >> 1) & 1) ^ 1, abort_flag);
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          if (!live) break;
+          live = mbar_wait(a_full + n, (uint32_t)it & 1u, abort_flag) && mbar_wait(x_full + xs, xphase, abort_flag);
+          if (!live) break;
+          fence_after();
+          const uint64_t x = x0 + (uint64_t)(xs * (kHalfBytes >> 4));
+          const uint32_t a_op = tmem_base + kTmemA + 64u * n;
+#pragma unroll
+          for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              mma_f16(d + (uint32_t)(r * TN), a_op + 128u * r + 8u * j, x + (uint64_t)(((j >> 2) * kAtomBytes + (j & 3) * 32) >> 4), idesc,
+                      (n | j) ? 1u : 0u);
+          mma_commit(a_free + n);
+          mma_commit(x_free + xs);
+          if (++xs == kHalves) { xs = 0; xphase ^= 1; }
+          issued = true;
+        }
+        if (issued) {
+          mma_commit(d_full + buf);
+          last = it;
+        }
+      }
+      if (!live && issued) {
+        // gave up: let the tensor core finish what was issued before the TMEM goes away (bounded)
+        for (int spins = 0; spins < (1 << 16) && !mbar_try_wait(d_full + (last & 1), (uint32_t)(last >> 1) & 1u); ++spins) {}
+      }
+    } else if (warp == kLoaderWarp && lane == 0) {
+      // -------------------------------------------------------------- activation loader (one thread)
+      bool live = true;
+      int xs = 0, xphase = 0, ms = 0, mphase = 0, sent_x = 0, sent_m = 0;
+      const uint32_t xbytes = (uint32_t)(TN / 8) * kGroupBytes, dbytes = (uint32_t)TN * 4;
+      int tile = blockIdx.x, kb = 0;
+      for (int it = 0; live && it < turns; ++it) {
+        const int c0 = (tile % nt) * TN;
+        for (int n = 0; live && n < 2; ++n) {
+          live = mbar_wait(x_free + xs, xphase ^ 1, abort_flag);
+          if (!live) break;
+          mbar_arrive_expect_tx(x_full + xs, xbytes);
+          bulk_g2s(smem + xs * kHalfBytes, p.x + ((size_t)(2 * kb + n) * (p.npad >> 3) + (c0 >> 3)) * kGroupBytes, xbytes, x_full + xs);
+          ++sent_x;
+          if (++xs == kHalves) { xs = 0; xphase ^= 1; }
+        }
+        live = live && mbar_wait(m_free + ms, mphase ^ 1, abort_flag);
+        if (live) {
+          mbar_arrive_expect_tx(m_full + ms, dbytes);
+          bulk_g2s(colmeta + ms * kMaxTN * 4, p.dx + (size_t)kb * p.npad + c0, dbytes, m_full + ms);
+          ++sent_m;
+          if (++ms == kColMetaSlots) { ms = 0; mphase ^= 1; }
+        }
+        if (++kb == nkb) { kb = 0; tile += gridDim.x; }
+      }
+      if (!live) {
+        // gave up: let the copies in flight land (bounded)
+        for (int i = max(0, sent_x - kHalves); i < sent_x; ++i)
+          for (int spins = 0; spins < (1 << 16) && !mbar_try_wait(x_full + i % kHalves, (i / kHalves) & 1); ++spins) {}
+        for (int i = max(0, sent_m - kColMetaSlots); i < sent_m; ++i)
+          for (int spins = 0; spins < (1 << 16) && !mbar_try_wait(m_full + i % kColMetaSlots, (i / kColMetaSlots) & 1); ++spins) {}
+      }
+    }
+  } else {
+    // ---------------------------------------------------------------- epilogue
+    // TMEM lanes are weight rows, TMEM columns the product's columns.  The warp owns 32 rows (its lane quarter) x TN/2
+    // columns; thread (g = lane/4, t = lane%4) holds rows g and g+8, columns 2t and 2t+1 of every 16 x 8 block.
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpilogueRegs));
+    const int quarter = warp & 3, col0 = ((warp - kEpilogueWarp0) >> 2) * (TN / 2), ncp = TN / 32;   // 16-column pieces
+    constexpr int kPieces = kMaxTN / 32;
+    const int g = lane >> 2, t = lane & 3;
+    int ms = 0, mphase = 0, tile = blockIdx.x, kb = 0;
+    f2 acc[kPieces][2][2][2];   // [piece][16-row half][8-column block][row g, g + 8]: columns 2t, 2t+1
+    const f2 up14 = pack2(16384.0f, 16384.0f), up18 = pack2(262144.0f, 262144.0f);
+    // added with fma(v, 1, acc), the 1 from a run-time value: ptxas contracts a packed multiply that only feeds a
+    // packed add (seen with 12.9, in spite of .rn), and the reference rounds both
+    const float one1 = p.K > 0 ? 1.0f : 2.0f;
+    const f2 one = pack2(one1, one1);
+    for (int it = 0; it < turns; ++it) {
+      const int buf = it & 1;
+      if (kb == 0) {
+#pragma unroll
+        for (int i = 0; i < 8 * kPieces; ++i) acc[i >> 3][(i >> 2) & 1][(i >> 1) & 1][i & 1] = 0ull;
+      }
+      bool live = mbar_wait(m_full + ms, mphase, abort_flag) && mbar_wait(d_full + buf, (uint32_t)(it >> 1) & 1u, abort_flag);
+      live = __all_sync(0xffffffffu, live);
+      if (!live) break;
+      fence_after();
+      const float* dxs = reinterpret_cast<const float*>(colmeta) + ms * kMaxTN + col0 + 2 * t;
+      const uint8_t* rmeta = rowmeta + ((it & (kRowMetaSlots - 1)) * BM + 32 * quarter + g) * 4;
+      const uint32_t tbase = tmem_base + (uint32_t)(2 * TN * buf) + ((uint32_t)(32 * quarter) << 16) + (uint32_t)col0;
+      f2 dw[4];                 // rows g, g + 8, g + 16, g + 24
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const float d = h2f((uint16_t)*reinterpret_cast<const uint32_t*>(rmeta + 32 * r));
+        dw[r] = pack2(d, d);
+      }
+#pragma unroll
+      for (int cp = 0; cp < kPieces; ++cp) {
+        if (cp >= ncp) break;
+        uint32_t lo[2][8], hi[2][8];
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+          tmem_ld_16x256b_x2(tbase + ((uint32_t)(16 * hh) << 16) + 16u * cp, lo[hh]);
+          tmem_ld_16x256b_x2(tbase + ((uint32_t)(16 * hh) << 16) + (uint32_t)TN + 16u * cp, hi[hh]);
+        }
+        f2 dx[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const float2 dxv = *reinterpret_cast<const float2*>(dxs + 16 * cp + 8 * q);
+          dx[q] = pack2(dxv.x, dxv.y);
+        }
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+          if (hh == 0) tmem_wait_ld();
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+#pragma unroll
+            for (int rr = 0; rr < 2; ++rr) {
+              const f2 dl = pack2u(lo[hh][4 * q + 2 * rr], lo[hh][4 * q + 2 * rr + 1]);
+              f2& a = acc[cp][hh][q][rr];
+              const f2 d_all = mul2(dx[q], dw[2 * hh + rr]);
+              const f2 isum = fma2(pack2u(hi[hh][4 * q + 2 * rr], hi[hh][4 * q + 2 * rr + 1]), up18, mul2(dl, up14));
+              a = fma2(mul2(d_all, isum), one, a);
+            }
+          }
+        }
+      }
+      fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(d_free + buf);
+        mbar_arrive(m_free + ms);
+      }
+      if (++ms == kColMetaSlots) { ms = 0; mphase ^= 1; }
+      if (++kb == nkb) {
+        const int tm = tile / nt, c0 = (tile - tm * nt) * TN + col0 + 2 * t;
+        const bool pairs = ((p.ldy | (int64_t)(reinterpret_cast<uintptr_t>(p.y) >> 2)) & 1) == 0;   // 8-byte stores
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const int row = tm * BM + 32 * quarter + 8 * r + g;
+          if (row >= p.M) continue;
+          float* yr = p.y + (size_t)row * p.ldy + c0;
+#pragma unroll
+          for (int nb = 0; nb < 2 * kPieces; ++nb) {
+            if (nb >= 2 * ncp) break;
+            const float2 v = unpack2(acc[nb >> 1][r >> 1][nb & 1][r & 1]);
+            const int c = c0 + 8 * nb;
+            if (pairs && c + 1 < p.N) {
+              *reinterpret_cast<float2*>(yr + 8 * nb) = v;
+            } else {
+              if (c < p.N) yr[8 * nb] = v.x;
+              if (c + 1 < p.N) yr[8 * nb + 1] = v.y;
+            }
+          }
+        }
+        kb = 0;
+        tile += gridDim.x;
+      }
+    }
+  }
+
+  fence_before();
+  __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, 1);
+  if (warp == kMmaWarp) {
+    fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+  }
+}
+
+int padded_columns(int ncols) { return (ncols + 127) / 128 * 128 + kColPad; }
+
+// columns per tile: 64, or 32 where the 64-column tiles leave SMs idle (a turn of 32 columns takes as long as the
+// producers need, about 0.7 of a 64-column one)
+int tile_columns(int M, int ncols, int sm_count) {
+  const int mt = (M + BM - 1) / BM;
+  const int waves64 = (mt * ((ncols + 63) / 64) + sm_count - 1) / sm_count, waves32 = (mt * ((ncols + 31) / 32) + sm_count - 1) / sm_count;
+  return 10 * waves64 <= 7 * waves32 ? 64 : 32;
+}
+
+}  // namespace
+
+size_t gemm_q6k_tc_workspace_bytes(int K, int ncols) { return (size_t)padded_columns(ncols) * (size_t)(K / QK_K) * (2 * QK_K + 4); }
+
+bool gemm_q6k_tc_supported(int type, const GemvArgs& a, int ncols) {
+  if (type != T_Q6_K || ncols < kGemmQ6kTcMinCols || a.K % QK_K != 0 || !a.tc_ws) return false;
+  if (a.residual || a.W2 || a.W3 || a.pro_x || a.rope_cos || a.join_in || a.join_out) return false;
+  if (gemm_q6k_mma_supported(type, a, ncols)) return false;
+  return reinterpret_cast<uintptr_t>(a.W) % 2 == 0 && a.row_bytes % 2 == 0 && reinterpret_cast<uintptr_t>(a.act.qs) % 16 == 0 &&
+         a.act.col_stride_qs % 16 == 0 && gemm_q6k_tc_workspace_bytes(a.K, ncols) <= a.tc_ws_bytes;
+}
+
+// two launches: the activation pre-pass (into the tensor-core workspace) and the product
+cudaError_t launch_gemm_q6k_tc(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st) {
+  GemmArgs g{};
+  g.W = a.W;
+  g.row_bytes = a.row_bytes;
+  g.M = a.M;
+  g.K = a.K;
+  g.N = ncols;
+  g.npad = padded_columns(ncols);
+  float* dx = reinterpret_cast<float*>(a.tc_ws + (size_t)(a.K / QK_K) * g.npad * (2 * QK_K));
+  g.x = a.tc_ws;
+  g.dx = dx;
+  tile_activations_f16_kernel<<<dim3(a.K / QK_K, (ncols + kPreCols - 1) / kPreCols), 256, 0, st>>>(a.act, a.col0, ncols, g.npad, a.tc_ws, dx);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  // per host thread (one context, one lane per thread): no shared mutable state between lanes
+  static thread_local unsigned configured = 0;  // one bit per device
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!(configured & (1u << (dev & 31)))) {
+    e = cudaFuncSetAttribute(gemm_q6k_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    if (e != cudaSuccess) return e;
+    configured |= 1u << (dev & 31);
+  }
+  g.TN = tile_columns(a.M, ncols, sm_count);
+  g.y = a.y + a.col0;
+  g.ldy = a.ldy;
+  g.status = a.status;
+  const int tiles = ((a.M + BM - 1) / BM) * ((ncols + g.TN - 1) / g.TN);
+  gemm_q6k_tc_kernel<<<tiles < sm_count ? tiles : sm_count, kThreads, kSmemBytes, st>>>(g);
+  return cudaGetLastError();
+}
+
+}  // namespace emelb

@@ -1,0 +1,81 @@
+"""The tcgen05 kernels of K-quant products (csrc/gemm_tc.cu, gemm_q6k_tc.cu): bits equal to the oracle's, which adds block values in
+the reference's x86 order.  Q6_K sums exact integers in f32, so the cases that could break it are the largest
+sums, every row alignment of 210-byte blocks, and partial tiles."""
+import numpy as np
+import pytest
+
+import emel_cpp_b200 as eb
+from oracle import bindings as ob
+from tests import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def be():
+    b = eb.Backend(0)
+    yield b
+    b.close()
+
+
+def check(be, port, t, w, k, m, x, n):
+    got, want = np.full((m, n), np.nan, np.float32), np.zeros((m, n), np.float32)
+    assert be.mul_mat(eb.mul_mat_op(w, t, k, m, x, n, got)), be.last_error
+    assert be.sync()
+    assert port.mul_mat(ob.mul_mat_op(w, t, k, m, x, n, want), route="blocks")
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), float(np.abs(got - want).max())
+
+
+def extreme_blocks(t, m, k):
+    """Rows of the largest and smallest codes in turn: quants all low, all high, alternating; scales at both ends."""
+    n = m * k // 256
+    b = np.zeros((n, eb.BLOCK_BYTES[t]), np.uint8)
+    i = np.arange(n)
+    quant = np.array([0x00, 0xff, 0x0f, 0xf0], np.uint8)[i % 4]
+    if t == eb.Q4_K:
+        b[:, 1], b[:, 3] = 0x20, 0x21                                     # d, dmin
+        b[:, 4:16] = np.where(i % 3 == 2, 0x3f, 0xff).astype(np.uint8)[:, None]
+        b[:, 16:] = quant[:, None]
+    else:
+        b[:, :192] = quant[:, None]
+        b[:, 192:208] = np.array([0x80, 0x7f, 0xf8, 0x07], np.uint8)[(i // 4) % 4][:, None]
+        b[:, 209] = 0x20
+    return b.reshape(-1)
+
+
+@pytest.mark.parametrize("t", [eb.Q4_K, eb.Q6_K])
+def test_largest_sums(be, port, t):
+    k, m, n = 768, 136, 40
+    x = np.ones((k, n), np.float32)
+    x[:, 1::4] = -1.0
+    x[::2, 2::4] = -1.0
+    x[:, 3::4] = np.where(np.arange(k) % 64 < 32, 1.0, -1.0)[:, None]
+    x *= np.linspace(0.5, 2.0, n, dtype=np.float32)
+    check(be, port, t, extreme_blocks(t, m, k), k, m, x, n)
+
+
+@pytest.mark.parametrize("t", [eb.Q4_K, eb.Q6_K])
+@pytest.mark.parametrize("k,m,n", [
+    (256, 1, 32), (256, 129, 5), (1280, 127, 33), (1792, 260, 64), (3328, 128, 65), (2816, 300, 96), (768, 384, 129),
+    (256, 3000, 300), (1280, 1300, 517), (1280, 300, 8),
+])
+def test_partial_tiles(be, port, t, k, m, n):
+    check(be, port, t, synth.random_blocks(t, 3 * k + n, m, k), k, m, synth.activations_f32(k + n, k, n).reshape(k, n), n)
+
+
+@pytest.mark.parametrize("offset", [2, 6, 10, 14])
+def test_q6_k_rows_at_even_addresses(be, port, offset):
+    torch = pytest.importorskip("torch")
+    k, m, n = 1280, 140, 70
+    w = synth.random_blocks(eb.Q6_K, 5, m, k)
+    x = synth.activations_f32(6, k, n).reshape(k, n)
+    want = np.zeros((m, n), np.float32)
+    assert port.mul_mat(ob.mul_mat_op(w, eb.Q6_K, k, m, x, n, want), route="blocks")
+    room = torch.zeros(w.size + 64, dtype=torch.uint8, device="cuda")
+    dev_w = room[offset:offset + w.size]
+    dev_w.copy_(torch.from_numpy(w.reshape(-1)))
+    dev_x, dev_y = torch.from_numpy(x).cuda(), torch.zeros((m, n), device="cuda")
+    torch.cuda.synchronize()
+    assert be.mul_mat(eb.mul_mat_op(dev_w, eb.Q6_K, k, m, dev_x, n, dev_y)), be.last_error
+    assert be.sync()
+    assert np.array_equal(dev_y.cpu().numpy().view(np.uint32), want.view(np.uint32))
