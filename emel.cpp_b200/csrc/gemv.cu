@@ -183,6 +183,10 @@ template <int T>
 cudaError_t launch_type(GemvArgs a, int ncols, bool argmax, bool fast, int sm_count, cudaStream_t st, int* launches,
                         int* grid_out) {
   cudaError_t e = cudaSuccess;
+  if (!fast && !argmax && gemv_odd_supported(T, a)) {
+    ++*launches;
+    return launch_gemv_odd(T, a, ncols, sm_count, st);
+  }
   if (!fast) {
     int grid = (a.M + 3) / 4;
     if (grid > sm_count * 8) grid = sm_count * 8;

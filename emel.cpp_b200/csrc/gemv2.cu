@@ -454,6 +454,166 @@ gemv2_kernel(const GemvArgs p) {
   }
 }
 
+// ---------------------------------------------------------------- any K
+// Mat-vec for K that the kernels above do not take (K % 2048 != 0: rows end inside a chunk, and 210-, 34- and 18-byte
+// blocks put them at even addresses).  A warp takes two rows and 32 blocks of each per turn: the bytes come by 16-byte
+// cp.async from the aligned window around them (two or four turns in flight), lane i computes block i's value for each
+// of NC columns, and lane (row, column) adds the 32 values in ascending block order from shared memory: the float
+// chain of every other route.  What it replaces read the blocks byte by byte: Q4_K 4096 x 11008 by one column 203 us,
+// Q6_K 264 us, Q4_0 56 us, Q4_K by 16 columns 3.2 ms; here 14.1, 17.0, 16.0 and 136 us.  It is bound by the block arithmetic's latency at 8 to 12 warps per SM.
+constexpr int kOddRows = 2, kOddWarps = 4;
+template <int T> struct Odd {
+  static constexpr int kRowBytes = (32 * block_bytes(T) + 15) / 16 * 16 + 32;   // window of 32 blocks at any offset, and a word past it
+  static constexpr int kStages = is_k_type(T) ? 2 : 4;
+  static constexpr int kStageBytes = kOddRows * kRowBytes;
+};
+template <int T, int NC>
+__host__ __device__ constexpr int odd_warp_bytes() { return Odd<T>::kStages * Odd<T>::kStageBytes + (kOddRows * NC * 33 * 4 + 15) / 16 * 16; }
+
+// one 32-weight block at an even shared address against one column: (float)sumi * (h(dw) * h(dx))
+template <int T>
+__device__ __forceinline__ void odd_block32(const uint8_t* blk, uint32_t (&q)[8], float& dw) {
+  const uint32_t base = smem_u32(blk) & ~3u, sh = (smem_u32(blk) & 2u) * 8;
+  constexpr int kWords = T == T_Q8_0 ? 9 : 5;   // 34 or 18 bytes: d, then the quants
+  uint32_t w[kWords + 1];
+#pragma unroll
+  for (int i = 0; i <= kWords; ++i) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[i]) : "r"(base + 4 * i));
+  uint32_t u[kWords];
+#pragma unroll
+  for (int i = 0; i < kWords; ++i) u[i] = __funnelshift_r(w[i], w[i + 1], sh);
+  dw = h2f((uint16_t)(u[0] & 0xffffu));
+  if constexpr (T == T_Q8_0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = __funnelshift_r(u[i], i + 1 < kWords ? u[i + 1] : 0u, 16);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t v = __funnelshift_r(u[i], u[i + 1], 16);
+      // nibble - 8 as int8: (n ^ 8) sign-extended from four bits
+      const uint32_t lo = (v & 0x0f0f0f0fu) ^ 0x08080808u, hi = ((v >> 4) & 0x0f0f0f0fu) ^ 0x08080808u;
+      q[i] = lo | ((lo & 0x08080808u) * 0x1eu);
+      q[4 + i] = hi | ((hi & 0x08080808u) * 0x1eu);
+    }
+  }
+}
+
+template <int T, int NC>
+__global__ void __launch_bounds__(32 * kOddWarps) gemv_odd_kernel(const GemvArgs p, int ncols) {
+  using O = Odd<T>;
+  constexpr bool KQ = is_k_type(T);
+  constexpr int BB = block_bytes(T), BE = block_elems(T), S = O::kStages;
+  extern __shared__ __align__(128) uint8_t smem_odd[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint8_t* ring = smem_odd + (size_t)warp * odd_warp_bytes<T, NC>();
+  float* table = reinterpret_cast<float*>(ring + S * O::kStageBytes);
+  const int nblk = p.K / BE, rounds = (nblk + 31) / 32, pairs = (p.M + kOddRows - 1) / kOddRows;
+  const int first = blockIdx.x * kOddWarps + warp, step = gridDim.x * kOddWarps;
+  const int turns = first < pairs ? ((pairs - 1 - first) / step + 1) * rounds : 0;
+  const int c0 = blockIdx.y * NC, nc = min(NC, ncols - c0);
+
+  auto source = [&](int pair, int r, int round) {   // rows past M repeat the last one; never stored
+    return reinterpret_cast<uintptr_t>(p.W) + (size_t)min(pair * kOddRows + r, p.M - 1) * p.row_bytes + (size_t)round * 32 * BB;
+  };
+  int ipair = first, iround = 0;
+  auto issue = [&](int t) {
+    if (t < turns) {
+      const int bytes = min(32, nblk - 32 * iround) * BB;
+#pragma unroll
+      for (int r = 0; r < kOddRows; ++r) {
+        const uintptr_t src = source(ipair, r, iround), base = src & ~uintptr_t(15);
+        const int n = (int)(src - base) + bytes;
+        uint8_t* dst = ring + (t % S) * O::kStageBytes + r * O::kRowBytes;
+        for (int o = 16 * lane; o < n; o += 512) cp_async16(dst + o, reinterpret_cast<const void*>(base + o));
+      }
+      if (++iround == rounds) { iround = 0; ipair += step; }
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int s = 0; s < S - 1; ++s) issue(s);
+
+  float acc = 0.0f;   // lane (row, column) = (lane / NC, lane % NC)
+  int pair = first, round = 0;
+  for (int t = 0; t < turns; ++t) {
+    issue(t + S - 1);
+    cp_async_wait<S - 1>();
+    __syncwarp();
+    const int blk = 32 * round + lane, cnt = min(32, nblk - 32 * round);
+    const uint8_t* at[kOddRows];
+#pragma unroll
+    for (int r = 0; r < kOddRows; ++r)
+      at[r] = ring + (t % S) * O::kStageBytes + r * O::kRowBytes + (source(pair, r, round) & 15) + lane * BB;
+    if (lane < cnt) {
+      if constexpr (KQ) {
+#pragma unroll 1
+        for (int j = 0; j < nc; ++j) {
+          Act256 x;
+          load_act<true, T == T_Q6_K>(x, p.act, p.col0 + c0 + j, 0, blk);
+#pragma unroll
+          for (int r = 0; r < kOddRows; ++r) {
+            float v;
+            if constexpr (T == T_Q4_K) v = q4_k_block_value(at[r], x);
+            else v = q6_k_block_value(at[r], x);
+            table[(r * NC + j) * 33 + lane] = v;
+          }
+        }
+      } else {
+        uint32_t q[kOddRows][8];
+        float dw[kOddRows];
+#pragma unroll
+        for (int r = 0; r < kOddRows; ++r) odd_block32<T>(at[r], q[r], dw[r]);
+#pragma unroll
+        for (int j = 0; j < NC; ++j) {
+          if (j >= nc) break;
+          const int64_t col = p.col0 + c0 + j;
+          const int4* xq = reinterpret_cast<const int4*>(p.act.qs + col * p.act.col_stride_qs + (int64_t)blk * 32);
+          const int4 a = __ldg(xq), b = __ldg(xq + 1);
+          const int xv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+          const float dx = __ldg(p.act.d + col * p.act.col_stride_d + blk);
+#pragma unroll
+          for (int r = 0; r < kOddRows; ++r) {
+            int s = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s = __dp4a((int)q[r][i], xv[i], s);
+            table[(r * NC + j) * 33 + lane] = __fmul_rn((float)s, __fmul_rn(dw[r], dx));
+          }
+        }
+      }
+    }
+    __syncwarp();
+    if (lane < kOddRows * NC) {
+      if (round == 0) acc = 0.0f;
+      const float* v = table + lane * 33;
+      if (cnt == 32) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) acc = __fadd_rn(acc, v[i]);
+      } else {
+        for (int i = 0; i < cnt; ++i) acc = __fadd_rn(acc, v[i]);
+      }
+      const int row = pair * kOddRows + lane / NC, j = lane % NC;
+      if (round == rounds - 1 && row < p.M && j < nc) {
+        const size_t o = (size_t)row * p.ldy + p.col0 + c0 + j;
+        p.y[o] = p.residual ? __fadd_rn(p.residual[o], acc) : acc;
+      }
+    }
+    __syncwarp();   // table and stage are free
+    if (++round == rounds) { round = 0; pair += step; }
+  }
+  cp_async_wait<0>();
+}
+
+template <int T, int NC>
+cudaError_t launch_odd(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st) {
+  constexpr int kSmem = kOddWarps * odd_warp_bytes<T, NC>();
+  const cudaError_t e = cudaFuncSetAttribute(gemv_odd_kernel<T, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  if (e != cudaSuccess) return e;
+  const int per_sm = (220 * 1024) / (kSmem + 1024), groups = (ncols + NC - 1) / NC;
+  const int blocks = (a.M + kOddRows * kOddWarps - 1) / (kOddRows * kOddWarps);
+  const int fill = sm_count * (per_sm < 1 ? 1 : per_sm > 4 ? 4 : per_sm);
+  gemv_odd_kernel<T, NC><<<dim3(blocks < fill ? blocks : fill, groups), 32 * kOddWarps, kSmem, st>>>(a, ncols);
+  return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------- third generation (one column)
 // Profiling the kernel above showed a warp retiring one instruction every ~13
 // cycles with only 3 warps per scheduler resident (122 registers, 18 KB of stages
@@ -1043,6 +1203,23 @@ cudaError_t launch_gemv_stream2(int type, const GemvArgs& a, int ncols, bool arg
     case T_Q8_0: return launch_type2<T_Q8_0>(a, ncols, argmax, sm_count, st, launches, grid_out);
     case T_Q4_0: return launch_type2<T_Q4_0>(a, ncols, argmax, sm_count, st, launches, grid_out);
     default: return cudaErrorInvalidValue;
+  }
+}
+
+bool gemv_odd_supported(int type, const GemvArgs& a) {
+  if (a.W2 || a.W3 || a.pro_x || a.rope_cos || a.join_in || a.join_out) return false;
+  const uintptr_t w = reinterpret_cast<uintptr_t>(a.W);
+  if (type == T_Q4_K ? (w % 16 != 0 || a.row_bytes % 16 != 0) : (w % 2 != 0 || a.row_bytes % 2 != 0)) return false;
+  if (reinterpret_cast<uintptr_t>(a.act.qs) % 16 != 0 || a.act.col_stride_qs % 16 != 0) return false;
+  return !is_k_type(type) || (reinterpret_cast<uintptr_t>(a.act.bsums) % 16 == 0 && a.act.col_stride_bs % 8 == 0);
+}
+
+cudaError_t launch_gemv_odd(int type, const GemvArgs& a, int ncols, int sm_count, cudaStream_t st) {
+  switch (type) {
+    case T_Q4_K: return ncols == 1 ? launch_odd<T_Q4_K, 1>(a, ncols, sm_count, st) : launch_odd<T_Q4_K, 4>(a, ncols, sm_count, st);
+    case T_Q6_K: return ncols == 1 ? launch_odd<T_Q6_K, 1>(a, ncols, sm_count, st) : launch_odd<T_Q6_K, 4>(a, ncols, sm_count, st);
+    case T_Q8_0: return ncols == 1 ? launch_odd<T_Q8_0, 1>(a, ncols, sm_count, st) : launch_odd<T_Q8_0, 8>(a, ncols, sm_count, st);
+    default: return ncols == 1 ? launch_odd<T_Q4_0, 1>(a, ncols, sm_count, st) : launch_odd<T_Q4_0, 8>(a, ncols, sm_count, st);
   }
 }
 
