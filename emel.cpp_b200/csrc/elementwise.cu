@@ -504,17 +504,28 @@ __global__ void __launch_bounds__(256) argmax_columns_part_kernel(const float* _
   }
 }
 
-__global__ void argmax_columns_finish_kernel(const float* part_val, const int* part_idx, int parts, int B, int* out_idx) {
-  const int col = threadIdx.x;
-  if (col >= B) return;
+// one warp per column (one thread that walked the 256 candidates of its column took 41 us, a load's latency each)
+__global__ void __launch_bounds__(32) argmax_columns_finish_kernel(const float* part_val, const int* part_idx, int parts, int B, int* out_idx) {
+  const int col = blockIdx.x;
   float bv = 0.0f;
   int bi = -1;
-  for (int p = 0; p < parts; ++p) {
+  for (int p = threadIdx.x; p < parts; p += 32) {
     const float v = part_val[p * B + col];
     const int r = part_idx[p * B + col];
-    if (r >= 0 && argmax_better(v, r, bv, bi)) { bv = v; bi = r; }
+    if (r >= 0 && v == v && argmax_better(v, r, bv, bi)) { bv = v; bi = r; }
   }
-  out_idx[col] = bi < 0 ? 0 : bi;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+    if (oi >= 0 && argmax_better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
+  }
+  if (threadIdx.x == 0) {
+    // a NaN in front is a candidate that nothing replaces; a later one never becomes one
+    const float first = part_val[col];
+    const int first_row = part_idx[col];
+    out_idx[col] = first_row >= 0 && first != first ? first_row : bi < 0 ? 0 : bi;
+  }
 }
 
 __global__ void add_inplace_kernel(float* __restrict__ acc, const float* __restrict__ y, int64_t n) {
@@ -744,7 +755,7 @@ cudaError_t launch_argmax_columns(const float* x, int rows, int B, float* part_v
   if (B < 1 || B > 256 || rows < 1) return cudaErrorInvalidValue;
   const int parts = rows < kArgmaxColumnParts ? rows : kArgmaxColumnParts;
   argmax_columns_part_kernel<<<parts, 256, 0, st>>>(x, rows, B, part_val, part_idx);
-  argmax_columns_finish_kernel<<<1, 256, 0, st>>>(part_val, part_idx, parts, B, out_idx);
+  argmax_columns_finish_kernel<<<B, 32, 0, st>>>(part_val, part_idx, parts, B, out_idx);
   return cudaGetLastError();
 }
 
