@@ -200,7 +200,9 @@ cudaError_t launch_w(const GemvArgs& a, int ncols, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// Many columns: 64-column tiles, 128 rows (64 while the 128-row grid would leave SMs without a CTA pair), two stages.
+// Many columns: 64-column tiles of 128 rows and two stages (of 64 rows and three while there are fewer than 3/5 of the SMs
+// of them; above that the wide ones win although they leave SMs without a second CTA: 5632 x 2048 by 333 columns 74 ->
+// 56 us, 14336 x 4096 by 128 108 -> 88, 8192 x 3072 by 200 117 -> 74, 2048 x 5632 by 333 79.7 -> 78.7).
 // Few columns: 8 / 16 / 32 / 64-column tiles of 64 rows with a deeper ring.  (Spreading a tile's columns over two or
 // four warps per row group measured slower at 32 and 64 columns: 45.8 against 35.8 us and 62.0 against 56.2 us for
 // 14336 x 4096 -- the kernel is bound by instructions per MMA, not by warps in flight)
@@ -209,8 +211,11 @@ cudaError_t launch_t(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st
   if (ncols <= 8) return launch_w<T, 4, 1, 4>(a, ncols, st);
   if (ncols <= 16) return launch_w<T, 4, 2, 4>(a, ncols, st);
   if (ncols <= 32) return launch_w<T, 4, 4, 3>(a, ncols, st);
+  // grids that leave half of the SMs idle: 16-column tiles (256 x 2048 by 333 columns 20.5 -> 10.4 us, 2048 x 5632 by 100
+  // 49.7 -> 28.2, 4096 x 4096 by 64 38.9 -> 25.5; with more tiles the wide ones win: 2048 x 5632 by 333 79 against 100 us)
+  if (2 * (int64_t)((a.M + 63) / 64) * ((ncols + 63) / 64) <= sm_count) return launch_w<T, 4, 2, 4>(a, ncols, st);
   const int64_t big = (int64_t)((a.M + 127) / 128) * ((ncols + 63) / 64);
-  return big >= 2 * (int64_t)sm_count ? launch_w<T, 8, 8, 2>(a, ncols, st) : launch_w<T, 4, 8, 3>(a, ncols, st);
+  return 5 * big >= 3 * (int64_t)sm_count ? launch_w<T, 8, 8, 2>(a, ncols, st) : launch_w<T, 4, 8, 3>(a, ncols, st);
 }
 
 }  // namespace
