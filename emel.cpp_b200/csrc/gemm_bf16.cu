@@ -63,6 +63,14 @@ __device__ __forceinline__ void tma_load(void* dst, const TmaMap* map, int x, in
                "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
                : "memory");
 }
+// one thread of the warp, in a form that tells the compiler that a single one issues what follows (128-row tiles of
+// 2048 prompt rows: 39.8 us a launch with a lane test, 38.8 with elect.sync)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e != 0;
+}
+
 // K-major operand in 8-row x 128-byte swizzled atoms, 1024 bytes apart (descriptor version 1, swizzle mode 2)
 __device__ __forceinline__ uint64_t operand_desc(uint32_t saddr) {
   return (uint64_t)((saddr >> 4) & 0x3fffu) | (uint64_t)1 << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
@@ -179,7 +187,7 @@ __global__ void __launch_bounds__(kThreads) gemm_bf16_kernel(const __grid_consta
     if (*abort_flag)
       for (int i = issued > T::kStages ? issued - T::kStages : 0; i < issued; ++i)
         for (int spin = 0; spin < 1 << 16 && !mbar_try_wait(full + i % T::kStages, (i / T::kStages) & 1); ++spin) {}
-  } else if (warp == kMmaWarp && lane == 0) {
+  } else if (warp == kMmaWarp && elect_one()) {
     for (int i = 0; i < nk; ++i) {
       const int s = i % T::kStages;
       if (!mbar_wait(full + s, (i / T::kStages) & 1, abort_flag)) break;
