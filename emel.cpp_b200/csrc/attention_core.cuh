@@ -15,8 +15,6 @@
 namespace emelb {
 namespace fa {
 
-constexpr int kMinRange = 64;
-
 struct CtaSync {
   __device__ __forceinline__ void operator()() const { __syncthreads(); }
 };
@@ -65,9 +63,7 @@ __device__ __forceinline__ void unit_reduce(float (&v)[NREP], float* scratch /*[
 // One unit: scores for the range (8 lanes per token row, 128-bit loads), exact range
 // maximum, probabilities, then the V accumulation with 128-bit loads; f32 throughout.
 // s_p: NREP * LMAX floats, s_red: 4 * NREP floats of shared memory owned by the unit.
-// T = live token count; ranges are L = ceil(T / splits) tokens (at most LMAX), but no fewer than kMinRange: a unit scores
-// 16 U rows at a time and sums SLOTS U value rows whatever its length, so shorter ranges only make more units of the same
-// duration (batch step of 16 sequences of 120 to 600 tokens, 20 ranges a session: 6.36 -> 5.49 ms with this bound).
+// T = live token count; ranges are L = ceil(T / splits) tokens (at most LMAX).
 // U = token rows a thread loads ahead (register budget of the caller; the results do not depend on it).
 // QL2: read q past L1 (the whole-token kernel rewrites q within a launch).
 template <int D, int NREP, int LMAX, int U, bool QL2, class Sync>
@@ -83,7 +79,6 @@ __device__ __forceinline__ void split_unit(const FlashArgs& a, int split, int kh
   const int n_rep = a.heads / a.kv_heads;
   const int head0 = kh * n_rep + zgroup * NREP;
   int L = (T + a.splits - 1) / a.splits;
-  L = L < kMinRange ? kMinRange : L;   // later ranges are then empty
   L = L > LMAX ? LMAX : L;  // the host sizes `splits` so this never clips
   const int t0 = split * L;
   const int t1 = min(T, t0 + L);
