@@ -243,6 +243,146 @@ __device__ __forceinline__ void split_unit(const FlashArgs& a, int split, int kh
   }
 }
 
+// The same unit for a range of at most kWarpRange tokens, by one warp: the same sums in the same order (a lane's eight
+// dims, the eight lanes of a row; the probabilities over the lanes; value rows t, t + SLOTS, ... of a slot, then the
+// slots in turn), so the same bits.  split_unit scores 16 U rows and synchronises 128 threads whatever the length of
+// the range; in a batch step of short sequences that is nearly all it does.  s_p: NREP * kWarpRange floats of the warp's.
+constexpr int kWarpRange = 32;
+
+template <int D, int NREP>
+__device__ __forceinline__ void split_warp(const FlashArgs& a, int split, int kh, int zgroup, int T, int lane, float* s_p) {
+  constexpr int DPL = D / 8, TPR = D / 8, SLOTS = 128 / TPR, HW = 32 / TPR;   // HW value rows at a time
+  const int head0 = kh * (a.heads / a.kv_heads) + zgroup * NREP;
+  const int L = (T + a.splits - 1) / a.splits;
+  const int t0 = split * L, n = min(T, t0 + L) - t0;
+  float* ml = a.part_ml + ((size_t)head0 * a.splits + split) * 2;
+  if (n <= 0) {
+#pragma unroll
+    for (int r = 0; r < NREP; ++r) {
+      for (int d = lane; d < D; d += 32) a.part_acc[((size_t)(head0 + r) * a.splits + split) * D + d] = 0.0f;
+      if (lane < 2) ml[(size_t)r * a.splits * 2 + lane] = lane ? 0.0f : -INFINITY;
+    }
+    return;
+  }
+  {
+    const int l8 = lane & 7;
+    float q[NREP][DPL];
+#pragma unroll
+    for (int r = 0; r < NREP; ++r)
+#pragma unroll
+      for (int i = 0; i < DPL; i += 4) {
+        const float4 t = __ldg(reinterpret_cast<const float4*>(a.q + (size_t)(head0 + r) * D + l8 * DPL + i));
+        q[r][i] = __half2float(__float2half_rn(t.x));
+        q[r][i + 1] = __half2float(__float2half_rn(t.y));
+        q[r][i + 2] = __half2float(__float2half_rn(t.z));
+        q[r][i + 3] = __half2float(__float2half_rn(t.w));
+      }
+    const char* kbase = reinterpret_cast<const char*>(a.k) + (size_t)kh * a.k_nb2 + (size_t)l8 * DPL * 2;
+    for (int tb = 0; tb < n; tb += 16) {
+      uint4 kv[4][DPL / 8];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const uint4* kp = reinterpret_cast<const uint4*>(kbase + (size_t)(t0 + min(tb + 4 * u + (lane >> 3), n - 1)) * a.k_nb1);
+#pragma unroll
+        for (int c = 0; c < DPL / 8; ++c) kv[u][c] = __ldg(kp + c);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float s[NREP];
+#pragma unroll
+        for (int r = 0; r < NREP; ++r) s[r] = 0.0f;
+#pragma unroll
+        for (int c = 0; c < DPL / 8; ++c) {
+          float kf[8];
+          unpack8(kv[u][c], kf);
+#pragma unroll
+          for (int r = 0; r < NREP; ++r)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s[r] = fmaf(q[r][8 * c + i], kf[i], s[r]);
+        }
+        const int tt = tb + 4 * u + (lane >> 3);
+#pragma unroll
+        for (int r = 0; r < NREP; ++r) {
+          float v = s[r];
+          v += __shfl_xor_sync(0xffffffffu, v, 1);
+          v += __shfl_xor_sync(0xffffffffu, v, 2);
+          v += __shfl_xor_sync(0xffffffffu, v, 4);
+          v *= a.scale;
+          if (tt < n && l8 == 0) s_p[r * kWarpRange + tt] = v;
+        }
+      }
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < NREP; ++r) {
+    const float s = lane < n ? s_p[r * kWarpRange + lane] : -INFINITY;
+    float mx = s;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    float sum = 0.0f;
+    if (lane < n) {
+      const float pr = expf(s - mx);
+      s_p[r * kWarpRange + lane] = pr;
+      sum += pr;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum = sum + __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) {
+      ml[(size_t)r * a.splits * 2] = mx;
+      ml[(size_t)r * a.splits * 2 + 1] = sum;
+    }
+  }
+  __syncwarp();
+  const int c = lane % TPR, h = lane / TPR;
+  const char* vbase = reinterpret_cast<const char*>(a.v) + (size_t)kh * a.v_nb2 + (size_t)c * 16;
+  float rsum[NREP][8];
+#pragma unroll
+  for (int r = 0; r < NREP; ++r)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) rsum[r][i] = 0.0f;
+#pragma unroll
+  for (int k = 0; k < SLOTS / HW; ++k) {
+    float acc[NREP][8];
+#pragma unroll
+    for (int r = 0; r < NREP; ++r)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[r][i] = 0.0f;
+    uint4 vv[kWarpRange / SLOTS];
+#pragma unroll
+    for (int u = 0; u < kWarpRange / SLOTS; ++u)
+      vv[u] = __ldg(reinterpret_cast<const uint4*>(vbase + (size_t)(t0 + min(k * HW + h + SLOTS * u, n - 1)) * a.v_nb1));
+#pragma unroll
+    for (int u = 0; u < kWarpRange / SLOTS; ++u) {
+      const int tt = k * HW + h + SLOTS * u;
+      if (tt < n) {
+        float vf[8];
+        unpack8(vv[u], vf);
+#pragma unroll
+        for (int r = 0; r < NREP; ++r) {
+          const float pr = s_p[r * kWarpRange + tt];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[r][i] = fmaf(pr, vf[i], acc[r][i]);
+        }
+      }
+    }
+#pragma unroll
+    for (int w = 0; w < HW; ++w)
+#pragma unroll
+      for (int r = 0; r < NREP; ++r)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) rsum[r][i] += __shfl_sync(0xffffffffu, acc[r][i], w * TPR + c);
+  }
+  if (h == 0) {
+#pragma unroll
+    for (int r = 0; r < NREP; ++r) {
+      float4* o = reinterpret_cast<float4*>(a.part_acc + ((size_t)(head0 + r) * a.splits + split) * D + c * 8);
+      o[0] = make_float4(rsum[r][0], rsum[r][1], rsum[r][2], rsum[r][3]);
+      o[1] = make_float4(rsum[r][4], rsum[r][5], rsum[r][6], rsum[r][7]);
+    }
+  }
+}
+
 // merge of the ranges of one head: out = sum_s e^{m_s-M} acc_s / sum_s e^{m_s-M} l_s.
 // One warp turns the head's (max, sum) pairs into weights w[0..63] and 1/denominator ...
 constexpr int kMergeMaxSplits = 64;
