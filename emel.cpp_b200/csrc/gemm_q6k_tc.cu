@@ -30,9 +30,10 @@
 // What bounds it: the epilogue (two warps per scheduler) and the producers, each a chain of dependent steps of 2000 to
 // 2800 cycles a turn; the MMAs take 1040 (64 columns).  Measured, B200, kernel alone: 4096 x 11008 by 77 columns 62 us (the
 // mat-vec kernel that took every K before: 20.2 ms), 5 and 16 columns 96 us (1.28 and 4.05 ms).
-// Dispatch: K that gemm_q6k_mma.cu does not take (its copies need rows of a multiple of 16 bytes, K % 2048 == 0).  Where
-// both work they are about equal (14336 x 4096 by 2048 columns 944 + 10 against 1047 us, 4096 x 14336 by 333: 273 + 7
-// against 247, by 32: 124 + 3 against 99), so that kernel keeps its sizes.
+// Dispatch: K and rows that the streaming kernels and gemm_q6k_mma.cu do not take (their copies need rows of a multiple
+// of 16 bytes, K % 2048 == 0).  Where both work, many columns are about equal (14336 x 4096 by 2048 columns 944 + 10
+// against 1047 us, 4096 x 14336 by 333: 273 + 7 against 247) and few are faster there (4096 x 14336 by 32: 124 + 3
+// against 99; by 8 127 against the mat-vec kernels' 60, by 5 127 against 49), so those kernels keep their sizes.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -577,7 +578,7 @@ size_t gemm_q6k_tc_workspace_bytes(int K, int ncols) { return (size_t)padded_col
 bool gemm_q6k_tc_supported(int type, const GemvArgs& a, int ncols) {
   if (type != T_Q6_K || ncols < kGemmQ6kTcMinCols || a.K % QK_K != 0 || !a.tc_ws) return false;
   if (a.residual || a.W2 || a.W3 || a.pro_x || a.rope_cos || a.join_in || a.join_out) return false;
-  if (gemm_q6k_mma_supported(type, a, ncols)) return false;
+  if (gemv_fast_path_ok(type, a.W, a.row_bytes, a.K)) return false;   // whatever the column count: see above
   return reinterpret_cast<uintptr_t>(a.W) % 2 == 0 && a.row_bytes % 2 == 0 && reinterpret_cast<uintptr_t>(a.act.qs) % 16 == 0 &&
          a.act.col_stride_qs % 16 == 0 && gemm_q6k_tc_workspace_bytes(a.K, ncols) <= a.tc_ws_bytes;
 }

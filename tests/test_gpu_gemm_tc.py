@@ -1,6 +1,7 @@
-"""The tcgen05 kernels of K-quant products (csrc/gemm_tc.cu, gemm_q6k_tc.cu): bits equal to the oracle's, which adds block values in
-the reference's x86 order.  Q6_K sums exact integers in f32, so the cases that could break it are the largest
-sums, every row alignment of 210-byte blocks, and partial tiles."""
+"""The tcgen05 kernels of K-quant products (csrc/gemm_tc.cu, gemm_q6k_tc.cu) and the lines between them and their neighbours:
+bits equal to the oracle's, which adds block values in the reference's x86 order.  Q6_K sums exact integers in f32, so
+the cases that could break it are the largest sums, every row alignment of 210-byte blocks, and partial tiles.  Which
+kernel a call takes shows in the number of launches: every route has the same bits."""
 import numpy as np
 import pytest
 
@@ -79,3 +80,21 @@ def test_q6_k_rows_at_even_addresses(be, port, offset):
     assert be.mul_mat(eb.mul_mat_op(dev_w, eb.Q6_K, k, m, dev_x, n, dev_y)), be.last_error
     assert be.sync()
     assert np.array_equal(dev_y.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+def launches_of(be, call):
+    before = be.diagnostics()["kernel_launches"]
+    call()
+    return be.diagnostics()["kernel_launches"] - before
+
+
+@pytest.mark.parametrize("k,m", [(2048, 70), (4096, 150), (8192, 33), (8192, 8200), (14336, 65)])
+@pytest.mark.parametrize("n", [4, 5, 6, 7, 8, 9])
+def test_q6_k_few_columns_of_long_aligned_rows(be, port, k, m, n):
+    """K a multiple of 2048 never takes the tcgen05 kernel (quantizer, operand layout, product: three launches): behind the
+    quantizer one mma.sync launch, or mat-vec launches of eight, four, two and one columns."""
+    w = synth.random_blocks(eb.Q6_K, 3 * k + n, m, k)
+    x = synth.activations_f32(k + n, k, n).reshape(k, n)
+    count = launches_of(be, lambda: check(be, port, eb.Q6_K, w, k, m, x, n))
+    few_long_rows = k >= 8192 and m < k   # the activations of eight columns do not fit beside the mat-vec kernel's rings
+    assert count == 1 + {4: 1, 5: 2, 6: 2, 7: 3 if few_long_rows else 1, 8: 2 if few_long_rows else 1, 9: 1}[n]
