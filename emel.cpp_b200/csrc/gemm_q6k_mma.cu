@@ -222,7 +222,7 @@ bool gemm_q6k_mma_supported(int type, const GemvArgs& a, int ncols) {
   // with K >= 8192 (activations too large for one pass) two: here while a row is short or there are many rows.  us a call,
   // calls one behind the other, there and here: 7 columns of 14336 x 4096 61.7 / 43.4, of 32000 x 4096 100.8 / 73.9, of
   // 14336 x 8192 98.3 / 72.0, of 1024 x 4096 31.1 / 31.1; of 2048 x 8192 49.6 / 55.1, of 4096 x 14336 78.2 / 90.4.  8 of
-  // 14336 x 8192 90.5 / 72.  5, 6 and 8 of 4096 x 14336 51.6, 59.7 and 60.1 there, 90.4 here
+  // 14336 x 8192 91.1 / 70.7.  5, 6 and 8 of 4096 x 14336 51.6, 59.7 and 60.1 there, 90.4 here
   const bool passes = ncols == 7 || (ncols == 8 && a.K >= 8192);
   const bool few = ncols < kGemmMmaMinCols && !(passes && (a.K <= 4096 || a.M >= a.K));
   if (type != T_Q6_K || few) return false;

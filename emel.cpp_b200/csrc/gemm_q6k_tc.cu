@@ -29,7 +29,7 @@
 //
 // What bounds it: the epilogue (two warps per scheduler) and the producers, each a chain of dependent steps of 2000 to
 // 2800 cycles a turn; the MMAs take 1040 (64 columns).  Measured, B200, kernel alone: 4096 x 11008 by 77 columns 62 us (the
-// mat-vec kernel that took every K before: 20.2 ms), 5 and 16 columns 96 us (1.28 and 4.05 ms).
+// mat-vec kernel that took every K before: 20.2 ms), 12 to 32 columns 96 us.
 // Dispatch: K and rows that the streaming kernels and gemm_q6k_mma.cu do not take (their copies need rows of a multiple
 // of 16 bytes, K % 2048 == 0).  Where both work, many columns are about equal (14336 x 4096 by 2048 columns 944 + 10
 // against 1047 us, 4096 x 14336 by 333: 273 + 7 against 247) and few are faster there (4096 x 14336 by 32: 124 + 3
@@ -575,9 +575,17 @@ int tile_columns(int M, int ncols, int sm_count) {
 
 size_t gemm_q6k_tc_workspace_bytes(int K, int ncols) { return (size_t)padded_columns(ncols) * (size_t)(K / QK_K) * (2 * QK_K + 4); }
 
+// Against gemv_odd_kernel (one pass over the weights per four columns, CTAs of eight rows): its time is that of the passes,
+// this kernel's that of K (2.25 us a super-block however few rows and columns there are), so the line is in passes x
+// rows.  us a call, calls one behind the other, there and here.  8192 row passes: 4096 x 11008 by 8 columns 92.5 / 107.5,
+// 1024 x 11008 by 32 84.7 / 108.2, 4096 x 2816 by 8 37.7 / 38.9, 1024 x 2816 by 32 37.2 / 40.6.  12288: 4096 x 11008 by 12
+// 142 / 108, 4096 x 2816 by 12 55.6 / 39.1.  Far from it: 256 x 11008 by 16 21.9 / 106.5, 14336 x 11008 by 5 262 / 108
+constexpr int64_t kMinRowPasses = 9216;
+
 bool gemm_q6k_tc_supported(int type, const GemvArgs& a, int ncols) {
   if (type != T_Q6_K || ncols < kGemmQ6kTcMinCols || a.K % QK_K != 0 || !a.tc_ws) return false;
   if (a.residual || a.W2 || a.W3 || a.pro_x || a.rope_cos || a.join_in || a.join_out) return false;
+  if ((int64_t)((ncols + 3) / 4) * ((a.M + 7) / 8 * 8) < kMinRowPasses) return false;
   if (gemv_fast_path_ok(type, a.W, a.row_bytes, a.K)) return false;   // whatever the column count: see above
   return reinterpret_cast<uintptr_t>(a.W) % 2 == 0 && a.row_bytes % 2 == 0 && reinterpret_cast<uintptr_t>(a.act.qs) % 16 == 0 &&
          a.act.col_stride_qs % 16 == 0 && gemm_q6k_tc_workspace_bytes(a.K, ncols) <= a.tc_ws_bytes;

@@ -237,7 +237,7 @@ cudaError_t launch_step_advance(int* state, const int* best_idx, int* tokens_out
 // gemm_tc.cu — Q4_K x Q8_K for many columns on the tensor cores (tcgen05, TMEM accumulators);
 // same numbers as the mat-vec kernels.  a.col0/a.y/a.ldy address the output as for launch_gemv.
 constexpr int kGemmTcMinCols = 32;
-constexpr int kGemmQ6kTcMinCols = 5;   // Q6_K, K no multiple of 2048: 96 us for up to 32 columns of 4096 x 11008, gemv_odd_kernel 17 us for one and one weight pass per four
+constexpr int kGemmQ6kTcMinCols = 5;   // Q6_K rows that no streaming kernel takes: fewer columns run gemv_odd_kernel (and so do more of a small matrix: gemm_q6k_tc.cu)
 constexpr int kGemmMmaMinCols = 9;   // Q6_K: fewer columns run the CUDA-core mat-vec kernels (7 and 8: gemm_q6k_mma.cu)
 constexpr int kGemmQ4kMmaMinCols = 5; // Q4_K: 8 columns take 39 / 63 us through the mat-vec kernel, 23-28 / 35 us through the mma.sync one (4096x14336 / 14336x4096)
 constexpr int kGemmQ8MmaMinCols = 3; // Q8_0 / Q4_0: from three columns on the mma.sync kernel (21-24 us for up to 8 columns of 14336x4096) beats the mat-vec kernels (29 us at 4 columns)

@@ -44,9 +44,9 @@ def extreme_blocks(t, m, k):
     return b.reshape(-1)
 
 
-@pytest.mark.parametrize("t", [eb.Q4_K, eb.Q6_K])
-def test_largest_sums(be, port, t):
-    k, m, n = 768, 136, 40
+@pytest.mark.parametrize("t,m", [(eb.Q4_K, 136), (eb.Q6_K, 136), (eb.Q6_K, 1000)])
+def test_largest_sums(be, port, t, m):
+    k, n = 768, 40
     x = np.ones((k, n), np.float32)
     x[:, 1::4] = -1.0
     x[::2, 2::4] = -1.0
@@ -58,16 +58,17 @@ def test_largest_sums(be, port, t):
 @pytest.mark.parametrize("t", [eb.Q4_K, eb.Q6_K])
 @pytest.mark.parametrize("k,m,n", [
     (256, 1, 32), (256, 129, 5), (1280, 127, 33), (1792, 260, 64), (3328, 128, 65), (2816, 300, 96), (768, 384, 129),
-    (256, 3000, 300), (1280, 1300, 517), (1280, 300, 8),
+    (256, 3000, 300), (1280, 1300, 517), (1280, 300, 8), (1280, 4630, 5), (1792, 1100, 33), (2816, 400, 96),
 ])
 def test_partial_tiles(be, port, t, k, m, n):
     check(be, port, t, synth.random_blocks(t, 3 * k + n, m, k), k, m, synth.activations_f32(k + n, k, n).reshape(k, n), n)
 
 
 @pytest.mark.parametrize("offset", [2, 6, 10, 14])
-def test_q6_k_rows_at_even_addresses(be, port, offset):
+@pytest.mark.parametrize("m", [140, 525])
+def test_q6_k_rows_at_even_addresses(be, port, offset, m):
     torch = pytest.importorskip("torch")
-    k, m, n = 1280, 140, 70
+    k, n = 1280, 70
     w = synth.random_blocks(eb.Q6_K, 5, m, k)
     x = synth.activations_f32(6, k, n).reshape(k, n)
     want = np.zeros((m, n), np.float32)
@@ -98,3 +99,16 @@ def test_q6_k_few_columns_of_long_aligned_rows(be, port, k, m, n):
     count = launches_of(be, lambda: check(be, port, eb.Q6_K, w, k, m, x, n))
     few_long_rows = k >= 8192 and m < k   # the activations of eight columns do not fit beside the mat-vec kernel's rings
     assert count == 1 + {4: 1, 5: 2, 6: 2, 7: 3 if few_long_rows else 1, 8: 2 if few_long_rows else 1, 9: 1}[n]
+
+
+@pytest.mark.parametrize("m,n,tc", [
+    (4608, 8, True), (4600, 8, False), (4601, 5, True), (1024, 33, True), (1024, 32, False), (9300, 4, False), (8, 4609, True), (8, 4604, False),
+    (1, 4609, True),
+])
+@pytest.mark.parametrize("k", [256, 2304])
+def test_q6_k_line_to_the_mat_vec_kernel(be, port, m, n, tc, k):
+    """Rows that no streaming kernel takes: the tcgen05 kernel (operand layout, product) from 9216 passes of four columns times
+    rows on, one mat-vec launch below."""
+    w = synth.random_blocks(eb.Q6_K, 5 * m + n, m, k)
+    x = synth.activations_f32(m + n, k, n).reshape(k, n)
+    assert launches_of(be, lambda: check(be, port, eb.Q6_K, w, k, m, x, n)) == (3 if tc else 2)
