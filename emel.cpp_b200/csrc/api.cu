@@ -351,8 +351,9 @@ uint32_t emelb_create(int device, emelb_ctx** out) {
   ok = ok && cudaMalloc(&c->act_qs, c->act_capacity) == cudaSuccess;
   ok = ok && cudaMalloc(&c->act_d, c->act_capacity / 32 * sizeof(float)) == cudaSuccess;
   ok = ok && cudaMalloc(&c->act_bsums, c->act_capacity / 16 * sizeof(int16_t)) == cudaSuccess;
-  // 256 K of a column: 512 bytes of f16, 36 of block sums and scales; columns padded to 128, and 128 more
-  c->tc_ws_bytes = c->act_capacity / 256 * 548 + (64u << 20);
+  // Q4_K: tiles of 128 columns x 256 K, 32 KB of int8 + 2.5 KB of block sums and scales; columns padded to 128.  Q6_K (512 bytes
+  // of f16 and a scale for 256 K of a column) takes the columns in as many turns as that holds: one at the default size
+  c->tc_ws_bytes = c->act_capacity / 32768 * 35328 + (64u << 20);
   ok = ok && cudaMalloc(&c->tc_ws, c->tc_ws_bytes) == cudaSuccess;
   ok = ok && cudaMalloc(&c->gemv_sched, (2 * kSchedSlots + 2) * sizeof(int)) == cudaSuccess;
   ok = ok && cudaMemset(c->gemv_sched, 0, (2 * kSchedSlots + 2) * sizeof(int)) == cudaSuccess;

@@ -53,7 +53,7 @@ static_assert(8 * 32 * kProducerRegs + 8 * 32 * kEpilogueRegs + 4 * 32 * kOtherR
 // 128-byte swizzle atoms (8 columns x 64 values)
 constexpr int kAtomBytes = 1024;
 constexpr int kGroupBytes = 2 * kAtomBytes;             // one 8-column group of a half
-constexpr int kColPad = 128;                            // columns of the workspace past the last one a tile may touch
+constexpr int kColPad = 64;                             // the workspace's columns come in groups: whole tiles, whole pre-pass blocks
 
 constexpr int kMaxTN = 64, kHalves = 6;
 // a row's half of a raw block: 17 words of ql, 9 of qh, 3 of scales, the word of d; an odd number: rows on all 32 banks
@@ -211,7 +211,7 @@ struct GemmArgs {
 // pre-pass: the quantized activation planes of columns col0.. -> operand order.  K position 128 n + 16 w + 8 c + j of
 // a super-block holds element 128 n + 64 c + 32 (j / 4) + 4 w + {0, 2, 1, 3}[j % 4], which is what the producers'
 // masks leave side by side.  grid (K/256, ceil(N/64)), 256 threads; columns past N are zero.
-constexpr int kPreCols = 64, kPreRow = QK_K + 4;   // 65 words: column-wise reads fall on all banks
+constexpr int kPreCols = kColPad, kPreRow = QK_K + 4;   // 65 words: column-wise reads fall on all banks
 
 __global__ void __launch_bounds__(256) tile_activations_f16_kernel(ActPlanes act, int col0, int N, int npad, uint8_t* x, float* dx) {
   __shared__ __align__(16) uint8_t t8[kPreCols * kPreRow];
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q6k_tc_kernel(const GemmArgs
   }
 }
 
-int padded_columns(int ncols) { return (ncols + 127) / 128 * 128 + kColPad; }
+int padded_columns(int ncols) { return (ncols + kColPad - 1) / kColPad * kColPad; }
 
 // columns per tile: 64, or 32 where the 64-column tiles leave SMs idle (a turn of 32 columns takes as long as the
 // producers need, about 0.7 of a 64-column one)
@@ -588,40 +588,48 @@ bool gemm_q6k_tc_supported(int type, const GemvArgs& a, int ncols) {
   if ((int64_t)((ncols + 3) / 4) * ((a.M + 7) / 8 * 8) < kMinRowPasses) return false;
   if (gemv_fast_path_ok(type, a.W, a.row_bytes, a.K)) return false;   // whatever the column count: see above
   return reinterpret_cast<uintptr_t>(a.W) % 2 == 0 && a.row_bytes % 2 == 0 && reinterpret_cast<uintptr_t>(a.act.qs) % 16 == 0 &&
-         a.act.col_stride_qs % 16 == 0 && gemm_q6k_tc_workspace_bytes(a.K, ncols) <= a.tc_ws_bytes;
+         a.act.col_stride_qs % 16 == 0 && gemm_q6k_tc_workspace_bytes(a.K, kColPad) <= a.tc_ws_bytes;
 }
 
-// two launches: the activation pre-pass (into the tensor-core workspace) and the product
-cudaError_t launch_gemm_q6k_tc(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st) {
-  GemmArgs g{};
-  g.W = a.W;
-  g.row_bytes = a.row_bytes;
-  g.M = a.M;
-  g.K = a.K;
-  g.N = ncols;
-  g.npad = padded_columns(ncols);
-  float* dx = reinterpret_cast<float*>(a.tc_ws + (size_t)(a.K / QK_K) * g.npad * (2 * QK_K));
-  g.x = a.tc_ws;
-  g.dx = dx;
-  tile_activations_f16_kernel<<<dim3(a.K / QK_K, (ncols + kPreCols - 1) / kPreCols), 256, 0, st>>>(a.act, a.col0, ncols, g.npad, a.tc_ws, dx);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
+// two launches: the activation pre-pass (into the tensor-core workspace) and the product; the two again for columns whose
+// operand the workspace does not hold beside the others'
+cudaError_t launch_gemm_q6k_tc(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st, int* launches) {
   // per host thread (one context, one lane per thread): no shared mutable state between lanes
   static thread_local unsigned configured = 0;  // one bit per device
   int dev = 0;
   cudaGetDevice(&dev);
   if (!(configured & (1u << (dev & 31)))) {
-    e = cudaFuncSetAttribute(gemm_q6k_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_q6k_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (e != cudaSuccess) return e;
     configured |= 1u << (dev & 31);
   }
-  g.TN = tile_columns(a.M, ncols, sm_count);
-  g.y = a.y + a.col0;
+  GemmArgs g{};
+  g.W = a.W;
+  g.row_bytes = a.row_bytes;
+  g.M = a.M;
+  g.K = a.K;
+  g.x = a.tc_ws;
   g.ldy = a.ldy;
   g.status = a.status;
-  const int tiles = ((a.M + BM - 1) / BM) * ((ncols + g.TN - 1) / g.TN);
-  gemm_q6k_tc_kernel<<<tiles < sm_count ? tiles : sm_count, kThreads, kSmemBytes, st>>>(g);
-  return cudaGetLastError();
+  const size_t groups = a.tc_ws_bytes / gemm_q6k_tc_workspace_bytes(a.K, kColPad);
+  const int fit = (int)(groups < 65535 ? groups : 65535) * kColPad;   // at least one group: gemm_q6k_tc_supported
+  for (int c = 0; c < ncols; c += fit) {
+    g.N = ncols - c < fit ? ncols - c : fit;
+    g.npad = padded_columns(g.N);
+    g.TN = tile_columns(a.M, g.N, sm_count);
+    g.y = a.y + a.col0 + c;
+    float* dx = reinterpret_cast<float*>(a.tc_ws + (size_t)(a.K / QK_K) * g.npad * (2 * QK_K));
+    g.dx = dx;
+    tile_activations_f16_kernel<<<dim3(a.K / QK_K, (g.N + kPreCols - 1) / kPreCols), 256, 0, st>>>(a.act, a.col0 + c, g.N, g.npad, a.tc_ws, dx);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const int tiles = ((a.M + BM - 1) / BM) * ((g.N + g.TN - 1) / g.TN);
+    gemm_q6k_tc_kernel<<<tiles < sm_count ? tiles : sm_count, kThreads, kSmemBytes, st>>>(g);
+    *launches += 2;
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace emelb

@@ -235,10 +235,7 @@ cudaError_t launch_gemv(int type, const GemvArgs& a, int ncols, bool argmax, int
     return launch_gemm_q4k_mma(a, ncols, sm_count, st);
   }
   // several columns of Q6_K, K no multiple of 2048 or rows unaligned: two f16 operands per weight on tcgen05 (gemm_q6k_tc.cu)
-  if (!argmax && gemm_q6k_tc_supported(type, a, ncols)) {
-    *launches += 2;
-    return launch_gemm_q6k_tc(a, ncols, sm_count, st);
-  }
+  if (!argmax && gemm_q6k_tc_supported(type, a, ncols)) return launch_gemm_q6k_tc(a, ncols, sm_count, st, launches);
   // nine or more columns of Q6_K: mma.sync per 16-weight scale group (gemm_q6k_mma.cu)
   if (!argmax && gemm_q6k_mma_supported(type, a, ncols)) {
     ++*launches;

@@ -133,7 +133,7 @@ cudaError_t launch_gemm_q6k_mma(const GemvArgs& a, int ncols, int sm_count, cuda
 bool gemm_q4k_mma_supported(int type, const GemvArgs& a, int ncols);
 // gemm_q6k_tc.cu: several columns of Q6_K weights on tcgen05, K that gemm_q6k_mma.cu does not take; overwrites the tensor-core workspace
 bool gemm_q6k_tc_supported(int type, const GemvArgs& a, int ncols);
-cudaError_t launch_gemm_q6k_tc(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st);
+cudaError_t launch_gemm_q6k_tc(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st, int* launches);
 cudaError_t launch_gemm_q4k_mma(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st);
 
 // gemv2.cu

@@ -112,3 +112,43 @@ def test_q6_k_line_to_the_mat_vec_kernel(be, port, m, n, tc, k):
     w = synth.random_blocks(eb.Q6_K, 5 * m + n, m, k)
     x = synth.activations_f32(m + n, k, n).reshape(k, n)
     assert launches_of(be, lambda: check(be, port, eb.Q6_K, w, k, m, x, n)) == (3 if tc else 2)
+
+
+def device_bytes_of_a_context(monkeypatch, melems):
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("EMELB_ACT_MELEMS", str(melems))
+    free = torch.cuda.mem_get_info()[0]
+    b = eb.Backend(0)
+    held = free - torch.cuda.mem_get_info()[0]
+    b.close()
+    return held
+
+
+def test_a_context_holds_one_copy_of_the_activations_in_operand_order(be, monkeypatch):
+    """1.25 bytes an element for the quantized planes and 1.08 for the Q4_K operand; the f16 operand of Q6_K shares it."""
+    grown = device_bytes_of_a_context(monkeypatch, 320) - device_bytes_of_a_context(monkeypatch, 64)
+    assert grown < 2.4 * (256 << 20)
+
+
+def test_q6_k_columns_in_turns(port, monkeypatch):
+    """More columns than the workspace holds in f16: the operand is laid out, and the product made, once per turn."""
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("EMELB_ACT_MELEMS", "72")
+    b = eb.Backend(0)
+    try:
+        k, m = 256, 3
+        n = (72 << 20) // k - 5
+        w = synth.random_blocks(eb.Q6_K, 9, m, k)
+        x = synth.activations_f32(10, k, n).reshape(k, n)
+        want = np.zeros((m, n), np.float32)
+        assert port.mul_mat(ob.mul_mat_op(w, eb.Q6_K, k, m, x, n, want), route="blocks")
+        dev_w, dev_x, dev_y = torch.from_numpy(w.reshape(-1)).cuda(), torch.from_numpy(x).cuda(), torch.zeros((m, n), device="cuda")
+        torch.cuda.synchronize()
+
+        def call():
+            assert b.mul_mat(eb.mul_mat_op(dev_w, eb.Q6_K, k, m, dev_x, n, dev_y)), b.last_error
+        assert launches_of(b, call) == 5      # quantizer, and two turns
+        assert b.sync()
+        assert np.array_equal(dev_y.cpu().numpy().view(np.uint32), want.view(np.uint32))
+    finally:
+        b.close()
