@@ -39,23 +39,24 @@ __global__ void __launch_bounds__(128) flash_split_kernel(const FlashArgs a) {
   fa::split_unit<D, NREP, LMAX, 8, false>(a, blockIdx.x, blockIdx.y, blockIdx.z, T, threadIdx.x, s_p, s_red, fa::CtaSync{});
 }
 
-// a batch of sequences: short ones take four ranges per CTA, one a warp, with the same bits (step of 16 sequences of
-// 120 to 600 tokens, 8B shape: 46 -> 23 us a launch, 6.23 -> 5.61 ms).  A kernel of its own: inside the one above it cost
-// the single sequence 5 % by its registers
+// several sequences: short ones take four ranges per CTA, one a warp, with the same bits.  The body for long ranges stands
+// first, where it is as fast as in the kernel above (the order of the two bodies and the size of the second matter: see
+// split_warp).  us a launch at 8B shape, this kernel against the one above: 16 sequences of 300 tokens 30 / 72, of 1100
+// 35.6 / 80.4, of 4000 98.6 / 98.2; 2 of 1100 11.8 / 16.2, of 4000 18.2 / 18.2; 1 of 1100 11.6 / 8.1 -- one sequence keeps to the other
 template <int D, int NREP>
 __global__ void __launch_bounds__(128) flash_split_seqs_kernel(const FlashArgs a) {
   pdl_trigger();
   pdl_wait();
   __shared__ __align__(16) float s_p[NREP * LMAX];
   __shared__ float s_red[4 * NREP];
-  const int T = a.tokens_dev ? a.tokens_dev[a.kv_heads_per_seq > 0 ? blockIdx.y / a.kv_heads_per_seq : 0] : a.tokens;
-  if (T <= fa::kWarpRange * a.splits) {
+  const int T = a.tokens_dev[blockIdx.y / a.kv_heads_per_seq];
+  if (T > fa::kWarpRange * a.splits) {
+    fa::split_unit<D, NREP, LMAX, 8, false>(a, blockIdx.x, blockIdx.y, blockIdx.z, T, threadIdx.x, s_p, s_red, fa::CtaSync{});
+  } else {
     const int split = blockIdx.x + (threadIdx.x >> 5);
     if (blockIdx.x % 4 != 0 || split >= a.splits) return;
     fa::split_warp<D, NREP>(a, split, blockIdx.y, blockIdx.z, T, threadIdx.x & 31, s_p + (threadIdx.x >> 5) * NREP * fa::kWarpRange);
-    return;
   }
-  fa::split_unit<D, NREP, LMAX, 8, false>(a, blockIdx.x, blockIdx.y, blockIdx.z, T, threadIdx.x, s_p, s_red, fa::CtaSync{});
 }
 
 // merge the ranges (attention_core.cuh).  One CTA of 256 threads = 256 consecutive
@@ -266,16 +267,18 @@ __global__ void flash_ref_sequential_kernel(const FlashArgs a, const float* scor
   }
 }
 
+template <int D, int NREP>
+cudaError_t launch_split_rep(const FlashArgs& a, int n_rep, cudaStream_t st) {
+  const bool several = a.kv_heads_per_seq > 0 && a.kv_heads > a.kv_heads_per_seq;
+  EMELB_LAUNCH((several ? flash_split_seqs_kernel<D, NREP> : flash_split_kernel<D, NREP>), dim3(a.splits, a.kv_heads, n_rep / NREP), 128, 0, st, a);
+  return cudaGetLastError();
+}
+
 template <int D>
 cudaError_t launch_split(const FlashArgs& a, int n_rep, cudaStream_t st) {
-  if (n_rep % 4 == 0) {
-    EMELB_LAUNCH((a.kv_heads_per_seq > 0 ? flash_split_seqs_kernel<D, 4> : flash_split_kernel<D, 4>), dim3(a.splits, a.kv_heads, n_rep / 4), 128, 0, st, a);
-  } else if (n_rep % 2 == 0) {
-    EMELB_LAUNCH((a.kv_heads_per_seq > 0 ? flash_split_seqs_kernel<D, 2> : flash_split_kernel<D, 2>), dim3(a.splits, a.kv_heads, n_rep / 2), 128, 0, st, a);
-  } else {
-    EMELB_LAUNCH((a.kv_heads_per_seq > 0 ? flash_split_seqs_kernel<D, 1> : flash_split_kernel<D, 1>), dim3(a.splits, a.kv_heads, n_rep), 128, 0, st, a);
-  }
-  return cudaGetLastError();
+  if (n_rep % 4 == 0) return launch_split_rep<D, 4>(a, n_rep, st);
+  if (n_rep % 2 == 0) return launch_split_rep<D, 2>(a, n_rep, st);
+  return launch_split_rep<D, 1>(a, n_rep, st);
 }
 
 }  // namespace

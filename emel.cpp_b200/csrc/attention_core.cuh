@@ -247,6 +247,9 @@ __device__ __forceinline__ void split_unit(const FlashArgs& a, int split, int kh
 // dims, the eight lanes of a row; the probabilities over the lanes; value rows t, t + SLOTS, ... of a slot, then the
 // slots in turn), so the same bits.  split_unit scores 16 U rows and synchronises 128 threads whatever the length of
 // the range; in a batch step of short sequences that is nearly all it does.  s_p: NREP * kWarpRange floats of the warp's.
+// The loops over rounds stay loops, with the value rows requested a round ahead: unrolled, this body made whichever of
+// the two stood second in a kernel 4 to 5 us later (its instructions are fetched anew in every launch) and, at D = 64, took
+// registers from the other (123 for 96).
 constexpr int kWarpRange = 32;
 
 template <int D, int NREP>
@@ -264,6 +267,15 @@ __device__ __forceinline__ void split_warp(const FlashArgs& a, int split, int kh
     }
     return;
   }
+  const int c = lane % TPR, h = lane / TPR;
+  const char* vbase = reinterpret_cast<const char*>(a.v) + (size_t)kh * a.v_nb2 + (size_t)c * 16;
+  uint4 vv[kWarpRange / SLOTS], ahead[kWarpRange / SLOTS];
+  auto load_rows = [&](int k, uint4 (&to)[kWarpRange / SLOTS]) {
+#pragma unroll
+    for (int u = 0; u < kWarpRange / SLOTS; ++u)
+      to[u] = __ldg(reinterpret_cast<const uint4*>(vbase + (size_t)(t0 + min(k * HW + h + SLOTS * u, n - 1)) * a.v_nb1));
+  };
+  load_rows(0, vv);
   {
     const int l8 = lane & 7;
     float q[NREP][DPL];
@@ -278,6 +290,7 @@ __device__ __forceinline__ void split_warp(const FlashArgs& a, int split, int kh
         q[r][i + 3] = __half2float(__float2half_rn(t.w));
       }
     const char* kbase = reinterpret_cast<const char*>(a.k) + (size_t)kh * a.k_nb2 + (size_t)l8 * DPL * 2;
+#pragma unroll 1
     for (int tb = 0; tb < n; tb += 16) {
       uint4 kv[4][DPL / 8];
 #pragma unroll
@@ -334,24 +347,19 @@ __device__ __forceinline__ void split_warp(const FlashArgs& a, int split, int kh
     }
   }
   __syncwarp();
-  const int c = lane % TPR, h = lane / TPR;
-  const char* vbase = reinterpret_cast<const char*>(a.v) + (size_t)kh * a.v_nb2 + (size_t)c * 16;
   float rsum[NREP][8];
 #pragma unroll
   for (int r = 0; r < NREP; ++r)
 #pragma unroll
     for (int i = 0; i < 8; ++i) rsum[r][i] = 0.0f;
-#pragma unroll
+#pragma unroll 1
   for (int k = 0; k < SLOTS / HW; ++k) {
+    if (k + 1 < SLOTS / HW) load_rows(k + 1, ahead);
     float acc[NREP][8];
 #pragma unroll
     for (int r = 0; r < NREP; ++r)
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[r][i] = 0.0f;
-    uint4 vv[kWarpRange / SLOTS];
-#pragma unroll
-    for (int u = 0; u < kWarpRange / SLOTS; ++u)
-      vv[u] = __ldg(reinterpret_cast<const uint4*>(vbase + (size_t)(t0 + min(k * HW + h + SLOTS * u, n - 1)) * a.v_nb1));
 #pragma unroll
     for (int u = 0; u < kWarpRange / SLOTS; ++u) {
       const int tt = k * HW + h + SLOTS * u;
@@ -372,6 +380,8 @@ __device__ __forceinline__ void split_warp(const FlashArgs& a, int split, int kh
       for (int r = 0; r < NREP; ++r)
 #pragma unroll
         for (int i = 0; i < 8; ++i) rsum[r][i] += __shfl_sync(0xffffffffu, acc[r][i], w * TPR + c);
+#pragma unroll
+    for (int u = 0; u < kWarpRange / SLOTS; ++u) vv[u] = ahead[u];
   }
   if (h == 0) {
 #pragma unroll

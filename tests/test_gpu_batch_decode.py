@@ -113,3 +113,36 @@ def test_buffers_grow_with_the_sequence_count(be, port):
         assert np.array_equal(nine[:, :2], two)
     finally:
         sess.close()
+
+
+@pytest.mark.parametrize("dim,heads", [(64, 8), (64, 16), (64, 32), (64, 64), (128, 8), (128, 16), (128, 32)])
+def test_sequences_of_every_range_length(be, port, dim, heads):
+    """37 ranges per sequence: the batch kernel takes ranges of up to 32 tokens by a warp each and longer ones by a CTA each;
+    one batch mixes both, with ranges of one scoring round and two, full and partial ones, and empty ones."""
+    cfg = dict(n_layer=1, n_embd=256, n_head=heads, n_head_kv=8, head_dim=dim, n_ff=256, n_vocab=256, n_ctx=1280)
+    tokens = [3, 37, 592, 593, 1147, 1184, 1185, 1270]
+    sess, cpu = build_model(be, port, cfg, {"embd": eb.Q4_K, "output": eb.Q6_K, "default": eb.Q4_K}, seed=dim + heads)
+    cpu.close()
+    try:
+        assert sess.set_sequences(len(tokens)), sess.last_error
+        rng = synth.rng(heads)
+        first, pos = [], [t - 1 for t in tokens]
+        for j, t in enumerate(tokens):
+            prompt = rng.integers(0, cfg["n_vocab"], size=t).tolist()
+            assert sess.select_sequence(j)
+            assert sess.prefill(prompt[:-1], 0), sess.last_error
+            first.append(prompt[-1])
+        alone_logits, alone_ids = [], []
+        for j in range(len(tokens)):
+            assert sess.select_sequence(j)
+            alone_logits.append(sess.decode(first[j], pos[j], want_logits=True))
+            alone_ids.append(list(sess.generate(first[j], pos[j], 3)))
+        for n in (len(tokens), 2, 1):
+            _, logits = sess.decode_batch(first[:n], pos[:n], want_logits=True)
+            for j in range(n):
+                assert np.array_equal(logits[j].view(np.uint32), alone_logits[j].view(np.uint32)), (n, tokens[j])
+        got = sess.generate_batch(first, pos, 3)              # 1184 tokens grow past the line
+        for j in range(len(tokens)):
+            assert list(got[:, j]) == alone_ids[j], tokens[j]
+    finally:
+        sess.close()
