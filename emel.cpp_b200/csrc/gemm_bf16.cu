@@ -20,7 +20,6 @@ namespace {
 constexpr int kThreads = 192, kTmaWarp = 4, kMmaWarp = 5;
 constexpr int kBM = kGemmWeightBox, kBK = 64;
 constexpr int kWeightTile = kBM * kBK * 2;
-constexpr int kSms = 148;
 constexpr int kWaitSpins = 1 << 22;
 constexpr uint32_t kSuspendHintNs = 10000;
 constexpr unsigned long long kWaitNs = 2000000000ull;
@@ -63,8 +62,8 @@ __device__ __forceinline__ void tma_load(void* dst, const TmaMap* map, int x, in
                "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
                : "memory");
 }
-// one thread of the warp, in a form that tells the compiler that a single one issues what follows (128-row tiles of
-// 2048 prompt rows: 39.8 us a launch with a lane test, 38.8 with elect.sync)
+// one thread of the warp, in a form that tells the compiler that a single one issues what follows (2048 prompt
+// rows: 39.8 and 75.4 us a launch of 128- and 256-row tiles with a lane test, 38.7 and 73.8 with elect.sync)
 __device__ __forceinline__ bool elect_one() {
   uint32_t e;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
@@ -124,8 +123,9 @@ struct GemmParams {
 };
 
 // DEEP: as many stages as one CTA per SM holds, for grids that give an SM no second CTA.  A stage's round trip (free ->
-// copy -> MMA) is over a microsecond, so the stages in flight set the rate: a request of
-// 300 prompt tokens and 24 steps at 4096 / 14336 features, 29.5 -> 28.8 ms; of 200 tokens at 2048 / 8192, 12.99 -> 12.84 ms
+// copy -> MMA) is over a microsecond, so the stages in flight set the rate.  Mean of 20 launches a prompt of 300 tokens,
+// 4096 / 14336 features: 57.6 -> 40.8 us; the two-matrix products of 200 tokens at 2048 / 8192: 38.9 -> 29.9 us.  A whole request
+// of these with 24 decoded steps, 29.6 and 13.0 ms, gains 1 to 3 %, little more than its runs differ
 template <int BN, bool GLU, bool DEEP>
 struct Tile {
   static constexpr int kStageBytes = (GLU ? 2 : 1) * kWeightTile + BN * kBK * 2;
@@ -287,8 +287,8 @@ cudaError_t launch_tile_stages(const TmaMap& wmap, const TmaMap& xmap, const Gem
 int64_t tiles_of(const GemmParams& p, int bn) { return (int64_t)((p.M + kBM - 1) / kBM) * ((p.rows + bn - 1) / bn); }
 
 template <int BN, bool GLU>
-cudaError_t launch_tile(const TmaMap& wmap, const TmaMap& xmap, const GemmParams& p, cudaStream_t st) {
-  return tiles_of(p, BN) <= kSms ? launch_tile_stages<BN, GLU, true>(wmap, xmap, p, st) : launch_tile_stages<BN, GLU, false>(wmap, xmap, p, st);
+cudaError_t launch_tile(const TmaMap& wmap, const TmaMap& xmap, const GemmParams& p, int sm_count, cudaStream_t st) {
+  return tiles_of(p, BN) <= sm_count ? launch_tile_stages<BN, GLU, true>(wmap, xmap, p, st) : launch_tile_stages<BN, GLU, false>(wmap, xmap, p, st);
 }
 
 }  // namespace
@@ -314,22 +314,22 @@ bool encode_bf16_map(TmaMap* map, const __nv_bfloat16* base, int64_t rows, int64
 }
 
 cudaError_t launch_gemm_bf16(const LinearArgs& a, const TmaMap& wmap, const XMaps& x, float* y, __nv_bfloat16* yb, int64_t ldy, int* status,
-                             cudaStream_t st) {
+                             int sm_count, cudaStream_t st) {
   if (yb && (ldy % 8 != 0 || reinterpret_cast<uintptr_t>(yb) % 16 != 0)) return cudaErrorInvalidValue;
   const bool glu = is_glu(a.act);
   GemmParams p{glu ? a.w.M / 2 : a.w.M, a.w.K, a.rows, a.bias, a.act, a.act_split, y, yb, ldy, status,
                a.out_scale, a.softcap, a.tail, a.tail_y, a.tail_ld};
   const int R = a.rows;
   if (glu) {
-    if (R <= 16) return launch_tile<16, true>(wmap, x.narrow, p, st);
-    if (R <= 64 || tiles_of(p, 64) <= kSms) return launch_tile<64, true>(wmap, x.narrow, p, st);
-    return launch_tile<128, true>(wmap, x.wide, p, st);
+    if (R <= 16) return launch_tile<16, true>(wmap, x.narrow, p, sm_count, st);
+    if (R <= 64 || tiles_of(p, 64) <= sm_count) return launch_tile<64, true>(wmap, x.narrow, p, sm_count, st);
+    return launch_tile<128, true>(wmap, x.wide, p, sm_count, st);
   }
-  if (R <= 16) return launch_tile<16, false>(wmap, x.narrow, p, st);
-  if (R <= 64 || tiles_of(p, 64) <= kSms) return launch_tile<64, false>(wmap, x.narrow, p, st);   // narrower tiles while every one has an SM
+  if (R <= 16) return launch_tile<16, false>(wmap, x.narrow, p, sm_count, st);
+  if (R <= 64 || tiles_of(p, 64) <= sm_count) return launch_tile<64, false>(wmap, x.narrow, p, sm_count, st);   // narrower tiles while every one has an SM
   // 256-row tiles once there are more of them than SMs
   if (tiles_of(p, 256) >= 180) return launch_tile_stages<256, false, false>(wmap, x.wide, p, st);
-  return launch_tile<128, false>(wmap, x.wide, p, st);
+  return launch_tile<128, false>(wmap, x.wide, p, sm_count, st);
 }
 
 }  // namespace emelb

@@ -738,7 +738,7 @@ bool latent_prompt_supported(const LatentArgs& a, int rows) {
 }
 
 cudaError_t launch_latent_prompt(const LatentArgs& a, const TmaMap& upmap, const Rows& rows, int pos0, __nv_bfloat16* out, int64_t ldo, int* status,
-                                 cudaStream_t st, int* launches) {
+                                 int sm_count, cudaStream_t st, int* launches) {
   latent_store_kernel<<<rows.n, kThreads, 0, st>>>(a, rows);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
@@ -749,7 +749,7 @@ cudaError_t launch_latent_prompt(const LatentArgs& a, const TmaMap& upmap, const
   XMaps x;
   if (!encode_bf16_map(&x.narrow, base, keys, a.rank, a.width, kGemmTokenBox) || !encode_bf16_map(&x.wide, base, keys, a.rank, a.width, 128))
     return cudaErrorInvalidValue;
-  e = launch_gemm_bf16(LinearArgs{a.up, nullptr, ACT_NONE, 0, keys}, upmap, x, nullptr, a.kv, a.kv_ld, status, st);
+  e = launch_gemm_bf16(LinearArgs{a.up, nullptr, ACT_NONE, 0, keys}, upmap, x, nullptr, a.kv, a.kv_ld, status, sm_count, st);
   if (e != cudaSuccess) return e;
   if (a.vdim <= 32) e = launch_prompt_tiles<4>(a, rows, key0, out, ldo, st);
   else if (a.vdim <= 64) e = launch_prompt_tiles<8>(a, rows, key0, out, ldo, st);

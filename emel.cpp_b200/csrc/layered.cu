@@ -283,7 +283,7 @@ bool x_maps(XMaps* x, const void* base, int64_t rows, int64_t k, int64_t ld) {
 void linear(Layered* m, LayeredRun& r, const LinearArgs& a, const TmaMap& wmap, const void* x, int64_t ldx, const XMaps& xm, float* y, bf16* yb,
             int64_t ldy) {
   if (m->f32) check(m, r, launch_linear_f32(a, static_cast<const float*>(x), ldx, y, ldy, r.st));
-  else check(m, r, launch_gemm_bf16(a, wmap, xm, y, yb, ldy, m->c->status_word(), r.st));
+  else check(m, r, launch_gemm_bf16(a, wmap, xm, y, yb, ldy, m->c->status_word(), m->c->sm_count, r.st));
 }
 
 // the mixer of one layer run over rows: in (operands, ld pad8(n_embd)) -> heads {rows, out_dim} at out
@@ -327,7 +327,7 @@ void mixer_rows(Layered* m, LayeredRun& r, const LayerS& l, const RunS& run, con
   } else if (l.latent()) {
     const LatentArgs a = latent_args(m, l, run, proj, ldp, tail, tail_ld);
     if (!m->f32 && rows.prompt && latent_prompt_supported(a, n))
-      check(m, r, launch_latent_prompt(a, l.w.up_map, rows, pos0, reinterpret_cast<bf16*>(out), ldo, m->c->status_word(), r.st, &r.launches), 0);
+      check(m, r, launch_latent_prompt(a, l.w.up_map, rows, pos0, reinterpret_cast<bf16*>(out), ldo, m->c->status_word(), m->c->sm_count, r.st, &r.launches), 0);
     else
       check(m, r, (launch_latent_rows<T, T, T>(a, rows, out, ldo, m->c->sm_count, false, r.st, &r.launches)), 0);
   } else {

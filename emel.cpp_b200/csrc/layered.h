@@ -87,7 +87,7 @@ bool encode_bf16_map(TmaMap* map, const __nv_bfloat16* base, int64_t rows, int64
 constexpr int kGemmWeightBox = 128, kGemmTokenBox = 16;
 struct XMaps { TmaMap narrow, wide; };   // the activations as boxes of kGemmTokenBox and of 128 rows
 cudaError_t launch_gemm_bf16(const LinearArgs& a, const TmaMap& wmap, const XMaps& x, float* y, __nv_bfloat16* yb, int64_t ldy,
-                             int* status, cudaStream_t st);
+                             int* status, int sm_count, cudaStream_t st);
 
 // ---- mixer_ops.cu: row kernels between the products.  T = operand type of the following product (float or bf16)
 // rms: 0 layer norm, 1 RMS norm; step (optional): added to the stream after that
@@ -225,7 +225,7 @@ cudaError_t launch_latent_rows(const LatentArgs& a, const Rows& rows, TO* out, i
 // prompts on the tensor cores: keys and values of every visible position are projected first (upmap: `up`)
 bool latent_prompt_supported(const LatentArgs& a, int rows);
 cudaError_t launch_latent_prompt(const LatentArgs& a, const TmaMap& upmap, const Rows& rows, int pos0, __nv_bfloat16* out, int64_t ldo, int* status,
-                                 cudaStream_t st, int* launches);
+                                 int sm_count, cudaStream_t st, int* launches);
 
 // ---- delta.cu: gated delta rule
 struct DeltaArgs {
