@@ -146,3 +146,46 @@ def test_sequences_of_every_range_length(be, port, dim, heads):
             assert list(got[:, j]) == alone_ids[j], tokens[j]
     finally:
         sess.close()
+
+
+def test_columns_argmax_ties_and_nans(be, port):
+    """The highest logit, the lowest row on ties; a NaN in row 0 is a candidate that nothing replaces, a later one never
+    becomes the result.  Rows of the output matrix are made equal, or NaN by their scales."""
+    sess, cpu = build_model(be, port, MIXED, {"embd": eb.Q8_0, "output": eb.Q8_0, "default": eb.Q8_0}, seed=33)
+    cpu.close()
+    kept = []
+
+    def bind_output(change):
+        rows = output.copy()
+        change(rows)
+        kept.append(rows)
+        be.upload(900_000 + len(kept), kept[-1], tensor_type=eb.Q8_0)
+        assert sess.bind_matrix(-1, el.OUTPUT, kept[-1], eb.Q8_0), sess.last_error
+
+    def make_nan(rows, which):
+        rows[which, 0:2] = np.array([0x00, 0x7e], np.uint8)      # the first block's f16 scale
+
+    try:
+        k, m = MIXED["n_embd"], MIXED["n_vocab"]
+        w = synth.rng(34).standard_normal((m, k), dtype=np.float32) * np.float32(0.05)
+        output = np.ascontiguousarray(port.encode_rows(eb.Q8_0, w, k, m)).reshape(m, -1)
+        assert sess.set_sequences(3)
+        first, pos = fill_sequences(sess, MIXED, 3, seed=6)
+        bind_output(lambda rows: None)
+        ids, logits = sess.decode_batch(first, pos, want_logits=True)
+        top = [int(np.argmax(l)) for l in logits]
+        assert list(ids) == top
+        low, high = [r for r in (13, 14, 15, 17, 18, 19) if r not in top][:2]
+        bind_output(lambda rows: rows.__setitem__([low, high], rows[top[1]]))
+        ids = sess.decode_batch(first, pos)
+        assert ids[1] == min(low, top[1])
+        # rows 6 and 7 and the last one: not the first row of a scanned range (four rows each)
+        bad = [r for r in (6, 7, 11, m - 1)]
+        bind_output(lambda rows: make_nan(rows, bad))
+        ids, logits = sess.decode_batch(first, pos, want_logits=True)
+        for j in range(3):
+            assert np.isnan(logits[j][bad]).all() and int(ids[j]) == int(np.nanargmax(logits[j])), j
+        bind_output(lambda rows: make_nan(rows, [0, 9]))
+        assert list(sess.decode_batch(first, pos)) == [0, 0, 0]
+    finally:
+        sess.close()

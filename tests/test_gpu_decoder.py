@@ -242,6 +242,24 @@ def test_batched_prompt_many_layers_within_attention_noise(be, port, cfg, types)
         sess.close()
 
 
+def test_batched_prompt_with_a_q6_k_key_projection_between_q4_k_ones(be, port):
+    """K = 512: the key projection lays its own operand over the one the query projection left for the value projection.
+    One layer, so bit-identical to the token-by-token walk."""
+    cfg = dict(TINY, n_layer=1, n_ctx=384)
+    sess, cpu = build_model(be, port, cfg, {"embd": eb.Q4_K, "output": eb.Q6_K, "default": eb.Q4_K, el.ATTN_K: eb.Q6_K}, seed=31)
+    cpu.close()
+    try:
+        prompt = synth.rng(41).integers(0, cfg["n_vocab"], size=321).tolist()
+        assert sess.set_prefill_batch(0)
+        base = _prompt_then_logits(be, sess, prompt, [320])
+        assert sess.set_prefill_batch(2048)
+        assert sess.prefill(synth.rng(5).integers(0, cfg["n_vocab"], size=320).tolist(), 0)    # scrub
+        got = _prompt_then_logits(be, sess, prompt, [320])
+        assert np.array_equal(got.view(np.uint32), base.view(np.uint32))
+    finally:
+        sess.close()
+
+
 def test_batched_prompt_fills_the_context_to_the_last_row(be, port):
     """A prompt that ends on the last but one cache row, batches of 2 and of 61 tokens, and the decode step
     on the last row: bit-identical to the token-by-token walk (one layer), and requests past the context
