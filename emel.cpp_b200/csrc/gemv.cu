@@ -76,8 +76,10 @@ __global__ void argmax_f32_kernel(const float* x, int n, float* out_val, int* ou
 
 // ---------------------------------------------------------------- generic kernel
 // Any K that is a multiple of the block size, any 2-byte-aligned base: one warp
-// per row, lanes stride over blocks, byte loads.  Used for shapes the streaming
-// kernel does not take (K % 2048 != 0 or an unaligned view); not a fast path.
+// per row, lanes stride over blocks, byte loads.  Used for the argmax product of
+// shapes the streaming kernel does not take (K % 2048 != 0 or an unaligned view),
+// and for views that gemv_odd_kernel does not take either (weights at odd
+// addresses, Q4_K rows that are not 16-byte aligned); not a fast path.
 __device__ __forceinline__ int scale_min_k4_sc(int j, const uint8_t* q) {
   return j < 4 ? (q[j] & 63) : ((q[j + 4] & 0x0f) | ((q[j - 4] >> 6) << 4));
 }

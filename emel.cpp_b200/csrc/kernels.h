@@ -127,11 +127,12 @@ bool gemv_takes_tensor_core(int type, const GemvArgs& a, int ncols);
 bool gemm_q8_mma_supported(int type, const GemvArgs& a, int ncols);
 cudaError_t launch_gemm_q8_mma(int type, const GemvArgs& a, int ncols, int sm_count, cudaStream_t st);
 
-// gemm_q4k_mma.cu: 5 to 31 columns of Q4_K weights (mma.sync int8, one sub-block per instruction)
+// gemm_q6k_mma.cu: nine and more columns of Q6_K weights, K % 2048 == 0 (mma.sync int8, one scale group per instruction)
 bool gemm_q6k_mma_supported(int type, const GemvArgs& a, int ncols);
 cudaError_t launch_gemm_q6k_mma(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st);
+// gemm_q4k_mma.cu: 5 to 31 columns of Q4_K weights (mma.sync int8, one sub-block per instruction)
 bool gemm_q4k_mma_supported(int type, const GemvArgs& a, int ncols);
-// gemm_q6k_tc.cu: several columns of Q6_K weights on tcgen05, K that gemm_q6k_mma.cu does not take; overwrites the tensor-core workspace
+// gemm_q6k_tc.cu: several columns of Q6_K weights on tcgen05, K and rows that gemm_q6k_mma.cu does not take; overwrites the tensor-core workspace
 bool gemm_q6k_tc_supported(int type, const GemvArgs& a, int ncols);
 cudaError_t launch_gemm_q6k_tc(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st, int* launches);
 cudaError_t launch_gemm_q4k_mma(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st);
