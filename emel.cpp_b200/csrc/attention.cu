@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(128) flash_split_kernel(const FlashArgs a) {
 // several sequences: short ones take four ranges per CTA, one a warp, with the same bits.  The body for long ranges stands
 // first, where it is as fast as in the kernel above (the order of the two bodies and the size of the second matter: see
 // split_warp).  us a launch at 8B shape, this kernel against the one above: 16 sequences of 300 tokens 30 / 72, of 1100
-// 35.6 / 80.4, of 4000 98.6 / 98.2; 2 of 1100 11.8 / 16.2, of 4000 18.2 / 18.2; 1 of 1100 11.6 / 8.1 -- one sequence keeps to the other
+// 35.6 / 80.4, of 4000 98.6 / 98.2; 2 of 1100 11.8 / 16.2, of 4000 18.2 / 18.2; 1 of 1100 11.6 / 8.1: see launch_split_rep
 template <int D, int NREP>
 __global__ void __launch_bounds__(128) flash_split_seqs_kernel(const FlashArgs a) {
   pdl_trigger();
@@ -267,18 +267,28 @@ __global__ void flash_ref_sequential_kernel(const FlashArgs a, const float* scor
   }
 }
 
+// a CTA per range for one sequence, and while all of them run at once: four warps finish a range before one does.  us a launch, a CTA a
+// range and a warp a range: 8B shape (444 CTAs at once), 2 sequences of 60 tokens in two ranges 6.9 / 8.5, of 600 in 20 9.1 / 11.7
+// (320 CTAs), 3 of 600 15.0 / 12.0 (480), 2 of 300 in 37 15.8 / 9.6 (592); D = 64 (740 at once), 4 of 600 9.1 / 13.7 (640), 2 of 300 in
+// 63 13.7 / 11.8 (1008)
 template <int D, int NREP>
-cudaError_t launch_split_rep(const FlashArgs& a, int n_rep, cudaStream_t st) {
-  const bool several = a.kv_heads_per_seq > 0 && a.kv_heads > a.kv_heads_per_seq;
+cudaError_t launch_split_rep(const FlashArgs& a, int n_rep, int sm_count, cudaStream_t st) {
+  bool several = a.kv_heads_per_seq > 0 && a.kv_heads > a.kv_heads_per_seq;
+  if (several) {
+    int per_sm = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, flash_split_kernel<D, NREP>, 128, 0);
+    if (e != cudaSuccess) return e;
+    several = (int64_t)a.splits * a.kv_heads * (n_rep / NREP) > (int64_t)per_sm * sm_count;
+  }
   EMELB_LAUNCH((several ? flash_split_seqs_kernel<D, NREP> : flash_split_kernel<D, NREP>), dim3(a.splits, a.kv_heads, n_rep / NREP), 128, 0, st, a);
   return cudaGetLastError();
 }
 
 template <int D>
-cudaError_t launch_split(const FlashArgs& a, int n_rep, cudaStream_t st) {
-  if (n_rep % 4 == 0) return launch_split_rep<D, 4>(a, n_rep, st);
-  if (n_rep % 2 == 0) return launch_split_rep<D, 2>(a, n_rep, st);
-  return launch_split_rep<D, 1>(a, n_rep, st);
+cudaError_t launch_split(const FlashArgs& a, int n_rep, int sm_count, cudaStream_t st) {
+  if (n_rep % 4 == 0) return launch_split_rep<D, 4>(a, n_rep, sm_count, st);
+  if (n_rep % 2 == 0) return launch_split_rep<D, 2>(a, n_rep, sm_count, st);
+  return launch_split_rep<D, 1>(a, n_rep, sm_count, st);
 }
 
 }  // namespace
@@ -305,10 +315,9 @@ bool flash_merge_can_quantize(const FlashArgs& a) { return (a.heads * a.head_dim
 
 cudaError_t launch_flash_decode(const FlashArgs& a, int sm_count, cudaStream_t st, int* launches, int out_family,
                                 ActPlanesMut out_planes) {
-  (void)sm_count;
   if (a.join_out && (a.heads * a.head_dim) % 256 != 0) return cudaErrorInvalidValue;
   const int n_rep = a.heads / a.kv_heads;
-  cudaError_t e = a.head_dim == 64 ? launch_split<64>(a, n_rep, st) : launch_split<128>(a, n_rep, st);
+  cudaError_t e = a.head_dim == 64 ? launch_split<64>(a, n_rep, sm_count, st) : launch_split<128>(a, n_rep, sm_count, st);
   if (e != cudaSuccess) return e;
   const int total = a.heads * a.head_dim;
   if (total % 256 == 0) {
