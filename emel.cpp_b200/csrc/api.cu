@@ -351,8 +351,8 @@ uint32_t emelb_create(int device, emelb_ctx** out) {
   ok = ok && cudaMalloc(&c->act_qs, c->act_capacity) == cudaSuccess;
   ok = ok && cudaMalloc(&c->act_d, c->act_capacity / 32 * sizeof(float)) == cudaSuccess;
   ok = ok && cudaMalloc(&c->act_bsums, c->act_capacity / 16 * sizeof(int16_t)) == cudaSuccess;
-  // Q4_K: tiles of 128 columns x 256 K, 32 KB of int8 + 2.5 KB of block sums and scales; columns padded to 128.  Q6_K (512 bytes
-  // of f16 and a scale for 256 K of a column) takes the columns in as many turns as that holds: one at the default size
+  // operands of the tcgen05 kernels: 512 bytes of f16 for 256 K of a column, with Q4_K 40 of block sums, scale and mean and the
+  // weights' table beside them.  Columns that it does not hold are taken in turns: one at the default size for 2048 columns
   c->tc_ws_bytes = c->act_capacity / 32768 * 35328 + (64u << 20);
   ok = ok && cudaMalloc(&c->tc_ws, c->tc_ws_bytes) == cudaSuccess;
   ok = ok && cudaMalloc(&c->gemv_sched, (2 * kSchedSlots + 2) * sizeof(int)) == cudaSuccess;

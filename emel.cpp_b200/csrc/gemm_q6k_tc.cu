@@ -39,9 +39,12 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "tc_common.cuh"
 
 namespace emelb {
 namespace {
+
+using namespace tc;
 
 constexpr int BM = 128;
 constexpr int kEpilogueWarp0 = 8, kEpilogueWarps = 8, kMmaWarp = 16, kLoaderWarp = 17;
@@ -49,9 +52,7 @@ constexpr int kThreads = 20 * 32;
 constexpr int kProducerRegs = 80, kEpilogueRegs = 136, kOtherRegs = 48;
 static_assert(8 * 32 * kProducerRegs + 8 * 32 * kEpilogueRegs + 4 * 32 * kOtherRegs <= kThreads * 96, "register split");
 
-// activations in the workspace, and in shared memory: half super-blocks of 128 K, 8-column groups of two K-major
-// 128-byte swizzle atoms (8 columns x 64 values)
-constexpr int kAtomBytes = 1024;
+// activations in the workspace, and in shared memory: half super-blocks of 128 K, 8-column groups of two swizzle atoms
 constexpr int kGroupBytes = 2 * kAtomBytes;             // one 8-column group of a half
 constexpr int kColPad = 64;                             // the workspace's columns come in groups: whole tiles, whole pre-pass blocks
 
@@ -68,133 +69,6 @@ constexpr int kOffBars = kOffColMeta + kColMetaSlots * kMaxTN * 4;
 constexpr int kSmemBytes = kOffBars + 256 + 1024;   // barriers; slack for the base's alignment
 
 constexpr uint32_t kTmemA = 256;   // first operand column
-
-constexpr int kWaitSpins = 1 << 26;
-constexpr unsigned long long kWaitNs = 2000000000ull;  // 2 s
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// bounded wait; false when it gave up or another role already raised the abort flag
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  unsigned long long t0 = 0;
-  for (int spins = 0; spins < kWaitSpins; ++spins) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((spins & 63) == 63) {
-      if (*abort_flag) return false;
-      unsigned long long now;
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-      if (t0 == 0) t0 = now;
-      else if (now - t0 > kWaitNs) break;
-    }
-  }
-  *abort_flag = 1;
-  return false;
-}
-
-// one thread of the warp; the compiler then knows that a single one issues what follows (an MMA loop under lane == 0
-// took 116-133 cycles an instruction, under elect.sync 84)
-__device__ __forceinline__ bool elect_one() {
-  uint32_t e;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
-  return e != 0;
-}
-
-// B operand: K-major, 128-byte swizzle, 8-column groups kGroupBytes apart (descriptor version 1)
-__device__ __forceinline__ uint64_t operand_desc(uint32_t saddr) {
-  return (uint64_t)((saddr >> 4) & 0x3fffu) | (uint64_t)1 << 16 | (uint64_t)(kGroupBytes >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
-}
-
-// D {128 lanes, N} (+)= A (TMEM, f16) * B (shared memory, f16), f32 accumulators
-__device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// 8 columns of the warp's TMEM lanes
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]),
-               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
-               : "memory");
-}
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// 16 TMEM lanes x 16 columns in the m16n8 accumulator-fragment layout: v[0..3] = columns 0-7, v[4..7] = columns
-// 8-15; within a block thread (g, t) gets (row g, col 2t), (row g, col 2t+1), (row g+8, col 2t), (row g+8, col 2t+1)
-__device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&v)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-               : "r"(taddr)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-
-using f2 = unsigned long long;   // two floats
-__device__ __forceinline__ f2 pack2(float a, float b) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ f2 pack2u(uint32_t a, uint32_t b) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
-  return r;
-}
-__device__ __forceinline__ float2 unpack2(f2 v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-  f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-  f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint32_t h2_bits(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
-__device__ __forceinline__ __half2 bits_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
-// exact: masked weight bits (f16 subnormals) * s + c
-__device__ __forceinline__ uint32_t expand2(uint32_t bits, __half2 s, __half2 c) { return h2_bits(__hfma2(bits_h2(bits), s, c)); }
 
 struct GemmArgs {
   const uint8_t* W;
@@ -253,25 +127,25 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q6k_tc_kernel(const GemmArgs
   uint8_t* raw = smem + kOffRaw;
   uint8_t* rowmeta = smem + kOffRowMeta;
   uint8_t* colmeta = smem + kOffColMeta;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kOffBars);
-  uint64_t* a_full = bars;                   // [2 halves] producers -> MMA
-  uint64_t* a_free = a_full + 2;
-  uint64_t* x_full = a_free + 2;             // [kHalves] bulk copies -> MMA
-  uint64_t* x_free = x_full + kHalves;
-  uint64_t* m_full = x_free + kHalves;       // [3] bulk copies -> epilogue: the columns' scales of a super-block
-  uint64_t* m_free = m_full + kColMetaSlots;
-  uint64_t* d_full = m_free + kColMetaSlots;   // [2] MMA -> epilogue: the accumulators hold a finished super-block
-  uint64_t* d_free = d_full + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_free + 2);
+  const uint32_t bars = smem_u32(smem + kOffBars);
+  const uint32_t a_full = bars;                      // [2 halves] producers -> MMA
+  const uint32_t a_free = a_full + 8 * 2;
+  const uint32_t x_full = a_free + 8 * 2;            // [kHalves] bulk copies -> MMA
+  const uint32_t x_free = x_full + 8 * kHalves;
+  const uint32_t m_full = x_free + 8 * kHalves;      // [3] bulk copies -> epilogue: the columns' scales of a super-block
+  const uint32_t m_free = m_full + 8 * kColMetaSlots;
+  const uint32_t d_full = m_free + 8 * kColMetaSlots;   // [2] MMA -> epilogue: the accumulators hold a finished super-block
+  const uint32_t d_free = d_full + 8 * 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kOffBars + 8 * (8 + 2 * kHalves + 2 * kColMetaSlots));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int TN = p.TN;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < 2; ++s) { mbar_init(a_full + s, 4); mbar_init(a_free + s, 1); }
-    for (int s = 0; s < kHalves; ++s) { mbar_init(x_full + s, 1); mbar_init(x_free + s, 1); }
-    for (int s = 0; s < kColMetaSlots; ++s) { mbar_init(m_full + s, 1); mbar_init(m_free + s, kEpilogueWarps); }
-    for (int s = 0; s < 2; ++s) { mbar_init(d_full + s, 1); mbar_init(d_free + s, kEpilogueWarps); }
+    for (int s = 0; s < 2; ++s) { mbar_init(a_full + 8 * s, 4); mbar_init(a_free + 8 * s, 1); }
+    for (int s = 0; s < kHalves; ++s) { mbar_init(x_full + 8 * s, 1); mbar_init(x_free + 8 * s, 1); }
+    for (int s = 0; s < kColMetaSlots; ++s) { mbar_init(m_full + 8 * s, 1); mbar_init(m_free + 8 * s, kEpilogueWarps); }
+    for (int s = 0; s < 2; ++s) { mbar_init(d_full + 8 * s, 1); mbar_init(d_free + 8 * s, kEpilogueWarps); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -331,7 +205,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q6k_tc_kernel(const GemmArgs
       const uint32_t* bw = reinterpret_cast<const uint32_t*>(blk);
       auto word = [&](int i) { return __funnelshift_r(bw[i], bw[i + 1], sh); };   // i: 0 ql, 17 qh, 26 scales of the half
       const uint32_t sw[2] = {word(26), word(27)};   // the half's eight scales
-      live = mbar_wait(a_free + n, (it & 1) ^ 1, abort_flag);
+      live = mbar_wait(a_free + 8 * n, (it & 1) ^ 1, abort_flag);
       live = __all_sync(0xffffffffu, live);
       if (!live) break;
       fence_after();
@@ -374,7 +248,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q6k_tc_kernel(const GemmArgs
       tmem_wait_st();
       fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(a_full + n);
+      if (lane == 0) mbar_arrive(a_full + 8 * n);
       if (++slot == kRawSlots) slot = 0;
       if (++kb == nkb) { kb = 0; tile += gridDim.x; }
     }
@@ -385,17 +259,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q6k_tc_kernel(const GemmArgs
       // -------------------------------------------------------------- MMA issue (one thread)
       // D = f32, A = B = f16, both K-major, M = 128 weight rows, N = TN columns
       const uint32_t idesc = (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-      const uint64_t x0 = operand_desc(smem_u32(smem));
+      const uint64_t x0 = operand_desc(smem_u32(smem), kGroupBytes);
       bool live = true, issued = false;
       int last = 0, xs = 0, xphase = 0;
       for (int it = 0; live && it < turns; ++it) {
         const int buf = it & 1;
         const uint32_t d = tmem_base + (uint32_t)(2 * TN * buf);
-        live = mbar_wait(d_free + buf, ((it >> 1) & 1) ^ 1, abort_flag);
+        live = mbar_wait(d_free + 8 * buf, ((it >> 1) & 1) ^ 1, abort_flag);
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
           if (!live) break;
-          live = mbar_wait(a_full + n, (uint32_t)it & 1u, abort_flag) && mbar_wait(x_full + xs, xphase, abort_flag);
+          live = mbar_wait(a_full + 8 * n, (uint32_t)it & 1u, abort_flag) && mbar_wait(x_full + 8 * xs, xphase, abort_flag);
           if (!live) break;
           fence_after();
           const uint64_t x = x0 + (uint64_t)(xs * (kHalfBytes >> 4));
@@ -406,19 +280,19 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q6k_tc_kernel(const GemmArgs
             for (int j = 0; j < 8; ++j)
               mma_f16(d + (uint32_t)(r * TN), a_op + 128u * r + 8u * j, x + (uint64_t)(((j >> 2) * kAtomBytes + (j & 3) * 32) >> 4), idesc,
                       (n | j) ? 1u : 0u);
-          mma_commit(a_free + n);
-          mma_commit(x_free + xs);
+          mma_commit(a_free + 8 * n);
+          mma_commit(x_free + 8 * xs);
           if (++xs == kHalves) { xs = 0; xphase ^= 1; }
           issued = true;
         }
         if (issued) {
-          mma_commit(d_full + buf);
+          mma_commit(d_full + 8 * buf);
           last = it;
         }
       }
       if (!live && issued) {
         // gave up: let the tensor core finish what was issued before the TMEM goes away (bounded)
-        for (int spins = 0; spins < (1 << 16) && !mbar_try_wait(d_full + (last & 1), (uint32_t)(last >> 1) & 1u); ++spins) {}
+        for (int spins = 0; spins < (1 << 16) && !mbar_try_wait(d_full + 8 * (last & 1), (uint32_t)(last >> 1) & 1u); ++spins) {}
       }
     } else if (warp == kLoaderWarp && lane == 0) {
       // -------------------------------------------------------------- activation loader (one thread)
@@ -429,17 +303,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q6k_tc_kernel(const GemmArgs
       for (int it = 0; live && it < turns; ++it) {
         const int c0 = (tile % nt) * TN;
         for (int n = 0; live && n < 2; ++n) {
-          live = mbar_wait(x_free + xs, xphase ^ 1, abort_flag);
+          live = mbar_wait(x_free + 8 * xs, xphase ^ 1, abort_flag);
           if (!live) break;
-          mbar_arrive_expect_tx(x_full + xs, xbytes);
-          bulk_g2s(smem + xs * kHalfBytes, p.x + ((size_t)(2 * kb + n) * (p.npad >> 3) + (c0 >> 3)) * kGroupBytes, xbytes, x_full + xs);
+          mbar_arrive_expect_tx(x_full + 8 * xs, xbytes);
+          bulk_g2s(smem + xs * kHalfBytes, p.x + ((size_t)(2 * kb + n) * (p.npad >> 3) + (c0 >> 3)) * kGroupBytes, xbytes, x_full + 8 * xs);
           ++sent_x;
           if (++xs == kHalves) { xs = 0; xphase ^= 1; }
         }
-        live = live && mbar_wait(m_free + ms, mphase ^ 1, abort_flag);
+        live = live && mbar_wait(m_free + 8 * ms, mphase ^ 1, abort_flag);
         if (live) {
-          mbar_arrive_expect_tx(m_full + ms, dbytes);
-          bulk_g2s(colmeta + ms * kMaxTN * 4, p.dx + (size_t)kb * p.npad + c0, dbytes, m_full + ms);
+          mbar_arrive_expect_tx(m_full + 8 * ms, dbytes);
+          bulk_g2s(colmeta + ms * kMaxTN * 4, p.dx + (size_t)kb * p.npad + c0, dbytes, m_full + 8 * ms);
           ++sent_m;
           if (++ms == kColMetaSlots) { ms = 0; mphase ^= 1; }
         }
@@ -448,9 +322,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q6k_tc_kernel(const GemmArgs
       if (!live) {
         // gave up: let the copies in flight land (bounded)
         for (int i = max(0, sent_x - kHalves); i < sent_x; ++i)
-          for (int spins = 0; spins < (1 << 16) && !mbar_try_wait(x_full + i % kHalves, (i / kHalves) & 1); ++spins) {}
+          for (int spins = 0; spins < (1 << 16) && !mbar_try_wait(x_full + 8 * (i % kHalves), (i / kHalves) & 1); ++spins) {}
         for (int i = max(0, sent_m - kColMetaSlots); i < sent_m; ++i)
-          for (int spins = 0; spins < (1 << 16) && !mbar_try_wait(m_full + i % kColMetaSlots, (i / kColMetaSlots) & 1); ++spins) {}
+          for (int spins = 0; spins < (1 << 16) && !mbar_try_wait(m_full + 8 * (i % kColMetaSlots), (i / kColMetaSlots) & 1); ++spins) {}
       }
     }
   } else {
@@ -474,7 +348,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q6k_tc_kernel(const GemmArgs
 #pragma unroll
         for (int i = 0; i < 8 * kPieces; ++i) acc[i >> 3][(i >> 2) & 1][(i >> 1) & 1][i & 1] = 0ull;
       }
-      bool live = mbar_wait(m_full + ms, mphase, abort_flag) && mbar_wait(d_full + buf, (uint32_t)(it >> 1) & 1u, abort_flag);
+      bool live = mbar_wait(m_full + 8 * ms, mphase, abort_flag) && mbar_wait(d_full + 8 * buf, (uint32_t)(it >> 1) & 1u, abort_flag);
       live = __all_sync(0xffffffffu, live);
       if (!live) break;
       fence_after();
@@ -521,8 +395,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q6k_tc_kernel(const GemmArgs
       fence_before();
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(d_free + buf);
-        mbar_arrive(m_free + ms);
+        mbar_arrive(d_free + 8 * buf);
+        mbar_arrive(m_free + 8 * ms);
       }
       if (++ms == kColMetaSlots) { ms = 0; mphase ^= 1; }
       if (++kb == nkb) {

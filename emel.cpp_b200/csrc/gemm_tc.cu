@@ -1,248 +1,274 @@
-// Q4_K x Q8_K matrix product for many columns (prompt processing) on the
-// Blackwell tensor cores: tcgen05.mma kind::i8 with int32 accumulators in TMEM.
+// Q4_K x Q8_K matrix product for many columns (prompt processing) on the Blackwell tensor cores: tcgen05.mma kind::f16,
+// weights as the A operand in TMEM, activations as the B operand in shared memory, f32 accumulators in TMEM that only
+// ever hold exact integers.
 //
 // What is computed is exactly the reference's per-super-block value,
-//   fma(d*dx, isum, -(dmin*dx)*msum),   isum = sum_j sc_j * dot_j(q, x),
-//   msum = sum_j m_j * bsum_j           (src/emel/kernel/x86_64/actions.hpp:859-866)
-// added in ascending block order, so the result equals the mat-vec kernels' (and
-// the x86 AVX2 route's) bit for bit.  The integer part runs on the tensor cores:
-//   * a 6-bit scale times a 4-bit quant does not fit int8, so sc_j = 8*hi_j + lo_j
-//     and two int8 operands are built per row, q*lo_j and q*hi_j (each <= 105);
-//     isum = D_lo + 8*D_hi, exact in int32;
-//   * one MMA has K = 32 = one sub-block.  The activations are the M operand (128
-//     tokens = TMEM lanes) and the two weight operands sit side by side in the N
-//     operand (128 rows of q*lo, then 128 rows of q*hi), so ONE 128 x 256 x 32 MMA
-//     per sub-block produces both D_lo (columns 0-127) and D_hi (128-255) and the
-//     activation slice is fetched from shared memory once; 8 MMAs cover a
-//     super-block of 256; then the accumulators are read back (tcgen05.ld) and
-//     folded into f32 registers with the block's scales — the float chain stays on
-//     the CUDA cores because its order and roundings are part of the contract.
+//   fma(d*dx, isum, -(dmin*dx)*msum),   isum = sum_j sc_j * dot_j(q, x),   msum = sum_j m_j * bsum_j
+//   (src/emel/kernel/x86_64/actions.hpp:859-866)
+// added in ascending block order, so the result equals the mat-vec kernels' (and the x86 AVX2 route's) bit for bit.
+//   * A weight times its scale, q * sc <= 15 * 63 = 945, is exact in f16, so one operand carries both.
+//   * f32 sums are exact below 2^24, which sum 945 * |x| over 256 can pass.  So the activations are centred: u = x - v with
+//     v = the rounded mean of the super-block's 256 values, an integer within +-255 and exact in f16.  The positive
+//     and the negative u of a super-block then sum to at most 16448 each, so any partial sum of q * sc * u stays
+//     below 945 * 16448 < 2^24 in any order, and (float)isum = fma(v, T, D) with T = sum q * sc of the row: v * T + D is
+//     the exact integer, rounded once.
+//   * msum comes from one K = 16 instruction: the row's mins (each twice) times the 16 block sums, all exact.
+// The expanded weights pass through neither the shared memory nor its port: a thread owns a weight row = a TMEM lane
+// and writes the operand with tcgen05.st.  Expanding two weights is one mask and one half2 fma: a masked 4-bit quant
+// under the exponent of 1024 is 1024 + q (1024 + 16 q), times sc (sc / 16) minus 1024 sc (64 sc) is q * sc without a
+// rounding.  The order of a super-block's 256 weights along the MMA's K is free (the sums are exact), so it follows
+// from the masks; a pre-pass lays the activations out alike.
 //
-// CTA = 128 rows x 128 columns, 21 warps:
-//   warps 0-3   producers: the 128 GGUF blocks of a super-block column are staged
-//               raw (16-byte cp.async, coalesced along rows) one iteration ahead;
-//               thread p expands row p into the two int8 operands in the
-//               canonical no-swizzle K-major layout (8 rows x 16 bytes core
-//               matrices).  The activation tile comes by bulk copy: a small
-//               pre-pass has already laid it out in that same layout (one
-//               contiguous 32 KB slab + per-column block sums and scales per
-//               128 columns x 256 K)
-//   warp  4     allocates TMEM, issues the MMAs, commits to two mbarriers
-//   warps 5-20  epilogue: four warps per TMEM lane quarter, 32 columns each; msum
-//               on the legacy mma.sync path in the accumulator-fragment layout
-//   warp  21    one thread starts the bulk copies of the next activation tile the
-//               moment an operand stage is released
-// Two operand stages are released by the MMA's completion, two TMEM accumulator
-// pairs and four small per-block scale slots by the epilogue, so producers,
-// tensor cores and epilogue work on different super-blocks at once.
-// Every mbarrier wait is bounded; on a timeout the CTA raises the status word,
-// stops issuing, and still frees its TMEM.
+// CTA = 128 weight rows (TMEM lanes) x TN columns (32, 64 or 128), one super-block of K per turn, 20 warps:
+//   warps 0-7   producers: two warps per TMEM lane quarter, one for each half (128 weights) of a super-block; a thread
+//               expands its row's half into TMEM, 64 weights at a time
+//   warps 8-15  epilogue: two warps per TMEM lane quarter, half of the columns each, a thread a row: the row's constants stay
+//               in registers, the float chain runs on packed f32x2 instructions
+//   warp  16    the MMAs of a super-block; TMEM allocation
+//   warp  17    the msum instructions
+//   warp  18    copies of the weights (TMA, 128 rows x 144 bytes) and of the activations, a quarter super-block each
+//   warp  19    copies of block sums, column scales and table
+// TMEM at TN = 128: two turns' accumulators (256 columns), msum of one turn (128, made and read in two parts, so that
+// the next turn's first part is made while the epilogue works on the second), the operand of one super-block (128, handed
+// over in quarters).  Narrower tiles keep two super-blocks of operand.
+// With several column tiles the mins' operand and {d, -dmin, T} of every row and super-block come from a table that a
+// pre-pass over the weights makes once (TN = 128); narrower tiles work them out while they expand.
+// Registers are split by setmaxnreg: 640 threads x 96 at launch = 256 x 80 + 256 x 136 + 128 x 48.
+// Every mbarrier wait is bounded; on a timeout the CTA raises the status word, lets its copies land and frees its TMEM.
+//
+// What bounds it: instruction issue, 60 % of the slots with some eight cycles between two instructions of a warp.  Per
+// 128 x 128 x 256: 6,600 warp instructions (1,536 packed float ones, 1,150 for the expansion), of 2,600 cycles the MMAs take
+// 1,090.  Measured, B200, 14336 x 4096 by 2048 columns: pre-passes and product 352 us, product alone 333 (340 and 722
+// TFLOP/s); the int8 kernel before it (two operands of scale pieces, sums of mins on mma.sync) 439.  Whole calls on planes,
+// before and now: 14336 x 4096 by 32 columns 47.7 -> 30.5, by 128 48.4 -> 44.6, by 512 159 -> 118; 4096 x 14336 by 32 134 -> 78,
+// by 333 136 -> 104, by 1900 517 -> 354; 1024 x 4096 by 333 47.6 -> 31.4.  What gave it: TMEM loads of whole lanes (32x32b, half
+// a cycle a register against two of 16x256b: 16 % of the product without its arithmetic), roles in few instructions (the
+// producers' loop not unrolled 374 -> 349), the table (233 -> 188 million instructions).  Without effect: tiles of 96 columns with
+// msum double-buffered (400), 16 epilogue warps (355), copies or MMAs left out (the memories and the tensor core wait).
+#include <cuda.h>
+#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "common.cuh"
 #include "kernels.h"
+#include "tc_common.cuh"
 
 namespace emelb {
 namespace {
 
-constexpr int BM = 128, BN = 128;
-constexpr int kProducerThreads = 128;
-constexpr int kMmaWarp = 4;
-constexpr int kEpilogueWarp0 = 5;
-constexpr int kLoaderWarp = 21;
-constexpr int kThreads = 22 * 32;
-constexpr int kEpilogueWarps = 16;
-constexpr int kStages = 2;
+using namespace tc;
 
-// shared memory map (bytes)
-constexpr int kOperandBytes = BM * 256;                 // one int8 operand tile of a super-block: 32 KB
-constexpr int kChunkStride = (BM / 8) * 128;            // activation tile: next 16-byte K chunk of the 128 tokens (2048 B)
-constexpr int kChunkStrideW = 2 * kChunkStride;         // weight tile: 256 operand rows (q*lo, then q*hi) per chunk (4096 B)
-constexpr int kGroupStride = 128;                       // next 8-row core matrix (stride byte offset)
-constexpr int kStageBytes = 3 * kOperandBytes;          // weights (q*lo | q*hi interleaved per K chunk: 64 KB), activations
-constexpr int kOffW = 0, kOffX = 2 * kOperandBytes;
-constexpr int kMetaSlots = 4;
-constexpr int kColMetaBytes = BN * 16 + BN * 4;         // per column: 8 pair sums as int8 low/high parts, then the scales dx
-constexpr int kRowMetaBytes = 12;                       // per row: {d, dmin} as f16 bits, mins[8]
-constexpr int kMetaBytes = BM * kRowMetaBytes + kColMetaBytes;
-constexpr int kOffRowMeta = 0, kOffColMeta = BM * kRowMetaBytes, kOffDx = kOffColMeta + BN * 16;
-constexpr int kRawBytes = BM * Q4_K_BYTES;              // raw GGUF blocks of one super-block column: 18,432 B
-constexpr int kBarBytes = 128;                          // full[2], mma_done[2], tmem_full[2], epi_done[2], tmem base, abort
-constexpr int kSmemBytes = kStages * kStageBytes + kMetaSlots * kMetaBytes + kRawBytes + kBarBytes + 128;  // + alignment slack
-// the activation tile a pre-pass writes for (128 columns, one super-block): operand B, then the column meta
-constexpr int kTileBytes = kOperandBytes + kColMetaBytes;
+constexpr int BM = 128;
+constexpr int kEpilogueWarp0 = 8, kEpilogueWarps = 8, kMmaWarp = 16, kSumWarp = 17, kLoaderWarp = 18;   // and the meta loader's warp
+constexpr int kThreads = 20 * 32;
 
-constexpr int kWaitSpins = 1 << 22;
-constexpr uint32_t kSuspendHintNs = 10000;
-constexpr unsigned long long kWaitNs = 2000000000ull;  // 2 s
+constexpr int kRawBytes = BM * Q4_K_BYTES;   // 128 rows of a super-block as they lie in memory; 144 bytes a row spread reads over the banks
+constexpr int kMetaSlots = 3;
+constexpr int kStageRow = 80;             // an epilogue warp's store: 16 columns of a row; a multiple of 16 that spreads rows over the banks
+constexpr int kRowMeta = 32;              // per row: d, d, -dmin, -dmin, then T of either half, each twice
+constexpr int kMinsBytes = BM * 32;       // A operand of the msum instruction: two 16-byte chunks of K
+constexpr int kSumBytes = 32;             // per column: 16 block sums as f16, two chunks
+constexpr int kPairBytes = 16;            // per two columns: dx, dx, v, v
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+constexpr int kTableRow = 24;             // per row of the table: d, d, -dmin, -dmin, T, T
+constexpr int kTableBytes = kMinsBytes + BM * kTableRow;   // of 128 rows x one super-block
 
-__device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"   // may sleep up to the hint instead of spinning
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(kSuspendHintNs)
-      : "memory");
-  return ok != 0;
-}
+template <int TN, bool kTable>
+struct Cfg {
+  static constexpr int kProducerRegs = 80, kEpilogueRegs = 136, kOtherRegs = 48;
+  static_assert(8 * kProducerRegs + 8 * kEpilogueRegs + 4 * kOtherRegs <= 20 * 96, "register split");
+  static constexpr int kTurns = TN == 32 ? 4 : 2;       // super-blocks of activations in shared memory
+  static constexpr int kRawSlots = TN == 128 ? 2 : 4;   // and of weights
+  static constexpr int kOperands = TN == 128 ? 1 : 2;   // super-blocks of operand in TMEM
+  static constexpr int kParts = TN >= 64 ? 2 : 1;       // of the columns: each has its msum made and is read by itself
+  static constexpr int kPart = TN / kParts;
+  // TMEM columns: accumulators of two turns, msum of one, then the operand
+  static constexpr uint32_t kTmemM = 2 * TN, kTmemA = TN == 128 ? 384 : 256;
+  static constexpr int kQuarterBytes = TN / 8 * kAtomBytes;   // activations of a quarter super-block (64 K)
+  // what a bulk-copied slot holds for a super-block: block sums, dx and v of the columns; with the table also mins and row meta
+  static constexpr int kOffPairs = TN * kSumBytes, kOffTable = kOffPairs + TN / 2 * kPairBytes;
+  static constexpr int kMetaBytes = kOffTable + (kTable ? kTableBytes : 0);
+  static constexpr int kMinsSlots = kTable ? 0 : kOperands + 2, kRowMetaSlots = kTable ? 0 : kOperands + 2;
+  // shared memory map
+  static constexpr int kOffRaw = 4 * kTurns * kQuarterBytes;
+  static constexpr int kOffMins = kOffRaw + kRawSlots * kRawBytes;
+  static constexpr int kOffRowMeta = kOffMins + kMinsSlots * kMinsBytes;
+  static constexpr int kOffMeta = kOffRowMeta + kRowMetaSlots * BM * kRowMeta;
+  static constexpr int kOffStage = kOffMeta + kMetaSlots * kMetaBytes;
+  static constexpr int kOffBars = kOffStage + kEpilogueWarps * 32 * kStageRow;
+  static constexpr int kSmemBytes = kOffBars + 512 + 1024;   // barriers; slack for the base's alignment
+  static_assert(kSmemBytes <= 227 * 1024, "shared memory");
+};
 
-// bounded wait; false when it gave up or another role already raised the abort flag
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  unsigned long long t0 = 0;
-  for (int spins = 0; spins < kWaitSpins; ++spins) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((spins & 15) == 15) {
-      if (*abort_flag) return false;
-      unsigned long long now;
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-      if (t0 == 0) t0 = now;
-      else if (now - t0 > kWaitNs) break;
-    }
-  }
-  *abort_flag = 1;
-  return false;
-}
-
-__device__ __forceinline__ uint64_t operand_desc(uint32_t saddr, uint32_t chunk_stride) {
-  // K-major, no swizzle: 14-bit fields in 16-byte units; descriptor version 1 (sm_100)
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3fffu);
-  d |= (uint64_t)((chunk_stride >> 4) & 0x3fffu) << 16;   // leading byte offset: between the two 16-byte K chunks
-  d |= (uint64_t)((kGroupStride >> 4) & 0x3fffu) << 32;   // stride byte offset: between 8-row groups
-  d |= (uint64_t)1 << 46;
-  return d;
-}
-
-// instruction descriptor: D = s32, A = B = signed 8-bit, both K-major, M = 128 tokens, N = 256 weight-operand rows
-constexpr uint32_t kInstrDesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)((2 * BM) >> 3) << 17) | ((uint32_t)(BN >> 4) << 24);
-
-__device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(da), "l"(db), "r"(kInstrDesc), "r"(accumulate)
-      : "memory");
-}
-
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-               : "r"(taddr)
-               : "memory");
-}
-
-// 16 TMEM lanes x 16 columns in the m16n8 accumulator-fragment layout: v[0..3] = columns 0-7, v[4..7] = columns
-// 8-15; within a block thread (g, t) gets (row g, col 2t), (row g, col 2t+1), (row g+8, col 2t), (row g+8, col 2t+1)
-__device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&v)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-               : "r"(taddr)
-               : "memory");
-}
-
-// D(16 tokens x 8 weight rows, f32) = A(16x16, f16) * B(16x8, f16) with A[token][k] = low parts (k < 8) and
-// 128 * high parts (k >= 8) of the token's block sums (a_lo0/a_lo1, a_hi0/a_hi1: tokens g, g+8) and
-// B[k][row] = B[k+8][row] = the weight row's k-th min
-__device__ __forceinline__ void mma_m16n8k16_f16(float (&dd)[4], uint32_t a_lo0, uint32_t a_lo1, uint32_t a_hi0, uint32_t a_hi1,
-                                                 uint32_t b_mins) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
-      : "=f"(dd[0]), "=f"(dd[1]), "=f"(dd[2]), "=f"(dd[3])
-      : "r"(a_lo0), "r"(a_lo1), "r"(a_hi0), "r"(a_hi1), "r"(b_mins), "r"(b_mins), "f"(0.0f), "f"(0.0f), "f"(0.0f), "f"(0.0f));
-}
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
+// K-major, no swizzle, 8-row groups of 128 bytes; chunk_stride: between the two 16-byte K chunks
+__device__ __forceinline__ uint64_t plain_desc(uint32_t saddr, uint32_t chunk_stride) {
+  return (uint64_t)((saddr >> 4) & 0x3fffu) | (uint64_t)(chunk_stride >> 4) << 16 | (uint64_t)(128 >> 4) << 32 | (uint64_t)1 << 46;
 }
 
 struct GemmArgs {
   const uint8_t* W;
   int64_t row_bytes;
   int M, K, N;
-  const uint8_t* tiles;   // [ceil(N/128)][K/256][kTileBytes]
+  const uint8_t* x;       // [K/64][npad/8] swizzle atoms of 8 columns
+  const uint8_t* sums;    // [K/256][2 chunks][npad][16 bytes]
+  const uint8_t* pairs;   // [K/256][npad/2]{dx, dx, v, v}
+  const uint8_t* table;   // [ceil(M/128)][K/256]{mins, row meta}
+  int npad;
   float* y;
   int64_t ldy;
   int* status;
 };
 
-// pre-pass: the quantized activation planes of columns col0.. -> tiles in operand order.
-// grid (K/256, ceil(N/128)), 256 threads; columns past N are zero.
-__global__ void __launch_bounds__(256) tile_activations_kernel(ActPlanes act, int col0, int N, int K, uint8_t* tiles) {
-  const int kb = blockIdx.x, tn = blockIdx.y, nkb = K / QK_K;
-  uint8_t* tile = tiles + ((size_t)tn * nkb + kb) * kTileBytes;
-  for (int q = threadIdx.x; q < BN * 16; q += 256) {
-    const int col = q & (BN - 1), c = q >> 7;           // piece q = (chunk c, column col) lands at q*16
-    const int gc = tn * BN + col;
+// pre-pass: the quantized activation planes of columns col0.. -> operand order.  K position 128 n + 16 w + 8 c + j of
+// a super-block holds element 128 n + 64 c + 32 (j / 4) + 4 w + {0, 2, 1, 3}[j % 4], which is what the producers'
+// masks leave side by side.  grid (K/256, npad/64), 256 threads; columns past N are zero.
+constexpr int kPreCols = 64, kPreRow = QK_K + 4;   // 65 words: column-wise reads fall on all banks
+
+__global__ void __launch_bounds__(256) centre_activations_kernel(ActPlanes act, int col0, int N, int npad, uint8_t* x, uint8_t* sums, uint8_t* pairs) {
+  __shared__ __align__(16) uint8_t t8[kPreCols * kPreRow];
+  __shared__ int mean[kPreCols];
+  const int kb = blockIdx.x, c0 = blockIdx.y * kPreCols;
+  for (int q = threadIdx.x; q < kPreCols * 16; q += 256) {
+    const int col = q >> 4, piece = q & 15;
     uint4 v = make_uint4(0, 0, 0, 0);
-    if (gc < N) v = *reinterpret_cast<const uint4*>(act.qs + (int64_t)(col0 + gc) * act.col_stride_qs + kb * QK_K + 16 * c);
-    *reinterpret_cast<uint4*>(tile + (size_t)q * 16) = v;
+    if (c0 + col < N) v = *reinterpret_cast<const uint4*>(act.qs + (int64_t)(col0 + c0 + col) * act.col_stride_qs + kb * QK_K + 16 * piece);
+    uint32_t* o = reinterpret_cast<uint32_t*>(t8 + col * kPreRow + 16 * piece);
+    o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
   }
-  if (threadIdx.x < BN) {
-    const int col = threadIdx.x, gc = tn * BN + col;
-    uint4 cm = make_uint4(0, 0, 0, 0);
-    float dx = 0.0f;
-    if (gc < N) {
-      const int4* bs = reinterpret_cast<const int4*>(act.bsums + (int64_t)(col0 + gc) * act.col_stride_bs + kb * 16);
+  if (threadIdx.x < kPreCols) {
+    const int col = threadIdx.x;
+    __half h[16];
+    float d = 0.0f;
+    int total = 0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) h[i] = __float2half_rn(0.0f);
+    if (c0 + col < N) {
+      const int4* bs = reinterpret_cast<const int4*>(act.bsums + (int64_t)(col0 + c0 + col) * act.col_stride_bs + kb * 16);
       const int4 b0 = bs[0], b1 = bs[1];
       const int w[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-      // pair sums (|s| <= 4064) split as s = 128*hi + lo with 0 <= lo < 128, so both parts are int8 for dp4a
-      uint32_t bl[8], bh[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int sj = (int)(short)(w[j] & 0xffff) + (w[j] >> 16);
-        bl[j] = (uint32_t)(sj & 127);
-        bh[j] = (uint32_t)(sj >> 7) & 0xffu;
+      for (int j = 0; j < 8; ++j) {   // |sum of 16| <= 2048: exact in f16
+        const int s0 = (int)(short)(w[j] & 0xffff), s1 = w[j] >> 16;
+        h[2 * j] = __int2half_rn(s0);
+        h[2 * j + 1] = __int2half_rn(s1);
+        total += s0 + s1;
       }
-      cm = make_uint4(bl[0] | (bl[1] << 8) | (bl[2] << 16) | (bl[3] << 24), bl[4] | (bl[5] << 8) | (bl[6] << 16) | (bl[7] << 24),
-                      bh[0] | (bh[1] << 8) | (bh[2] << 16) | (bh[3] << 24), bh[4] | (bh[5] << 8) | (bh[6] << 16) | (bh[7] << 24));
-      dx = act.d[(int64_t)(col0 + gc) * act.col_stride_d + kb];
+      d = act.d[(int64_t)(col0 + c0 + col) * act.col_stride_d + kb];
     }
-    *reinterpret_cast<uint4*>(tile + kOperandBytes + col * 16) = cm;
-    *reinterpret_cast<float*>(tile + kOperandBytes + BN * 16 + col * 4) = dx;
+    const int v = (total + 128) >> 8;
+    mean[col] = v;
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      *reinterpret_cast<uint4*>(sums + (((size_t)kb * 2 + c) * npad + c0 + col) * 16) = *reinterpret_cast<const uint4*>(h + 8 * c);
+    float* p = reinterpret_cast<float*>(pairs + ((size_t)kb * (npad >> 1) + ((c0 + col) >> 1)) * kPairBytes) + (col & 1);
+    p[0] = d;
+    p[2] = (float)v;
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < kPreCols * 32; q += 256) {
+    const int col = q & (kPreCols - 1), ch = q >> 6;               // chunk ch of 8 K positions
+    const int n = ch >> 4, w = (ch >> 1) & 7, c = ch & 1;
+    const uint8_t* s = t8 + col * kPreRow + 128 * n + 64 * c + 4 * w;
+    const __half2 bias = __float2half2_rn(-1152.0f - (float)mean[col]);   // (x ^ 0x80) | 0x6400 is 1152 + x
+    auto halves = [&](uint32_t word, uint32_t& even, uint32_t& odd) {     // four int8 -> f16 {0, 2}, {1, 3}
+      const uint32_t u = word ^ 0x80808080u;
+      even = h2_bits(__hadd2(bits_h2((u & 0x00ff00ffu) | 0x64006400u), bias));
+      odd = h2_bits(__hadd2(bits_h2(((u >> 8) & 0x00ff00ffu) | 0x64006400u), bias));
+    };
+    uint4 o;
+    halves(*reinterpret_cast<const uint32_t*>(s), o.x, o.y);
+    halves(*reinterpret_cast<const uint32_t*>(s + 32), o.z, o.w);
+    uint8_t* dst = x + ((size_t)(4 * kb + (ch >> 3)) * (npad >> 3) + ((c0 + col) >> 3)) * kAtomBytes + (col & 7) * 128 + (((ch ^ col) & 7) << 4);
+    *reinterpret_cast<uint4*>(dst) = o;
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 1) gemm_q4k_tc_kernel(const GemmArgs p) {
+// pre-pass over the weights, for products of several column tiles: the mins as the msum instruction's A operand, and d, -dmin
+// and T = sum q * sc of every row and super-block, which the producers would else work out anew for each column tile.
+// grid (K/256, ceil(M/128)), 128 threads; rows past M repeat the last one
+__global__ void __launch_bounds__(128) q4k_table_kernel(const uint8_t* W, int64_t row_bytes, int M, uint8_t* table) {
+  __shared__ __align__(16) uint8_t blocks[BM * Q4_K_BYTES];
+  const int kb = blockIdx.x, r0 = blockIdx.y * BM, t = threadIdx.x;
+#pragma unroll
+  for (int j = 0; j < 9; ++j) {
+    const int g = t + BM * j, rr = g / 9, part = g - 9 * rr;
+    *reinterpret_cast<uint4*>(blocks + 16 * g) =
+        *reinterpret_cast<const uint4*>(W + (size_t)min(r0 + rr, M - 1) * row_bytes + (size_t)kb * Q4_K_BYTES + 16 * part);
+  }
+  __syncthreads();
+  const uint4* blk = reinterpret_cast<const uint4*>(blocks + t * Q4_K_BYTES);
+  const uint4 h = blk[0];
+  const uint32_t sc[2] = {h.y & 0x3f3f3f3fu, (h.w & 0x0f0f0f0fu) | (((h.y >> 6) & 0x03030303u) << 4)};
+  const uint32_t mn[2] = {h.z & 0x3f3f3f3fu, ((h.w >> 4) & 0x0f0f0f0fu) | (((h.z >> 6) & 0x03030303u) << 4)};
+  int total = 0;
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {          // sub-blocks 2g (low nibbles), 2g + 1
+    int lo = 0, hi = 0;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint4 v = blk[1 + 2 * g + i];
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        lo = __dp4a(w[k] & 0x0f0f0f0fu, 0x01010101u, (unsigned)lo);
+        hi = __dp4a((w[k] >> 4) & 0x0f0f0f0fu, 0x01010101u, (unsigned)hi);
+      }
+    }
+    const uint32_t s = sc[g >> 1] >> (16 * (g & 1));
+    total += (int)(s & 0xffu) * lo + (int)((s >> 8) & 0xffu) * hi;
+  }
+  uint8_t* out = table + ((size_t)blockIdx.y * gridDim.x + kb) * kTableBytes;
+#pragma unroll
+  for (int n = 0; n < 2; ++n) {
+    __half2 m[4];
+#pragma unroll
+    for (int f = 0; f < 4; ++f) m[f] = __half2half2(__ushort2half_rn((unsigned short)((mn[n] >> (8 * f)) & 0xffu)));
+    *reinterpret_cast<uint4*>(out + n * (BM * 16) + t * 16) = *reinterpret_cast<const uint4*>(m);
+  }
+  const float d = h2f((uint16_t)(h.x & 0xffffu)), dm = -h2f((uint16_t)(h.x >> 16)), tt = (float)total;
+  float2* row = reinterpret_cast<float2*>(out + kMinsBytes + t * kTableRow);
+  row[0] = make_float2(d, d);
+  row[1] = make_float2(dm, dm);
+  row[2] = make_float2(tt, tt);
+}
+
+template <int TN, bool kTable>
+__global__ void __launch_bounds__(kThreads, 1) gemm_q4k_tc_kernel(const GemmArgs p, const __grid_constant__ CUtensorMap wmap) {
+  using C = Cfg<TN, kTable>;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
-  uint8_t* meta = smem + kStages * kStageBytes;
-  uint8_t* raw = meta + kMetaSlots * kMetaBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(raw + kRawBytes);
-  uint64_t* full = bars;            // [2] producers + bulk copies -> MMA: operands of a super-block are in shared memory
-  uint64_t* mma_done = bars + 2;    // [2] MMA -> producers: the operand stage may be overwritten
-  uint64_t* tmem_full = bars + 4;   // [2] MMA -> epilogue: the accumulator pair holds a finished super-block
-  uint64_t* epi_done = bars + 6;    // [2] epilogue -> MMA (accumulator pair free) and producers (scale slot free)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* raw = smem + C::kOffRaw;
+  uint8_t* mins = smem + C::kOffMins;
+  uint8_t* rowmeta = smem + C::kOffRowMeta;
+  uint8_t* meta = smem + C::kOffMeta;
+  // barriers, by their shared memory addresses
+  const uint32_t bars = smem_u32(smem + C::kOffBars);
+  const uint32_t h_full = bars;                       // [turns][4 quarters] producers and bulk copies -> MMA; the last quarter brings the meta slot
+  const uint32_t h_free = h_full + 8 * 4 * C::kTurns; // MMA -> producers and loader
+  const uint32_t r_full = h_free + 8 * 4 * C::kTurns; // [raw slots] TMA -> producers: the weights of a super-block
+  const uint32_t r_free = r_full + 8 * C::kRawSlots;
+  const uint32_t m_free = r_free + 8 * C::kRawSlots;  // [3] epilogue -> loader: the meta slot is read
+  const uint32_t s_full = m_free + 8 * kMetaSlots;  // [parts] msum warp -> epilogue: the part's accumulators and msum are complete
+  const uint32_t s_free = s_full + 8 * 2;           // [parts] epilogue -> msum warp: they are read
+  const uint32_t d_full = s_free + 8 * 2;           // [2 turns] MMA -> msum warp: the accumulators are complete
+  const uint32_t d_free = d_full + 8 * 2;           // [2 turns] epilogue -> MMA: they are read
+  const uint32_t drained = d_free + 8 * 2;          // [2] only after a wait that gave up
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::kOffBars + 8 * 60);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // from one lane: the compiler then keeps what follows from it in uniform registers (TMEM addresses, barriers, pointers)
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(full + s, kProducerThreads + 1);
-      mbar_init(mma_done + s, 1);
-      mbar_init(tmem_full + s, 1);
-      mbar_init(epi_done + s, kEpilogueWarps);
+    for (int s = 0; s < C::kRawSlots; ++s) { mbar_init(r_full + 8 * s, 1); mbar_init(r_free + 8 * s, 8); }
+    for (int s = 0; s < 4 * C::kTurns; ++s) { mbar_init(h_full + 8 * s, (s & 3) == 3 ? 6 : 5); mbar_init(h_free + 8 * s, 1); }
+    for (int s = 0; s < kMetaSlots; ++s) mbar_init(m_free + 8 * s, kEpilogueWarps);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(s_full + 8 * s, 1);
+      mbar_init(s_free + 8 * s, kEpilogueWarps);
+      mbar_init(d_full + 8 * s, 1);
+      mbar_init(d_free + 8 * s, kEpilogueWarps);
+      mbar_init(drained + 8 * s, 1);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -252,306 +278,495 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q4k_tc_kernel(const GemmArgs
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  fence_before();
   __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = *tmem_slot;
+  fence_after();
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
-  const int mt = (p.M + BM - 1) / BM, nt = (p.N + BN - 1) / BN, ntiles = mt * nt, nkb = p.K / QK_K;
+  const int mt = (p.M + BM - 1) / BM, nt = (p.N + TN - 1) / TN, ntiles = mt * nt, nkb = p.K / QK_K;
+  const int my_tiles = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  const int turns = my_tiles * nkb;   // super-blocks this CTA walks
 
-  if (warp < 4) {
+  if (warp < 8) {
     // ---------------------------------------------------------------- producers
-    const int t = threadIdx.x;  // row t of the weight tile
-    const uint32_t core_off = (uint32_t)(t >> 3) * kGroupStride + (uint32_t)(t & 7) * 16;
-    // raw staging of iteration (tile, kb): 1152 16-byte pieces, piece g = (row g/9, part g%9) lands at g*16
-    auto issue_raw = [&](int tile, int kb) {
-      const int tm = tile / nt;
-      const uint32_t rbase = smem_u32(raw);
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kProducerRegs));
+    const int quarter = warp & 3, n = warp >> 2;   // TMEM lanes 32 * quarter .., half n of every super-block
+    const uint32_t a_lane = tmem_base + C::kTmemA + ((uint32_t)(32 * quarter) << 16) + 64u * n;
+    const uint32_t low = in_register(0x000f000fu), high = in_register(0x00f000f0u), k1024 = in_register(0x64006400u);
+    int slot = 0, mslot = 0, rslot = 0;
+    uint32_t rphase = 0;
+    bool live = true;
+    for (int it = 0; it < turns; ++it) {
+      live = mbar_wait(r_full + 8 * slot, rphase, abort_flag);
+      live = __all_sync(0xffffffffu, live);
+      if (!live) break;
+      const int buf = it & 1, hb = 4 * (it & (C::kTurns - 1)) + 2 * n;
+      const uint8_t* blk = raw + slot * kRawBytes + (32 * quarter + lane) * Q4_K_BYTES;
+      const uint4 h = *reinterpret_cast<const uint4*>(blk);
+      const uint32_t scw = n ? (h.w & 0x0f0f0f0fu) | (((h.y >> 6) & 0x03030303u) << 4) : h.y & 0x3f3f3f3fu;   // of sub-blocks 4n .. 4n+3
+      const uint32_t mnw = n ? ((h.w >> 4) & 0x0f0f0f0fu) | (((h.z >> 6) & 0x03030303u) << 4) : h.z & 0x3f3f3f3fu;
+      const __half2 bias = __float2half2_rn(-1024.0f);
+      __half2 s[4], c[4];    // even sub-blocks {sc, -1024 sc}, odd ones {sc / 16, -64 sc}
 #pragma unroll
-      for (int j = 0; j < 9; ++j) {
-        const int g = t + 128 * j;
-        const int rr = g / 9, part = g - 9 * rr;
-        const int row = min(tm * BM + rr, p.M - 1);           // rows past M repeat the last one; never stored
-        const uint8_t* src = p.W + (size_t)row * p.row_bytes + (size_t)kb * Q4_K_BYTES + 16 * part;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(rbase + 16u * (uint32_t)g), "l"(src) : "memory");
+      for (int f = 0; f < 4; ++f) {
+        const __half2 sc = __hadd2(bits_h2(__byte_perm(scw, 0x64646464u, 0x4040 | (f * 0x0101))), bias);
+        s[f] = f & 1 ? __hmul2(sc, __float2half2_rn(0.0625f)) : sc;
+        c[f] = __hmul2(sc, __float2half2_rn(f & 1 ? -64.0f : -1024.0f));
       }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    // One flat loop over (tile, super-block).  The 128 producers meet at named barriers every
-    // iteration, so nobody leaves early: a wait that gave up only skips work, and the loop ends
-    // for everyone at the abort check right after a barrier.
-    int it = 0, tile = blockIdx.x, kb = 0;
-    if (tile < ntiles) issue_raw(tile, 0);
-    for (; tile < ntiles; ++it) {
-      const int tn = tile % nt;
-      const int s = it & 1, m = it & (kMetaSlots - 1);
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-      asm volatile("bar.sync 1, 128;" ::: "memory");          // everybody's pieces of this iteration's raw blocks landed
-      uint4 blk[9];
+      uint32_t sum[4] = {0u, 0u, 0u, 0u};   // of the masked words: 16 exponents and the quants of either lane
+      auto expand = [&](int w, uint32_t* o, const uint4& a, const uint4& b) {   // words w & 3 of a (sub-blocks 4n, 4n+1) and b (4n+2, 4n+3)
+        const uint32_t av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-      for (int i = 0; i < 9; ++i) blk[i] = *reinterpret_cast<const uint4*>(raw + t * Q4_K_BYTES + 16 * i);
-      asm volatile("bar.sync 1, 128;" ::: "memory");          // everybody has read: the staging buffer is free
-      if (*abort_flag) break;
-      int ntile = tile, nkbi = kb + 1;
-      if (nkbi == nkb) { nkbi = 0; ntile += gridDim.x; }
-      if (ntile < ntiles) issue_raw(ntile, nkbi);
-      // operand stage s was consumed by the MMAs of iteration it-2; those were issued after the epilogue of
-      // it-4 had finished, which is the last reader of scale slot m
-      const bool ok = mbar_wait(mma_done + s, ((it >> 1) & 1) ^ 1, abort_flag);
-      if (ok) {
-        uint8_t* st = smem + s * kStageBytes;
-        uint8_t* mt_ = meta + m * kMetaBytes;
-        // weights of row t: scales, then the two int8 operands
-        const uint4 h = blk[0];
-        const uint32_t s0 = h.y, s1 = h.z, s2 = h.w;
-        const uint32_t sc_lo4 = s0 & 0x3f3f3f3fu, mn_lo4 = s1 & 0x3f3f3f3fu;
-        const uint32_t sc_hi4 = (s2 & 0x0f0f0f0fu) | (((s0 >> 6) & 0x03030303u) << 4);
-        const uint32_t mn_hi4 = ((s2 >> 4) & 0x0f0f0f0fu) | (((s1 >> 6) & 0x03030303u) << 4);
-        {
-          uint32_t* rmw = reinterpret_cast<uint32_t*>(mt_ + kOffRowMeta + t * kRowMetaBytes);
-          rmw[0] = h.x;
-          rmw[1] = mn_lo4;
-          rmw[2] = mn_hi4;
+        for (int e = 0; e < 2; ++e) {
+          const uint32_t u = e ? bv[w] : av[w], u8 = u >> 8;
+          const uint32_t l0 = mask_or(u, low, k1024), l1 = mask_or(u8, low, k1024), h0 = mask_or(u, high, k1024), h1 = mask_or(u8, high, k1024);
+          if constexpr (!kTable) {
+            sum[2 * e] += l0 + l1;
+            sum[2 * e + 1] += h0 + h1;
+          }
+          o[4 * e + 0] = expand2(l0, s[2 * e], c[2 * e]);
+          o[4 * e + 1] = expand2(l1, s[2 * e], c[2 * e]);
+          o[4 * e + 2] = expand2(h0, s[2 * e + 1], c[2 * e + 1]);
+          o[4 * e + 3] = expand2(h1, s[2 * e + 1], c[2 * e + 1]);
         }
-        uint8_t* alo = st + kOffW + core_off;                  // operand rows 0-127: q*lo
-        uint8_t* ahi = alo + kChunkStride;                     // operand rows 128-255: q*hi (16 core-matrix groups further)
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          const uint4 v0 = blk[1 + 2 * g], v1 = blk[2 + 2 * g];
-          const uint32_t scw = g < 2 ? sc_lo4 : sc_hi4;
-          const uint32_t sca = (scw >> (16 * (g & 1))) & 0xffu, scb = (scw >> (16 * (g & 1) + 8)) & 0xffu;
-          const uint32_t la = sca & 7u, ha = sca >> 3, lb = scb & 7u, hb = scb >> 3;
-          const uint32_t q[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-          uint32_t lo[8], hi[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) { lo[i] = q[i] & 0x0f0f0f0fu; hi[i] = (q[i] >> 4) & 0x0f0f0f0fu; }
-          // sub-block 2g (low nibbles): chunks 4g, 4g+1; sub-block 2g+1 (high nibbles): chunks 4g+2, 4g+3
-          *reinterpret_cast<uint4*>(alo + (4 * g + 0) * kChunkStrideW) = make_uint4(lo[0] * la, lo[1] * la, lo[2] * la, lo[3] * la);
-          *reinterpret_cast<uint4*>(alo + (4 * g + 1) * kChunkStrideW) = make_uint4(lo[4] * la, lo[5] * la, lo[6] * la, lo[7] * la);
-          *reinterpret_cast<uint4*>(alo + (4 * g + 2) * kChunkStrideW) = make_uint4(hi[0] * lb, hi[1] * lb, hi[2] * lb, hi[3] * lb);
-          *reinterpret_cast<uint4*>(alo + (4 * g + 3) * kChunkStrideW) = make_uint4(hi[4] * lb, hi[5] * lb, hi[6] * lb, hi[7] * lb);
-          *reinterpret_cast<uint4*>(ahi + (4 * g + 0) * kChunkStrideW) = make_uint4(lo[0] * ha, lo[1] * ha, lo[2] * ha, lo[3] * ha);
-          *reinterpret_cast<uint4*>(ahi + (4 * g + 1) * kChunkStrideW) = make_uint4(lo[4] * ha, lo[5] * ha, lo[6] * ha, lo[7] * ha);
-          *reinterpret_cast<uint4*>(ahi + (4 * g + 2) * kChunkStrideW) = make_uint4(hi[0] * hb, hi[1] * hb, hi[2] * hb, hi[3] * hb);
-          *reinterpret_cast<uint4*>(ahi + (4 * g + 3) * kChunkStrideW) = make_uint4(hi[4] * hb, hi[5] * hb, hi[6] * hb, hi[7] * hb);
+      };
+      // a quarter's columns are free once the MMAs of the turn that used them last are done.  Not unrolled: six roles'
+      // instructions share the caches
+      const int prev = it - C::kOperands;
+#pragma unroll 1
+      for (int e = 0; e < 2; ++e) {
+        const uint8_t* quants = blk + 16 + 64 * n + 16 * e;
+        const uint4 a = *reinterpret_cast<const uint4*>(quants), b = *reinterpret_cast<const uint4*>(quants + 32);
+        if (e == 1) {                          // the slot is read
+          __syncwarp();
+          mbar_arrive_if(lane == 0, r_free + 8 * slot);
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy writes -> visible to the tensor core's reads
-        mbar_arrive(full + s);
+        uint32_t o[32];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) expand(w, o + 8 * w, a, b);
+        live = prev < 0 || mbar_wait(h_free + 8 * (4 * (prev & (C::kTurns - 1)) + 2 * n + e), (uint32_t)(prev / C::kTurns) & 1u, abort_flag);
+        live = __all_sync(0xffffffffu, live);
+        if (!live) break;
+        fence_after();
+        tmem_st32(a_lane + (C::kOperands == 2 ? 128u * buf : 0u) + 32u * e, o);
+        if (!kTable && e == 1) {
+          // row meta: the slot's last readers, the epilogue of the turn two before prev, were done before the MMAs of prev
+          // could be issued, and so were the mins' last readers, that turn's msum instructions
+          {
+            float t = 0.0f;
+#pragma unroll
+            for (int f = 0; f < 4; ++f) {
+              const uint32_t pair = sum[f] - 16u * 0x64006400u;
+              const int q = (int)((pair & 0xffffu) + (pair >> 16));
+              t += (float)(((int)(scw >> (8 * f)) & 0xff) * (f & 1 ? q >> 4 : q));
+            }
+            uint8_t* rm = rowmeta + (rslot * BM + 32 * quarter + lane) * kRowMeta;
+            if (n == 0) {
+              const float d = h2f((uint16_t)(h.x & 0xffffu)), dm = -h2f((uint16_t)(h.x >> 16));
+              *reinterpret_cast<float4*>(rm) = make_float4(d, d, dm, dm);
+            }
+            *reinterpret_cast<float2*>(rm + 16 + 8 * n) = make_float2(t, t);
+            uint4 mv;
+            mv.x = h2_bits(__hadd2(bits_h2(__byte_perm(mnw, 0x64646464u, 0x4040)), bias));
+            mv.y = h2_bits(__hadd2(bits_h2(__byte_perm(mnw, 0x64646464u, 0x4141)), bias));
+            mv.z = h2_bits(__hadd2(bits_h2(__byte_perm(mnw, 0x64646464u, 0x4242)), bias));
+            mv.w = h2_bits(__hadd2(bits_h2(__byte_perm(mnw, 0x64646464u, 0x4343)), bias));
+            *reinterpret_cast<uint4*>(mins + mslot * kMinsBytes + n * (BM * 16) + (32 * quarter + lane) * 16) = mv;
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the mins -> visible to the tensor core's reads
+        }
+        tmem_wait_st();
+        fence_before();
+        __syncwarp();
+        mbar_arrive_if(lane == 0, h_full + 8 * (hb + e));
       }
-      tile = ntile;
-      kb = nkbi;
+      if (!live) break;
+      if (++slot == C::kRawSlots) { slot = 0; rphase ^= 1u; }
+      if (++mslot >= C::kMinsSlots) mslot = 0;
+      if (++rslot >= C::kRowMetaSlots) rslot = 0;
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-  } else if (warp == kMmaWarp) {
-    // ---------------------------------------------------------------- MMA issue (one thread)
-    if (lane == 0) {
-      int it = 0, last_commit = -1;
-      bool live = true;
-      for (int tile = blockIdx.x; live && tile < ntiles; tile += gridDim.x) {
-        for (int kb = 0; kb < nkb; ++kb, ++it) {
-          const int s = it & 1;
-          // operands in place, and the accumulator pair drained by the epilogue of iteration it-2
-          if (!mbar_wait(full + s, (it >> 1) & 1, abort_flag)) { live = false; break; }
-          if (!mbar_wait(epi_done + s, ((it >> 1) & 1) ^ 1, abort_flag)) { live = false; break; }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          uint8_t* st = smem + s * kStageBytes;
-          const uint32_t xop = smem_u32(st + kOffX), wop = smem_u32(st + kOffW);
-          const uint32_t d_acc = tmem_base + (uint32_t)s * 256u;   // columns 0-127: D_lo, 128-255: D_hi
+  } else if (warp >= kMmaWarp) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kOtherRegs));
+    // One lane issues, but the whole warp walks the loops, so that descriptors and addresses are worked out in uniform
+    // registers.  D = f32, A = B = f16, both K-major, M = 128 weight rows, N = columns
+    constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(BM >> 4) << 24);
+    const bool leader = elect_one();
+    bool live = true;
+    if (warp == kMmaWarp) {
+      // -------------------------------------------------------------- accumulators: 16 instructions a turn
+      constexpr uint32_t kIdescD = kIdesc | ((uint32_t)(TN >> 3) << 17);
+      const uint64_t x0 = operand_desc(smem_u32(smem), kAtomBytes);
+#pragma unroll 1
+      for (int it = 0; it < turns; ++it) {
+        const int buf = it & 1;
+        const uint32_t d = tmem_base + (uint32_t)(TN * buf), phase = (uint32_t)(it >> 1) & 1u;
+        live = mbar_wait(d_free + 8 * buf, phase ^ 1u, abort_flag);
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+          const int hq = 4 * (it & (C::kTurns - 1)) + q;
+          live = live && mbar_wait(h_full + 8 * hq, (uint32_t)(it / C::kTurns) & 1u, abort_flag);
+          live = __all_sync(0xffffffffu, live);
+          if (!live) break;
+          fence_after();
+          const uint64_t x = x0 + (uint64_t)(hq * (C::kQuarterBytes >> 4));
+          const uint32_t a_op = tmem_base + C::kTmemA + (C::kOperands == 2 ? 128u * buf : 0u) + 32u * q;
+          if (leader) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            mma_i8(d_acc, operand_desc(xop + 2 * j * kChunkStride, kChunkStride), operand_desc(wop + 2 * j * kChunkStrideW, kChunkStrideW),
-                   j > 0 ? 1u : 0u);
-          mma_commit(mma_done + s);
-          mma_commit(tmem_full + s);
-          last_commit = it;
+            for (int j = 0; j < 4; ++j) mma_f16(d, a_op + 8u * j, x + (uint64_t)(2 * j), kIdescD, (q | j) ? 1u : 0u);
+            mma_commit(h_free + 8 * hq);
+            if (q == 3) mma_commit(d_full + 8 * buf);
+          }
+          __syncwarp();
+        }
+        if (!live) break;
+      }
+    } else if (warp == kSumWarp) {
+      // -------------------------------------------------------------- msum: one instruction a part.  The accumulators have two
+      // buffers, a part's msum one: made when the epilogue has read the part of the turn before
+      constexpr uint32_t kIdescS = kIdesc | ((uint32_t)(C::kPart >> 3) << 17);
+      const uint64_t sums0 = plain_desc(smem_u32(meta), TN * 16);
+      const uint64_t mins0 = plain_desc(smem_u32(kTable ? meta + C::kOffTable : mins), BM * 16);
+      int ms = 0, mslot = 0;
+#pragma unroll 1
+      for (int it = 0; it < turns; ++it) {
+        live = mbar_wait(d_full + 8 * (it & 1), (uint32_t)(it >> 1) & 1u, abort_flag);
+#pragma unroll 1
+        for (int s = 0; s < C::kParts; ++s) {
+          live = live && mbar_wait(s_free + 8 * s, ((uint32_t)it & 1u) ^ 1u, abort_flag);
+          live = __all_sync(0xffffffffu, live);
+          if (!live) break;
+          fence_after();
+          if (leader) {
+            mma_f16_ss(tmem_base + C::kTmemM + (uint32_t)(s * C::kPart), mins0 + (uint64_t)((kTable ? ms * C::kMetaBytes : mslot * kMinsBytes) >> 4),
+                       sums0 + (uint64_t)((ms * C::kMetaBytes + s * C::kPart * 16) >> 4), kIdescS);
+            mma_commit(s_full + 8 * s);
+          }
+          __syncwarp();
+        }
+        if (!live) break;
+        if (++ms == kMetaSlots) ms = 0;
+        if (++mslot >= C::kMinsSlots) mslot = 0;
+      }
+    } else if (warp == kLoaderWarp) {
+      // -------------------------------------------------------------- activations, a quarter super-block a copy, and weights
+      const size_t stride = (size_t)(p.npad >> 3) * kAtomBytes;
+      int kb = 0, tile = blockIdx.x, it = 0;
+      const uint8_t* src = p.x + (size_t)((tile % nt) * (TN / 8)) * kAtomBytes;
+      int wkb = 0, wtile = blockIdx.x, wslot = 0, asked = 0;
+      uint32_t wphase = 1u;
+      auto weights = [&]() {                   // of the next turn not asked for yet
+        if (asked >= turns) return true;
+        bool ok = mbar_wait(r_free + 8 * wslot, wphase, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok && leader) {
+          mbar_arrive_expect_tx(r_full + 8 * wslot, kRawBytes);
+          tma_load_2d(raw + wslot * kRawBytes, &wmap, wkb * Q4_K_BYTES, wtile / nt * BM, r_full + 8 * wslot);
+        }
+        __syncwarp();
+        ++asked;
+        if (++wslot == C::kRawSlots) { wslot = 0; wphase ^= 1u; }
+        if (++wkb == nkb) { wkb = 0; wtile += gridDim.x; }
+        return ok;
+      };
+      for (int i = 0; i < C::kRawSlots - 1; ++i) live = live && weights();
+#pragma unroll 1
+      for (; live && it < turns; ++it) {
+        live = weights();
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+          const int hq = 4 * (it & (C::kTurns - 1)) + q;
+          const uint32_t full = h_full + 8 * hq;
+          live = live && mbar_wait(h_free + 8 * hq, ((uint32_t)(it / C::kTurns) & 1u) ^ 1u, abort_flag);
+          live = __all_sync(0xffffffffu, live);
+          if (!live) break;
+          if (leader) {
+            mbar_arrive_expect_tx(full, C::kQuarterBytes);
+            bulk_g2s(smem + hq * C::kQuarterBytes, src, C::kQuarterBytes, full);
+          }
+          __syncwarp();
+          src += stride;
+        }
+        if (++kb == nkb) {
+          kb = 0;
+          tile += gridDim.x;
+          src = p.x + (size_t)((tile % nt) * (TN / 8)) * kAtomBytes;
         }
       }
-      if (!live && last_commit >= 0) {
-        // gave up: let the tensor core finish what was issued before the TMEM goes away (bounded)
-        uint64_t* bar = tmem_full + (last_commit & 1);
-        const uint32_t parity = (last_commit >> 1) & 1;
-        for (int spins = 0; spins < (1 << 20) && !mbar_try_wait(bar, parity); ++spins) {}
-      }
-    }
-  } else if (warp == kLoaderWarp) {
-    // ---------------------------------------------------------------- activation tile loader (one thread)
-    if (lane == 0) {
-      int it = 0;
-      bool live = true;
-      for (int tile = blockIdx.x; live && tile < ntiles; tile += gridDim.x) {
-        const int tn = tile % nt;
-        for (int kb = 0; kb < nkb; ++kb, ++it) {
-          const int s = it & 1;
-          if (!mbar_wait(mma_done + s, ((it >> 1) & 1) ^ 1, abort_flag)) { live = false; break; }
-          uint8_t* st = smem + s * kStageBytes;
-          uint8_t* mt_ = meta + (it & (kMetaSlots - 1)) * kMetaBytes;
-          const uint8_t* tile_src = p.tiles + ((size_t)tn * nkb + kb) * kTileBytes;
-          mbar_arrive_expect_tx(full + s, kTileBytes);
-#pragma unroll
+      if (!live && leader) {
+        // gave up: let the copies in flight land (bounded).  A quarter's barrier also counts producers, who may have gone:
+        // the copies' landing shows in its phase only if all came, so this waits out its bound otherwise
+        for (int i = max(0, it - C::kTurns); i <= it; ++i)
           for (int q = 0; q < 4; ++q)
-            bulk_g2s(st + kOffX + q * (kOperandBytes / 4), tile_src + q * (kOperandBytes / 4), kOperandBytes / 4, full + s);
-          bulk_g2s(mt_ + kOffColMeta, tile_src + kOperandBytes, kColMetaBytes, full + s);
-          // the tile this stage gets next (two super-blocks ahead, same tile row while kb + 2 < nkb) towards L2:
-          // the copy above is issued only when the stage frees up, so its latency is on the critical path
-          if (kb + 2 < nkb)
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(tile_src + 2 * (size_t)kTileBytes), "r"(kTileBytes) : "memory");
+            for (int spins = 0; spins < (1 << 14) && !mbar_try_wait(h_full + 8 * (4 * (i & (C::kTurns - 1)) + q), (uint32_t)(i / C::kTurns) & 1u); ++spins) {}
+        for (int i = max(0, asked - C::kRawSlots); i < asked; ++i)
+          for (int spins = 0; spins < (1 << 14) && !mbar_try_wait(r_full + 8 * (i % C::kRawSlots), (uint32_t)(i / C::kRawSlots) & 1u); ++spins) {}
+      }
+    } else {
+      // -------------------------------------------------------------- block sums, scales and table of a super-block
+      int kb = 0, tile = blockIdx.x, it = 0, ms = 0;
+      uint32_t phase = 1u;
+#pragma unroll 1
+      for (; it < turns; ++it) {
+        const int hq = 4 * (it & (C::kTurns - 1)) + 3;
+        const uint32_t full = h_full + 8 * hq;
+        live = mbar_wait(m_free + 8 * ms, phase, abort_flag);
+        // the barrier's phase before this one is over once the accumulators of turn it - kTurns are complete
+        live = live && mbar_wait(h_free + 8 * hq, ((uint32_t)(it / C::kTurns) & 1u) ^ 1u, abort_flag);
+        live = __all_sync(0xffffffffu, live);
+        if (!live) break;
+        if (leader) {
+          const int tm = tile / nt, c0 = (tile - tm * nt) * TN;
+          uint8_t* cm = meta + ms * C::kMetaBytes;
+          mbar_arrive_expect_tx(full, C::kMetaBytes);
+#pragma unroll
+          for (int c = 0; c < 2; ++c) bulk_g2s(cm + c * TN * 16, p.sums + (((size_t)kb * 2 + c) * p.npad + c0) * 16, TN * 16, full);
+          bulk_g2s(cm + C::kOffPairs, p.pairs + ((size_t)kb * (p.npad >> 1) + (c0 >> 1)) * kPairBytes, TN / 2 * kPairBytes, full);
+          if (kTable) bulk_g2s(cm + C::kOffTable, p.table + ((size_t)tm * nkb + kb) * kTableBytes, kTableBytes, full);
         }
+        __syncwarp();
+        if (++ms == kMetaSlots) { ms = 0; phase ^= 1u; }
+        if (++kb == nkb) { kb = 0; tile += gridDim.x; }
+      }
+      if (!live && leader) {
+        for (int i = max(0, it - C::kTurns); i <= it; ++i)
+          for (int spins = 0; spins < (1 << 14) && !mbar_try_wait(h_full + 8 * (4 * (i & (C::kTurns - 1)) + 3), (uint32_t)(i / C::kTurns) & 1u); ++spins) {}
       }
     }
+    if (warp <= kSumWarp && !live && leader) {
+      // gave up: let the tensor core finish what was issued before the TMEM goes away (bounded)
+      const uint32_t mine = drained + 8 * (warp - kMmaWarp);
+      mma_commit(mine);
+      for (int spins = 0; spins < (1 << 16) && !mbar_try_wait(mine, 0u); ++spins) {}
+    }
+    __syncwarp();
   } else {
     // ---------------------------------------------------------------- epilogue
-    // TMEM lanes are tokens, TMEM columns weight rows.  The warp owns 32 tokens (its lane quarter) x 32 weight
-    // rows.  Accumulators are read in the 16x256b shape, whose register layout is the m16n8 C fragment: thread
-    // (g = lane/4, t = lane%4) holds tokens g and g+8, weight rows 2t and 2t+1 of every 8-row block.
-    // msum = sum_j bsum_j * m_j for the same elements comes from one legacy-path mma.sync per (16 tokens x 8
-    // weight rows): A = the token's block sums split as lo + 128*hi, B = the weight row's 8 mins (twice), so
-    // every f16 operand and every f32 partial sum is an exact integer.
-    const int quarter = warp & 3;                       // the TMEM lanes this warp may read: tokens 32*quarter ..
-    const int cgroup = (warp - kEpilogueWarp0) >> 2;    // weight rows 32*cgroup .. 32*cgroup+31
-    const int g = lane >> 2, t = lane & 3;
-    int it = 0;
+    // TMEM lanes are weight rows, TMEM columns the product's columns.  The warp owns 32 rows (its lane quarter) and of every
+    // column part one half, a thread one row: its d, -dmin and T stay in registers, the columns' dx and v come as
+    // broadcasts.  (TMEM loads of whole lanes take half a cycle a register, those in the m16n8 fragment layout two.)
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kEpilogueRegs));
+    constexpr int kMine = C::kPart / 2, kLoads = kMine / 8;        // columns of a part; loads of eight
+    const int quarter = warp & 3, side = (warp - kEpilogueWarp0) >> 2;
+    const uint32_t tb = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(kMine * side), lead = lane == 0;
+    int ms = 0, rslot = 0, it = 0;
     bool live = true;
     for (int tile = blockIdx.x; live && tile < ntiles; tile += gridDim.x) {
-      const int tm = tile / nt, tn = tile - tm * nt;
-      float acc[4][4][2];   // [token g + 8*j][8-row block][weight row 2t + e]
+      f2 acc[C::kParts][kLoads][4];       // [part][load][column pair]
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int nb = 0; nb < 4; ++nb) acc[j][nb][0] = acc[j][nb][1] = 0.0f;
+      for (int i = 0; i < 4 * kLoads * C::kParts; ++i) acc[i / (4 * kLoads)][(i >> 2) % kLoads][i & 3] = 0ull;
+#pragma unroll 1
       for (int kb = 0; kb < nkb; ++kb, ++it) {
-        const int s = it & 1;
-        if (!mbar_wait(tmem_full + s, (it >> 1) & 1, abort_flag)) { live = false; break; }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint8_t* mt_ = meta + (it & (kMetaSlots - 1)) * kMetaBytes;
-        const uint8_t* tokmeta = mt_ + kOffColMeta + (32 * quarter) * 16;                       // per token: 8 lo, 8 hi parts
-        const float* dxs = reinterpret_cast<const float*>(mt_ + kOffDx) + 32 * quarter;          // per token: dx
-        const uint8_t* wmeta = mt_ + kOffRowMeta + (32 * cgroup) * kRowMetaBytes;                // per weight row: {d, dmin}, mins
-        // B fragments of the four 8-row blocks: weight row g of the block, mins 2t and 2t+1
-        uint32_t bfm[4];
+        const uint8_t* cm = meta + ms * C::kMetaBytes + C::kOffPairs + kMine / 2 * side * kPairBytes;
+        const uint8_t* rmeta = kTable ? meta + ms * C::kMetaBytes + C::kOffTable + kMinsBytes + (32 * quarter + lane) * kTableRow
+                                      : rowmeta + (rslot * BM + 32 * quarter + lane) * kRowMeta;
+        const uint32_t parity = (uint32_t)it & 1u;
+        f2 dw, ndm, tq;          // d, -dmin, T of the row, each twice
 #pragma unroll
-        for (int nb = 0; nb < 4; ++nb) {
-          const uint32_t m2 = *reinterpret_cast<const uint16_t*>(wmeta + (8 * nb + g) * kRowMetaBytes + 4 + 2 * t);
-          const __half2 fm = __halves2half2(__ushort2half_rn((unsigned short)(m2 & 0xffu)), __ushort2half_rn((unsigned short)(m2 >> 8)));
-          bfm[nb] = *reinterpret_cast<const uint32_t*>(&fm);
-        }
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          // tokens g + 16*hh and g + 8 + 16*hh: scale and the A fragments (block sums 2t, 2t+1: low parts, high parts)
-          float dx[2];
-          uint32_t afl[2], afh[2];
-#pragma unroll
-          for (int rr = 0; rr < 2; ++rr) {
-            const int tok = 16 * hh + 8 * rr + g;
-            dx[rr] = dxs[tok];
-            const uint32_t l2 = *reinterpret_cast<const uint16_t*>(tokmeta + tok * 16 + 2 * t);
-            const uint32_t h2 = *reinterpret_cast<const uint16_t*>(tokmeta + tok * 16 + 8 + 2 * t);
-            const __half2 fl = __halves2half2(__ushort2half_rn((unsigned short)(l2 & 0xffu)), __ushort2half_rn((unsigned short)(l2 >> 8)));
-            const __half2 fh = __halves2half2(__short2half_rn((short)((int)(int8_t)(h2 & 0xffu) * 128)),
-                                              __short2half_rn((short)((int)(int8_t)(h2 >> 8) * 128)));
-            afl[rr] = *reinterpret_cast<const uint32_t*>(&fl);
-            afh[rr] = *reinterpret_cast<const uint32_t*>(&fh);
+        for (int s = 0; s < C::kParts; ++s) {
+          const uint32_t td = tb + TN * parity + C::kPart * s, tm = tb + C::kTmemM + C::kPart * s;
+          // after a wait that gave up the turn's arithmetic is nonsense, which nobody stores
+          live = mbar_wait(s_full + 8 * s, parity, abort_flag) && live;
+          __syncwarp();
+          fence_after();
+          uint32_t dv[2][8], sv[2][8];
+          tmem_ld8(td, dv[0]);
+          tmem_ld8(tm, sv[0]);
+          if (s == 0) {
+            if constexpr (kTable) {
+              const f2* m = reinterpret_cast<const f2*>(rmeta);
+              dw = m[0];
+              ndm = m[1];
+              tq = m[2];
+            } else {
+              const ulonglong2 m = *reinterpret_cast<const ulonglong2*>(rmeta), tt = *reinterpret_cast<const ulonglong2*>(rmeta + 16);
+              dw = m.x;
+              ndm = m.y;
+              tq = add2(tt.x, tt.y);
+            }
           }
-          const uint32_t tbase = tmem_base + ((uint32_t)(32 * quarter + 16 * hh) << 16) + (uint32_t)s * 256u + (uint32_t)(32 * cgroup);
 #pragma unroll
-          for (int cp = 0; cp < 2; ++cp) {
-            uint32_t lo[8], hi[8];
-            tmem_ld_16x256b_x2(tbase + (uint32_t)(16 * cp), lo);
-            tmem_ld_16x256b_x2(tbase + 128u + (uint32_t)(16 * cp), hi);
-            float ms[2][4];
+          for (int i = 0; i < kLoads; ++i) {
+            tmem_wait_ld(dv[i & 1], sv[i & 1]);
+            if (i + 1 == kLoads) {
+              fence_before();
+              __syncwarp();
+              mbar_arrive_if(lead, s_free + 8 * s);
+              if (s + 1 == C::kParts) mbar_arrive_if(lead, d_free + 8 * parity);
+            } else {
+              tmem_ld8(td + 8u * (i + 1), dv[(i + 1) & 1]);
+              tmem_ld8(tm + 8u * (i + 1), sv[(i + 1) & 1]);
+            }
 #pragma unroll
-            for (int q2 = 0; q2 < 2; ++q2) mma_m16n8k16_f16(ms[q2], afl[0], afl[1], afh[0], afh[1], bfm[2 * cp + q2]);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int q2 = 0; q2 < 2; ++q2) {
-              const int nb = 2 * cp + q2;
-              const uint8_t* wm = wmeta + (8 * nb + 2 * t) * kRowMetaBytes;
-              const uint32_t db0 = *reinterpret_cast<const uint32_t*>(wm), db1 = *reinterpret_cast<const uint32_t*>(wm + kRowMetaBytes);
-              const float dw[2] = {h2f((uint16_t)(db0 & 0xffffu)), h2f((uint16_t)(db1 & 0xffffu))};
-              const float dminw[2] = {h2f((uint16_t)(db0 >> 16)), h2f((uint16_t)(db1 >> 16))};
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const int rr = e >> 1, ce = e & 1;
-                const int isum = (int)lo[4 * q2 + e] + 8 * (int)hi[4 * q2 + e];
-                const float d_all = __fmul_rn(dx[rr], dw[ce]), d_min = __fmul_rn(dx[rr], dminw[ce]);
-                const float bv = __fmaf_rn(d_all, (float)isum, -__fmul_rn(d_min, ms[q2][e]));
-                acc[2 * hh + rr][nb][ce] = __fadd_rn(acc[2 * hh + rr][nb][ce], bv);
-              }
+            for (int q = 0; q < 4; ++q) {
+              const ulonglong2 cv = *reinterpret_cast<const ulonglong2*>(cm + (C::kPart / 2 * s + 4 * i + q) * kPairBytes);   // dx, dx, v, v
+              const f2 isum = fma2(cv.y, tq, pack2u(dv[i & 1][2 * q], dv[i & 1][2 * q + 1]));
+              const f2 off = mul2(mul2(cv.x, ndm), pack2u(sv[i & 1][2 * q], sv[i & 1][2 * q + 1]));
+              acc[s][i][q] = add2(acc[s][i][q], fma2(mul2(cv.x, dw), isum, off));
             }
           }
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(epi_done + s);
+        live = __all_sync(0xffffffffu, live);
+        if (!live) break;
+        mbar_arrive_if(lead, m_free + 8 * ms);
+        if (++ms == kMetaSlots) ms = 0;
+        if (++rslot >= C::kRowMetaSlots) rslot = 0;
       }
       if (!live) break;
+      // rows leave through shared memory, 16 columns at a time, four lanes a row: 64 bytes of a row side by side (16 bytes
+      // of 32 rows an instruction took twice as long, and longer than the pairs of the fragment layout)
+      const int tm = tile / nt, r0 = tm * BM + 32 * quarter, j = lane & 3;
+      uint8_t* stage = smem + C::kOffStage + (warp - kEpilogueWarp0) * 32 * kStageRow;
+      const bool aligned = ((p.ldy | (int64_t)(reinterpret_cast<uintptr_t>(p.y) >> 2)) & 3) == 0;
 #pragma unroll
-      for (int nb = 0; nb < 4; ++nb)
+      for (int s = 0; s < C::kParts; ++s)
 #pragma unroll
-        for (int ce = 0; ce < 2; ++ce) {
-          const int row = tm * BM + 32 * cgroup + 8 * nb + 2 * t + ce;      // weight row
-          if (row < p.M) {
-            float* yr = p.y + (size_t)row * p.ldy + tn * BN + 32 * quarter + g;
+        for (int i = 0; i < kLoads; i += 2) {
+          const int n = kLoads > 1 ? 2 : 1;     // loads of this round
+          __syncwarp();
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-              if (tn * BN + 32 * quarter + 8 * j + g < p.N) yr[8 * j] = acc[j][nb][ce];
+          for (int e = 0; e < 2 * n; ++e)
+            *reinterpret_cast<ulonglong2*>(stage + lane * kStageRow + 16 * e) = make_ulonglong2(acc[s][i + (e >> 1)][2 * (e & 1)], acc[s][i + (e >> 1)][2 * (e & 1) + 1]);
+          __syncwarp();
+          const int c = (tile - tm * nt) * TN + C::kPart * s + kMine * side + 8 * i + 4 * j;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int row = r0 + 8 * k + (lane >> 2);
+            const float4 v = *reinterpret_cast<const float4*>(stage + (8 * k + (lane >> 2)) * kStageRow + 16 * j);
+            if (row >= p.M || j >= 2 * n) continue;
+            float* yr = p.y + (size_t)row * p.ldy + c;
+            if (aligned && c + 3 < p.N) {
+              *reinterpret_cast<float4*>(yr) = v;
+            } else {
+              if (c < p.N) yr[0] = v.x;
+              if (c + 1 < p.N) yr[1] = v.y;
+              if (c + 2 < p.N) yr[2] = v.z;
+              if (c + 3 < p.N) yr[3] = v.w;
+            }
           }
         }
     }
   }
 
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  fence_before();
   __syncthreads();
   if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, 1);
   if (warp == kMmaWarp) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
   }
 }
 
+// the workspace's columns: whole tiles, whole pre-pass blocks
+int padded_columns(int ncols) { return ncols <= 64 ? 64 : (ncols + 127) / 128 * 128; }
+
+constexpr size_t kColumnBytes = 2 * QK_K + kSumBytes + kPairBytes / 2;   // of a super-block
+
 }  // namespace
 
-size_t gemm_tc_workspace_bytes(int K, int ncols) {
-  return (size_t)((ncols + BN - 1) / BN) * (size_t)(K / QK_K) * kTileBytes;
-}
+size_t gemm_tc_workspace_bytes(int K, int ncols) { return (size_t)padded_columns(ncols) * (size_t)(K / QK_K) * kColumnBytes; }
 
 bool gemm_tc_supported(int type, int K, int ncols, const void* W, int64_t row_bytes, const ActPlanes& act) {
   return type == T_Q4_K && ncols >= kGemmTcMinCols && K % QK_K == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0 && row_bytes % 16 == 0 &&
-         act.bsums != nullptr && (reinterpret_cast<uintptr_t>(act.qs) & 15) == 0 && act.col_stride_qs % 16 == 0 &&
+         row_bytes < (1 << 27) && act.bsums != nullptr && (reinterpret_cast<uintptr_t>(act.qs) & 15) == 0 && act.col_stride_qs % 16 == 0 &&
          (reinterpret_cast<uintptr_t>(act.bsums) & 15) == 0 && act.col_stride_bs % 8 == 0;
 }
 
-// two launches: the activation tiling pre-pass (into `workspace`, gemm_tc_workspace_bytes) and the product
-cudaError_t launch_gemm_q4k_tc(const GemvArgs& a, int ncols, int sm_count, uint8_t* workspace, cudaStream_t st) {
+// the weights as bytes {rows, K/256 * 144}, boxes of 128 rows x one block
+static bool encode_rows(CUtensorMap* map, const GemvArgs& a) {
+  static const PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) != cudaSuccess) {
+      cudaGetLastError();
+      fn = nullptr;
+    }
+    return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+  }();
+  const cuuint64_t dims[2] = {(cuuint64_t)(a.K / QK_K) * Q4_K_BYTES, (cuuint64_t)a.M}, strides[1] = {(cuuint64_t)a.row_bytes};
+  const cuuint32_t box[2] = {Q4_K_BYTES, BM}, estr[2] = {1, 1};
+  return encode && encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(a.W), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int TN, bool kTable>
+static cudaError_t launch_tiles(const GemmArgs& g, const CUtensorMap& wmap, int sm_count, cudaStream_t st) {
+  constexpr int kSmem = Cfg<TN, kTable>::kSmemBytes;
   // per host thread (one context, one lane per thread): no shared mutable state between lanes
   static thread_local unsigned configured = 0;  // one bit per device
   int dev = 0;
   cudaGetDevice(&dev);
   if (!(configured & (1u << (dev & 31)))) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_q4k_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_q4k_tc_kernel<TN, kTable>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
     if (e != cudaSuccess) return e;
     configured |= 1u << (dev & 31);
   }
-  const int nt = (ncols + BN - 1) / BN;
-  cudaError_t e = cudaSuccess;
-  if (!a.tc_ws_reuse) {  // else the workspace still holds these planes in operand order (same K, columns, col0)
-    tile_activations_kernel<<<dim3(a.K / QK_K, nt), 256, 0, st>>>(a.act, a.col0, ncols, a.K, workspace);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
+  const int tiles = ((g.M + BM - 1) / BM) * ((g.N + TN - 1) / TN);
+  gemm_q4k_tc_kernel<TN, kTable><<<tiles < sm_count ? tiles : sm_count, kThreads, kSmem, st>>>(g, wmap);
+  return cudaGetLastError();
+}
+
+// Columns per tile: the fewest waves of CTAs, weighted with what a wave takes (4096 x 14336, one wave: 78, 88 and 97 us with
+// tiles of 32, 64 and 128 columns; 1024 x 4096: 31, 34.5 and 40).  Each is up to 1.4 times as fast as the others somewhere
+static int tile_columns(int M, int ncols, int sm_count, bool wide) {
+  const int mt = (M + BM - 1) / BM;
+  auto waves = [&](int tn) { return (mt * ((ncols + tn - 1) / tn) + sm_count - 1) / sm_count; };
+  const int c128 = 100 * waves(128), c64 = 90 * waves(64), c32 = 81 * waves(32);
+  if (wide && ncols > 64 && c128 <= c64 && c128 <= c32) return 128;
+  return c64 <= c32 ? 64 : 32;
+}
+
+// launches: the activation pre-pass (into the workspace), the pre-pass over the weights where several column tiles share
+// its results, and the product; the three again for columns whose operand the workspace does not hold beside the others'
+cudaError_t launch_gemm_q4k_tc(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st, int* launches) {
   GemmArgs g{};
   g.W = a.W;
   g.row_bytes = a.row_bytes;
   g.M = a.M;
   g.K = a.K;
-  g.N = ncols;
-  g.tiles = workspace;
-  g.y = a.y + a.col0;
+  g.x = a.tc_ws;
   g.ldy = a.ldy;
   g.status = a.status;
-  const int tiles = ((a.M + BM - 1) / BM) * nt;
-  const int grid = tiles < sm_count ? tiles : sm_count;
-  gemm_q4k_tc_kernel<<<grid, kThreads, kSmemBytes, st>>>(g);
-  return cudaGetLastError();
+  const int nkb = a.K / QK_K, mt = (a.M + BM - 1) / BM;
+  const size_t table_bytes = (size_t)mt * nkb * kTableBytes;
+  // columns of a turn: what the workspace holds, and a grid's y extent
+  const size_t group = gemm_tc_workspace_bytes(a.K, 128);
+  auto columns = [&](size_t room) { return (int)(room / group < 32767 ? room / group : 32767) * 128; };
+  const bool table_fits = table_bytes + group <= a.tc_ws_bytes;
+  int fit = columns(table_fits ? a.tc_ws_bytes - table_bytes : a.tc_ws_bytes);
+  if (fit >= ncols || (ncols <= 64 && fit == 0)) fit = ncols;   // a single group of 64 columns may fit where 128 do not
+  CUtensorMap wmap;
+  if (!encode_rows(&wmap, a)) return cudaErrorNotSupported;
+  for (int c = 0; c < ncols; c += fit) {
+    g.N = ncols - c < fit ? ncols - c : fit;
+    g.npad = padded_columns(g.N);
+    g.y = a.y + a.col0 + c;
+    uint8_t* sums = a.tc_ws + (size_t)nkb * g.npad * (2 * QK_K);
+    uint8_t* pairs = sums + (size_t)nkb * g.npad * kSumBytes;
+    uint8_t* table = pairs + (size_t)nkb * g.npad * (kPairBytes / 2);
+    g.sums = sums;
+    g.pairs = pairs;
+    g.table = table;
+    cudaError_t e = cudaSuccess;
+    if (!a.tc_ws_reuse || fit < ncols) {  // else the workspace still holds these planes in operand order (same K, columns, col0)
+      centre_activations_kernel<<<dim3(nkb, g.npad / kPreCols), 256, 0, st>>>(a.act, a.col0 + c, g.N, g.npad, a.tc_ws, sums, pairs);
+      ++*launches;
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
+    }
+    const int tn = tile_columns(a.M, g.N, sm_count, table_fits && mt <= 65535);
+    if (tn == 128) {
+      q4k_table_kernel<<<dim3(nkb, mt), BM, 0, st>>>(a.W, a.row_bytes, a.M, table);
+      ++*launches;
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
+      e = launch_tiles<128, true>(g, wmap, sm_count, st);
+    } else {
+      e = tn == 64 ? launch_tiles<64, false>(g, wmap, sm_count, st) : launch_tiles<32, false>(g, wmap, sm_count, st);
+    }
+    ++*launches;
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace emelb

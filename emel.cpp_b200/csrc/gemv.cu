@@ -221,7 +221,7 @@ bool gemv_fast_path_ok(int type, const void* w, int64_t row_bytes, int K) {
 
 bool gemv_takes_tensor_core(int type, const GemvArgs& a, int ncols) {
   return a.tc_ws && gemm_tc_supported(type, a.K, ncols, a.W, a.row_bytes, a.act) &&
-         gemm_tc_workspace_bytes(a.K, ncols) <= a.tc_ws_bytes;
+         gemm_tc_workspace_bytes(a.K, ncols < 128 ? ncols : 128) <= a.tc_ws_bytes;
 }
 
 cudaError_t launch_gemv(int type, const GemvArgs& a, int ncols, bool argmax, int sm_count, cudaStream_t st,
@@ -244,10 +244,7 @@ cudaError_t launch_gemv(int type, const GemvArgs& a, int ncols, bool argmax, int
     return launch_gemm_q6k_mma(a, ncols, sm_count, st);
   }
   // many columns of Q4_K: the tensor-core kernel (same numbers, see gemm_tc.cu)
-  if (!argmax && gemv_takes_tensor_core(type, a, ncols)) {
-    *launches += a.tc_ws_reuse ? 1 : 2;
-    return launch_gemm_q4k_tc(a, ncols, sm_count, a.tc_ws, st);
-  }
+  if (!argmax && gemv_takes_tensor_core(type, a, ncols)) return launch_gemm_q4k_tc(a, ncols, sm_count, st, launches);
   const bool fast = gemv_fast_path_ok(type, a.W, a.row_bytes, a.K);
   int grid = 0;
   cudaError_t e;

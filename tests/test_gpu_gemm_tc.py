@@ -64,6 +64,28 @@ def test_partial_tiles(be, port, t, k, m, n):
     check(be, port, t, synth.random_blocks(t, 3 * k + n, m, k), k, m, synth.activations_f32(k + n, k, n).reshape(k, n), n)
 
 
+def one_sided(k, n):
+    """Activations whose means, and sums on either side of them, are the largest that 8 bits allow: all one value, halves and
+    quarters at opposite ends in several orders, one value far from the others, ramps."""
+    x = np.ones((k, n), np.float32)
+    i = np.arange(k)
+    for j in range(n):
+        x[:, j] = [np.ones(k), -np.ones(k), np.where(i % 2, 1, -1), np.where(i % 256 < 128, 1, -1), np.where(i % 256 < 192, 1, -1),
+                   np.where(i % 256 < 64, 1, -1), np.where(i % 256 == 7, 1, -0.99), (i % 256) / 255.0 * 2 - 1, np.where(i % 4, 0, 1)][j % 9]
+    return x * np.linspace(0.5, 2.0, n, dtype=np.float32)
+
+
+@pytest.mark.parametrize("m,n", [(136, 32), (300, 33), (2400, 128), (14300, 130), (12700, 131), (2500, 1154)])
+@pytest.mark.parametrize("extreme", [False, True])
+def test_q4_k_tiles_of_every_width(be, port, m, n, extreme):
+    """Tiles of 32, 64 (2400 rows: one wave) and 128 columns (the last three: fewer waves), whole and ragged, with and without
+    8-byte rows of results."""
+    k = 512
+    w = extreme_blocks(eb.Q4_K, m, k) if extreme else synth.random_blocks(eb.Q4_K, m + n, m, k)
+    x = one_sided(k, n) if extreme else synth.activations_f32(m * n, k, n).reshape(k, n)
+    check(be, port, eb.Q4_K, w, k, m, x, n)
+
+
 @pytest.mark.parametrize("offset", [2, 6, 10, 14])
 @pytest.mark.parametrize("m", [140, 525])
 def test_q6_k_rows_at_even_addresses(be, port, offset, m):
@@ -148,6 +170,30 @@ def test_q6_k_columns_in_turns(port, monkeypatch):
         def call():
             assert b.mul_mat(eb.mul_mat_op(dev_w, eb.Q6_K, k, m, dev_x, n, dev_y)), b.last_error
         assert launches_of(b, call) == 5      # quantizer, and two turns
+        assert b.sync()
+        assert np.array_equal(dev_y.cpu().numpy().view(np.uint32), want.view(np.uint32))
+    finally:
+        b.close()
+
+
+def test_q4_k_columns_in_turns(port, monkeypatch):
+    """More columns than the workspace holds in f16: layout, table and product once per turn."""
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("EMELB_ACT_MELEMS", "72")
+    b = eb.Backend(0)
+    try:
+        k, m = 256, 3
+        n = (72 << 20) // k - 5
+        w = synth.random_blocks(eb.Q4_K, 9, m, k)
+        x = synth.activations_f32(10, k, n).reshape(k, n)
+        want = np.zeros((m, n), np.float32)
+        assert port.mul_mat(ob.mul_mat_op(w, eb.Q4_K, k, m, x, n, want), route="blocks")
+        dev_w, dev_x, dev_y = torch.from_numpy(w.reshape(-1)).cuda(), torch.from_numpy(x).cuda(), torch.zeros((m, n), device="cuda")
+        torch.cuda.synchronize()
+
+        def call():
+            assert b.mul_mat(eb.mul_mat_op(dev_w, eb.Q4_K, k, m, dev_x, n, dev_y)), b.last_error
+        assert launches_of(b, call) == 7      # quantizer, and two turns
         assert b.sync()
         assert np.array_equal(dev_y.cpu().numpy().view(np.uint32), want.view(np.uint32))
     finally:
