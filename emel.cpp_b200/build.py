@@ -31,6 +31,7 @@ SOURCES = {
     "gemm_q4k_mma.cu": [],
     "gemm_q6k_mma.cu": [],
     "gemm_q6k_tc.cu": [],
+    "gemm_q6k_wide.cu": [],
     "linear.cu": [],
     "gemm_bf16.cu": [],
     "mixer_ops.cu": [],

@@ -68,8 +68,7 @@ constexpr int kMetaSlots = 3;
 constexpr int kStageRow = 80;             // an epilogue warp's store: 16 columns of a row; a multiple of 16 that spreads rows over the banks
 constexpr int kRowMeta = 32;              // per row: d, d, -dmin, -dmin, then T of either half, each twice
 constexpr int kMinsBytes = BM * 32;       // A operand of the msum instruction: two 16-byte chunks of K
-constexpr int kSumBytes = 32;             // per column: 16 block sums as f16, two chunks
-constexpr int kPairBytes = 16;            // per two columns: dx, dx, v, v
+constexpr int kSumBytes = kColumnSumBytes, kPairBytes = kColumnPairBytes;
 
 constexpr int kTableRow = 24;             // per row of the table: d, d, -dmin, -dmin, T, T
 constexpr int kTableBytes = kMinsBytes + BM * kTableRow;   // of 128 rows x one super-block
@@ -125,7 +124,7 @@ struct GemmArgs {
 // masks leave side by side.  grid (K/256, npad/64), 256 threads; columns past N are zero.
 constexpr int kPreCols = 64, kPreRow = QK_K + 4;   // 65 words: column-wise reads fall on all banks
 
-__global__ void __launch_bounds__(256) centre_activations_kernel(ActPlanes act, int col0, int N, int npad, uint8_t* x, uint8_t* sums, uint8_t* pairs) {
+__global__ void __launch_bounds__(256) operand_layout_kernel(ActPlanes act, int col0, int N, int npad, bool centre, uint8_t* x, uint8_t* sums, uint8_t* pairs) {
   __shared__ __align__(16) uint8_t t8[kPreCols * kPreRow];
   __shared__ int mean[kPreCols];
   const int kb = blockIdx.x, c0 = blockIdx.y * kPreCols;
@@ -156,7 +155,7 @@ __global__ void __launch_bounds__(256) centre_activations_kernel(ActPlanes act, 
       }
       d = act.d[(int64_t)(col0 + c0 + col) * act.col_stride_d + kb];
     }
-    const int v = (total + 128) >> 8;
+    const int v = centre ? (total + 128) >> 8 : 0;
     mean[col] = v;
 #pragma unroll
     for (int c = 0; c < 2; ++c)
@@ -659,16 +658,35 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q4k_tc_kernel(const GemmArgs
 // the workspace's columns: whole tiles, whole pre-pass blocks
 int padded_columns(int ncols) { return ncols <= 64 ? 64 : (ncols + 127) / 128 * 128; }
 
-constexpr size_t kColumnBytes = 2 * QK_K + kSumBytes + kPairBytes / 2;   // of a super-block
-
 }  // namespace
 
-size_t gemm_tc_workspace_bytes(int K, int ncols) { return (size_t)padded_columns(ncols) * (size_t)(K / QK_K) * kColumnBytes; }
+
+size_t operand_layout_bytes(int K, int npad) { return (size_t)npad * (size_t)(K / QK_K) * (2 * QK_K + kSumBytes + kPairBytes / 2); }
+
+OperandLayout operand_layout(uint8_t* workspace, int K, int npad) {
+  const size_t columns = (size_t)(K / QK_K) * npad;
+  OperandLayout o;
+  o.x = workspace;
+  o.sums = o.x + columns * (2 * QK_K);
+  o.pairs = o.sums + columns * kSumBytes;
+  return o;
+}
+
+cudaError_t launch_operand_layout(const ActPlanes& act, int col0, int ncols, int npad, int K, const OperandLayout& out, bool centre, cudaStream_t st) {
+  operand_layout_kernel<<<dim3(K / QK_K, npad / kPreCols), 256, 0, st>>>(act, col0, ncols, npad, centre, out.x, out.sums, out.pairs);
+  return cudaGetLastError();
+}
+
+bool planes_aligned(const ActPlanes& act) {
+  return act.bsums != nullptr && (reinterpret_cast<uintptr_t>(act.qs) & 15) == 0 && act.col_stride_qs % 16 == 0 &&
+         (reinterpret_cast<uintptr_t>(act.bsums) & 15) == 0 && act.col_stride_bs % 8 == 0;
+}
+
+size_t gemm_tc_workspace_bytes(int K, int ncols) { return operand_layout_bytes(K, padded_columns(ncols)); }
 
 bool gemm_tc_supported(int type, int K, int ncols, const void* W, int64_t row_bytes, const ActPlanes& act) {
   return type == T_Q4_K && ncols >= kGemmTcMinCols && K % QK_K == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0 && row_bytes % 16 == 0 &&
-         row_bytes < (1 << 27) && act.bsums != nullptr && (reinterpret_cast<uintptr_t>(act.qs) & 15) == 0 && act.col_stride_qs % 16 == 0 &&
-         (reinterpret_cast<uintptr_t>(act.bsums) & 15) == 0 && act.col_stride_bs % 8 == 0;
+         row_bytes < (1 << 27) && planes_aligned(act);
 }
 
 // the weights as bytes {rows, K/256 * 144}, boxes of 128 rows x one block
@@ -723,7 +741,6 @@ cudaError_t launch_gemm_q4k_tc(const GemvArgs& a, int ncols, int sm_count, cudaS
   g.row_bytes = a.row_bytes;
   g.M = a.M;
   g.K = a.K;
-  g.x = a.tc_ws;
   g.ldy = a.ldy;
   g.status = a.status;
   const int nkb = a.K / QK_K, mt = (a.M + BM - 1) / BM;
@@ -740,17 +757,16 @@ cudaError_t launch_gemm_q4k_tc(const GemvArgs& a, int ncols, int sm_count, cudaS
     g.N = ncols - c < fit ? ncols - c : fit;
     g.npad = padded_columns(g.N);
     g.y = a.y + a.col0 + c;
-    uint8_t* sums = a.tc_ws + (size_t)nkb * g.npad * (2 * QK_K);
-    uint8_t* pairs = sums + (size_t)nkb * g.npad * kSumBytes;
-    uint8_t* table = pairs + (size_t)nkb * g.npad * (kPairBytes / 2);
-    g.sums = sums;
-    g.pairs = pairs;
+    const OperandLayout x = operand_layout(a.tc_ws, a.K, g.npad);
+    uint8_t* table = a.tc_ws + operand_layout_bytes(a.K, g.npad);
+    g.x = x.x;
+    g.sums = x.sums;
+    g.pairs = x.pairs;
     g.table = table;
     cudaError_t e = cudaSuccess;
     if (!a.tc_ws_reuse || fit < ncols) {  // else the workspace still holds these planes in operand order (same K, columns, col0)
-      centre_activations_kernel<<<dim3(nkb, g.npad / kPreCols), 256, 0, st>>>(a.act, a.col0 + c, g.N, g.npad, a.tc_ws, sums, pairs);
+      e = launch_operand_layout(a.act, a.col0 + c, g.N, g.npad, a.K, x, true, st);
       ++*launches;
-      e = cudaGetLastError();
       if (e != cudaSuccess) return e;
     }
     const int tn = tile_columns(a.M, g.N, sm_count, table_fits && mt <= 65535);

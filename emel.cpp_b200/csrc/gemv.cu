@@ -236,6 +236,8 @@ cudaError_t launch_gemv(int type, const GemvArgs& a, int ncols, bool argmax, int
     ++*launches;
     return launch_gemm_q4k_mma(a, ncols, sm_count, st);
   }
+  // prompts, Q6_K: two f16 operands per weight from blocks unpacked once (gemm_q6k_wide.cu)
+  if (!argmax && gemm_q6k_wide_supported(type, a, ncols, sm_count)) return launch_gemm_q6k_wide(a, ncols, sm_count, st, launches);
   // several columns of Q6_K, K no multiple of 2048 or rows unaligned: two f16 operands per weight on tcgen05 (gemm_q6k_tc.cu)
   if (!argmax && gemm_q6k_tc_supported(type, a, ncols)) return launch_gemm_q6k_tc(a, ncols, sm_count, st, launches);
   // nine or more columns of Q6_K: mma.sync per 16-weight scale group (gemm_q6k_mma.cu)

@@ -242,6 +242,22 @@ constexpr int kGemmQ6kTcMinCols = 5;   // Q6_K rows that no streaming kernel tak
 constexpr int kGemmMmaMinCols = 9;   // Q6_K: fewer columns run the CUDA-core mat-vec kernels (7 and 8: gemm_q6k_mma.cu)
 constexpr int kGemmQ4kMmaMinCols = 5; // Q4_K: 8 columns take 39 / 63 us through the mat-vec kernel, 23-28 / 35 us through the mma.sync one (4096x14336 / 14336x4096)
 constexpr int kGemmQ8MmaMinCols = 3; // Q8_0 / Q4_0: from three columns on the mma.sync kernel (21-24 us for up to 8 columns of 14336x4096) beats the mat-vec kernels (29 us at 4 columns)
+// activations of the tcgen05 kernels in the workspace: columns of f16 in swizzle atoms of 8 columns x 64 K, {dx, dx, mean, mean} a
+// column pair and, as f16, the 16 block sums a column
+constexpr int kColumnSumBytes = 32, kColumnPairBytes = 16;
+struct OperandLayout {
+  uint8_t* x;       // [K/64][npad/8] atoms
+  uint8_t* sums;    // [K/256][2][npad][16 bytes]
+  uint8_t* pairs;   // [K/256][npad/2]
+};
+size_t operand_layout_bytes(int K, int npad);
+OperandLayout operand_layout(uint8_t* workspace, int K, int npad);
+// centre: values minus their super-block's rounded mean; else the values, and 0 for the mean.  npad: a multiple of 64
+cudaError_t launch_operand_layout(const ActPlanes& act, int col0, int ncols, int npad, int K, const OperandLayout& out, bool centre, cudaStream_t st);
+bool planes_aligned(const ActPlanes& act);   // 16-byte pieces of the K-quant planes
+// gemm_q6k_wide.cu: many columns of Q6_K weights on tcgen05, rows at even addresses; overwrites the tensor-core workspace
+bool gemm_q6k_wide_supported(int type, const GemvArgs& a, int ncols, int sm_count);
+cudaError_t launch_gemm_q6k_wide(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st, int* launches);
 bool gemm_tc_supported(int type, int K, int ncols, const void* W, int64_t row_bytes, const ActPlanes& act);
 // true when launch_gemv would run the kernel that honours GemvArgs::pro_x for this matrix
 bool gemv_prologue_supported(int type, const void* w, int64_t row_bytes, int K);

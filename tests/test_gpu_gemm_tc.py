@@ -105,6 +105,58 @@ def test_q6_k_rows_at_even_addresses(be, port, offset, m):
     assert np.array_equal(dev_y.cpu().numpy().view(np.uint32), want.view(np.uint32))
 
 
+@pytest.mark.parametrize("k,m,n", [(2048, 4737, 130), (2048, 10000, 96), (10240, 130, 97), (256, 6500, 201), (1280, 9472, 192), (10496, 128, 192)])
+@pytest.mark.parametrize("extreme", [False, True])
+def test_q6_k_prompts(be, port, k, m, n, extreme):
+    """The prompt kernel's sizes: streamed rows and others, whole and ragged tiles, rows of 8 bytes and not."""
+    w = extreme_blocks(eb.Q6_K, m, k) if extreme else synth.random_blocks(eb.Q6_K, m + n, m, k)
+    x = one_sided(k, n) if extreme else synth.activations_f32(m * n, k, n).reshape(k, n)
+    count = launches_of(be, lambda: check(be, port, eb.Q6_K, w, k, m, x, n))
+    assert count == 4      # quantizer, operand layout, slabs, product
+
+
+@pytest.mark.parametrize("offset", [2, 8, 14])
+def test_q6_k_prompts_at_even_addresses(be, port, offset):
+    torch = pytest.importorskip("torch")
+    k, m, n = 768, 6500, 194
+    w = synth.random_blocks(eb.Q6_K, 5, m, k)
+    x = synth.activations_f32(6, k, n).reshape(k, n)
+    want = np.zeros((m, n), np.float32)
+    assert port.mul_mat(ob.mul_mat_op(w, eb.Q6_K, k, m, x, n, want), route="blocks")
+    room = torch.zeros(w.size + 64, dtype=torch.uint8, device="cuda")
+    dev_w = room[offset:offset + w.size]
+    dev_w.copy_(torch.from_numpy(w.reshape(-1)))
+    dev_x, dev_y = torch.from_numpy(x).cuda(), torch.zeros((m, n), device="cuda")
+    torch.cuda.synchronize()
+    assert be.mul_mat(eb.mul_mat_op(dev_w, eb.Q6_K, k, m, dev_x, n, dev_y)), be.last_error
+    assert be.sync()
+    assert np.array_equal(dev_y.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+def test_q6_k_prompt_rows_in_turns(monkeypatch):
+    """More rows than the workspace holds unpacked: slabs and product once per turn.  Four columns equal those of the mat-vec kernels."""
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("EMELB_ACT_MELEMS", "1")
+    b = eb.Backend(0)
+    try:
+        k, m, n = 256, 220000, 192
+        w = torch.from_numpy(synth.random_blocks(eb.Q6_K, 9, 1000, k).reshape(1000, -1)).cuda()
+        w = w[torch.arange(m, device="cuda") * 7 % 997].contiguous()
+        x = torch.from_numpy(synth.activations_f32(10, k, n).reshape(k, n)).cuda()
+        y, few = torch.zeros((m, n), device="cuda"), torch.zeros((m, 4), device="cuda")
+        x4 = x[:, :4].contiguous()
+        torch.cuda.synchronize()
+
+        def call():
+            assert b.mul_mat(eb.mul_mat_op(w, eb.Q6_K, k, m, x, n, y)), b.last_error
+        assert launches_of(b, call) == 6      # quantizer, operand layout, and two turns
+        assert b.mul_mat(eb.mul_mat_op(w, eb.Q6_K, k, m, x4, 4, few)), b.last_error
+        assert b.sync()
+        assert torch.equal(y[:, :4].contiguous().view(torch.int32), few.view(torch.int32))
+    finally:
+        b.close()
+
+
 def launches_of(be, call):
     before = be.diagnostics()["kernel_launches"]
     call()
