@@ -60,7 +60,7 @@ namespace {
 using namespace tc;
 
 constexpr int BM = 128;
-constexpr int kEpilogueWarp0 = 8, kEpilogueWarps = 8, kMmaWarp = 16, kSumWarp = 17, kLoaderWarp = 18;   // and the meta loader's warp
+constexpr int kEpilogueWarp0 = 8, kEpilogueWarps = 8, kMmaWarp = 16, kLoaderWarp = 18;   // two MMA warps; the meta loader's warp
 constexpr int kThreads = 20 * 32;
 
 constexpr int kRawBytes = BM * Q4_K_BYTES;   // 128 rows of a super-block as they lie in memory; 144 bytes a row spread reads over the banks
@@ -248,11 +248,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q4k_tc_kernel(const GemmArgs
   const uint32_t r_full = h_free + 8 * 4 * C::kTurns; // [raw slots] TMA -> producers: the weights of a super-block
   const uint32_t r_free = r_full + 8 * C::kRawSlots;
   const uint32_t m_free = r_free + 8 * C::kRawSlots;  // [3] epilogue -> loader: the meta slot is read
-  const uint32_t s_full = m_free + 8 * kMetaSlots;  // [parts] msum warp -> epilogue: the part's accumulators and msum are complete
-  const uint32_t s_free = s_full + 8 * 2;           // [parts] epilogue -> msum warp: they are read
-  const uint32_t d_full = s_free + 8 * 2;           // [2 turns] MMA -> msum warp: the accumulators are complete
-  const uint32_t d_free = d_full + 8 * 2;           // [2 turns] epilogue -> MMA: they are read
-  const uint32_t drained = d_free + 8 * 2;          // [2] only after a wait that gave up
+  const uint32_t s_full = m_free + 8 * kMetaSlots;    // [parts] MMA -> epilogue: the part's accumulators and msum are complete
+  const uint32_t s_free = s_full + 8 * 2;             // [parts] epilogue -> MMA: they are read
+  const uint32_t drained = s_free + 8 * 2;            // [2] only after a wait that gave up
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::kOffBars + 8 * 60);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -260,13 +258,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q4k_tc_kernel(const GemmArgs
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kRawSlots; ++s) { mbar_init(r_full + 8 * s, 1); mbar_init(r_free + 8 * s, 8); }
-    for (int s = 0; s < 4 * C::kTurns; ++s) { mbar_init(h_full + 8 * s, (s & 3) == 3 ? 6 : 5); mbar_init(h_free + 8 * s, 1); }
+    for (int s = 0; s < 4 * C::kTurns; ++s) { mbar_init(h_full + 8 * s, (s & 3) == 3 ? 6 : 5); mbar_init(h_free + 8 * s, C::kParts); }
     for (int s = 0; s < kMetaSlots; ++s) mbar_init(m_free + 8 * s, kEpilogueWarps);
     for (int s = 0; s < 2; ++s) {
       mbar_init(s_full + 8 * s, 1);
       mbar_init(s_free + 8 * s, kEpilogueWarps);
-      mbar_init(d_full + 8 * s, 1);
-      mbar_init(d_free + 8 * s, kEpilogueWarps);
       mbar_init(drained + 8 * s, 1);
     }
     *abort_flag = 0;
@@ -391,60 +387,59 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q4k_tc_kernel(const GemmArgs
     constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(BM >> 4) << 24);
     const bool leader = elect_one();
     bool live = true;
-    if (warp == kMmaWarp) {
-      // -------------------------------------------------------------- accumulators: 16 instructions a turn
-      constexpr uint32_t kIdescD = kIdesc | ((uint32_t)(TN >> 3) << 17);
-      const uint64_t x0 = operand_desc(smem_u32(smem), kAtomBytes);
-#pragma unroll 1
-      for (int it = 0; it < turns; ++it) {
-        const int buf = it & 1;
-        const uint32_t d = tmem_base + (uint32_t)(TN * buf), phase = (uint32_t)(it >> 1) & 1u;
-        live = mbar_wait(d_free + 8 * buf, phase ^ 1u, abort_flag);
-#pragma unroll 1
+    if (warp < kLoaderWarp) {
+      // -------------------------------------------------------------- MMA issue: a warp for either part of the columns, so that
+      // the one's waits pass while the other's instructions run.  A part's accumulators have two buffers, its msum one:
+      // when the epilogue has read the part of turn it - 1, msum of turn it and the accumulators of turn it + 1 are made
+      constexpr uint32_t kIdescN = kIdesc | ((uint32_t)(C::kPart >> 3) << 17);
+      const int s = warp - kMmaWarp;
+      const uint64_t x0 = operand_desc(smem_u32(smem), kAtomBytes) + (uint64_t)((C::kPart / 8 * s * kAtomBytes) >> 4);
+      const uint64_t sums0 = plain_desc(smem_u32(meta), TN * 16) + (uint64_t)(C::kPart * s);
+      const uint64_t mins0 = plain_desc(smem_u32(kTable ? meta + C::kOffTable : mins), BM * 16);
+      const uint32_t d0 = tmem_base + (uint32_t)(C::kPart * s);
+      auto accumulate = [&](int it) {
+        const int buf = it & 1, h0 = 4 * (it & (C::kTurns - 1));
+        bool ok = true;
+#pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const int hq = 4 * (it & (C::kTurns - 1)) + q;
-          live = live && mbar_wait(h_full + 8 * hq, (uint32_t)(it / C::kTurns) & 1u, abort_flag);
-          live = __all_sync(0xffffffffu, live);
-          if (!live) break;
+          ok = ok && mbar_wait(h_full + 8 * (h0 + q), (uint32_t)(it / C::kTurns) & 1u, abort_flag);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
           fence_after();
-          const uint64_t x = x0 + (uint64_t)(hq * (C::kQuarterBytes >> 4));
+          const uint64_t x = x0 + (uint64_t)((h0 + q) * (C::kQuarterBytes >> 4));
           const uint32_t a_op = tmem_base + C::kTmemA + (C::kOperands == 2 ? 128u * buf : 0u) + 32u * q;
           if (leader) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) mma_f16(d, a_op + 8u * j, x + (uint64_t)(2 * j), kIdescD, (q | j) ? 1u : 0u);
-            mma_commit(h_free + 8 * hq);
-            if (q == 3) mma_commit(d_full + 8 * buf);
+            for (int j = 0; j < 4; ++j) mma_f16(d0 + (uint32_t)(TN * buf), a_op + 8u * j, x + (uint64_t)(2 * j), kIdescN, (q | j) ? 1u : 0u);
+            mma_commit(h_free + 8 * (h0 + q));
           }
           __syncwarp();
         }
-        if (!live) break;
-      }
-    } else if (warp == kSumWarp) {
-      // -------------------------------------------------------------- msum: one instruction a part.  The accumulators have two
-      // buffers, a part's msum one: made when the epilogue has read the part of the turn before
-      constexpr uint32_t kIdescS = kIdesc | ((uint32_t)(C::kPart >> 3) << 17);
-      const uint64_t sums0 = plain_desc(smem_u32(meta), TN * 16);
-      const uint64_t mins0 = plain_desc(smem_u32(kTable ? meta + C::kOffTable : mins), BM * 16);
+        return ok;
+      };
+      const int my_turns = s < C::kParts ? turns : 0;
       int ms = 0, mslot = 0;
 #pragma unroll 1
-      for (int it = 0; it < turns; ++it) {
-        live = mbar_wait(d_full + 8 * (it & 1), (uint32_t)(it >> 1) & 1u, abort_flag);
-#pragma unroll 1
-        for (int s = 0; s < C::kParts; ++s) {
-          live = live && mbar_wait(s_free + 8 * s, ((uint32_t)it & 1u) ^ 1u, abort_flag);
+      for (int it = -1; live && it < my_turns; ++it) {
+        if (it >= 0) {
+          live = mbar_wait(s_free + 8 * s, ((uint32_t)it & 1u) ^ 1u, abort_flag);
           live = __all_sync(0xffffffffu, live);
           if (!live) break;
           fence_after();
           if (leader) {
-            mma_f16_ss(tmem_base + C::kTmemM + (uint32_t)(s * C::kPart), mins0 + (uint64_t)((kTable ? ms * C::kMetaBytes : mslot * kMinsBytes) >> 4),
-                       sums0 + (uint64_t)((ms * C::kMetaBytes + s * C::kPart * 16) >> 4), kIdescS);
+            mma_f16_ss(d0 + C::kTmemM, mins0 + (uint64_t)((kTable ? ms * C::kMetaBytes : mslot * kMinsBytes) >> 4), sums0 + (uint64_t)(ms * C::kMetaBytes >> 4), kIdescN);
             mma_commit(s_full + 8 * s);
           }
           __syncwarp();
+          if (++ms == kMetaSlots) ms = 0;
+          if (++mslot >= C::kMinsSlots) mslot = 0;
         }
-        if (!live) break;
-        if (++ms == kMetaSlots) ms = 0;
-        if (++mslot >= C::kMinsSlots) mslot = 0;
+        if (it + 1 < my_turns) live = accumulate(it + 1);
+      }
+      if (!live && leader) {
+        // gave up: let the tensor core finish what was issued before the TMEM goes away (bounded)
+        mma_commit(drained + 8 * s);
+        for (int spins = 0; spins < (1 << 16) && !mbar_try_wait(drained + 8 * s, 0u); ++spins) {}
       }
     } else if (warp == kLoaderWarp) {
       // -------------------------------------------------------------- activations, a quarter super-block a copy, and weights
@@ -531,12 +526,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q4k_tc_kernel(const GemmArgs
           for (int spins = 0; spins < (1 << 14) && !mbar_try_wait(h_full + 8 * (4 * (i & (C::kTurns - 1)) + 3), (uint32_t)(i / C::kTurns) & 1u); ++spins) {}
       }
     }
-    if (warp <= kSumWarp && !live && leader) {
-      // gave up: let the tensor core finish what was issued before the TMEM goes away (bounded)
-      const uint32_t mine = drained + 8 * (warp - kMmaWarp);
-      mma_commit(mine);
-      for (int spins = 0; spins < (1 << 16) && !mbar_try_wait(mine, 0u); ++spins) {}
-    }
     __syncwarp();
   } else {
     // ---------------------------------------------------------------- epilogue
@@ -590,7 +579,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q4k_tc_kernel(const GemmArgs
               fence_before();
               __syncwarp();
               mbar_arrive_if(lead, s_free + 8 * s);
-              if (s + 1 == C::kParts) mbar_arrive_if(lead, d_free + 8 * parity);
             } else {
               tmem_ld8(td + 8u * (i + 1), dv[(i + 1) & 1]);
               tmem_ld8(tm + 8u * (i + 1), sv[(i + 1) & 1]);
