@@ -1,14 +1,30 @@
 // y {rows, M} = act(x {rows, K} W {M, K}^T + bias) with bf16 operands on the Blackwell tensor cores: tcgen05.mma
 // kind::f16, f32 accumulators in TMEM, operands brought by TMA in the 128-byte swizzled K-major layout.
 //
-// The weights are the M operand (128 rows = TMEM lanes), BN rows of x the N operand, so few rows cost a narrow tile.
-// One output tile per CTA, 6 warps: warps 0-3 read the accumulators back (one TMEM lane quarter each), warp 4 issues
-// the TMA copies, warp 5 owns the TMEM allocation and issues the MMAs.  GLU tiles hold a gate tile and the up tile of
-// the same outputs side by side in TMEM and store silu(gate) * up.
+// The weights are the M operand (TMEM lanes), BN rows of x the N operand, so few rows cost a narrow tile.  GLU tiles hold a
+// gate tile and the up tile of the same outputs side by side in TMEM and store silu(gate) * up.
+//
+// A tile belongs to the two CTAs of a cluster on neighbouring SMs (cta_group::2): 256 features x BN rows, of which either CTA
+// holds the weights and accumulators of 128 features, but half of the rows of x, which the tensor cores of both read.  Pairs
+// stay for tile after tile, one CTA per SM: 10 warps, of which warp 8 issues the TMA copies, warp 9 of the first CTA the MMAs of
+// the pair (its copies and those of the second CTA count on its barriers, its commits arrive at both), and warps 0-7 read the
+// accumulators back (a TMEM lane quarter and half of the columns each) while the next tile's MMAs fill the other half of
+// TMEM.
+//
+// What it replaced, a CTA and a tile of 128 features each, two CTAs per SM with 2 to 4 stages, waited on copies (a round trip
+// is over a microsecond) and on last waves.  us, mean of 8 launches: 14336 x 2 x 4096, 2048 rows 438 -> 329 (1,460 TFLOP/s), 300
+// rows 125 -> 84; 8192 x 2 x 2048, 2048 rows 144 -> 99; 4096 x 14336, 2048 rows 182 -> 162 (1,480), 300 rows 62 -> 50; 2048 x 8192,
+// 200 rows 49 -> 27.  Bounds: large products the tensor cores, few rows the chain of a wait, the MMAs and a commit per stage
+// (about 290 cycles beside the MMAs' own, whether addresses are constants of an unrolled loop or not, hence two slabs of K a
+// stage where shared memory has room for enough of these).
+// Short sums: a cluster's start costs 1 to 2 us more than a CTA's, tiles of many rows win it back (K = 512: 2048 features, 1500 rows
+// 10.4 -> 12.4; 14336 features, 8 rows 6.3 -> 7.6, 2048 rows 47 -> 39).
 // Every wait is bounded; on a timeout the CTA raises the status word, lets its copies land and frees its TMEM.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "act.cuh"
 #include "common.cuh"
@@ -17,7 +33,7 @@
 namespace emelb {
 namespace {
 
-constexpr int kThreads = 192, kTmaWarp = 4, kMmaWarp = 5;
+constexpr int kEpilogueWarps = 8, kTmaWarp = 8, kMmaWarp = 9, kThreads = 320;
 constexpr int kBM = kGemmWeightBox, kBK = 64;
 constexpr int kWeightTile = kBM * kBK * 2;
 constexpr int kWaitSpins = 1 << 22;
@@ -57,11 +73,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   *abort_flag = 1;
   return false;
 }
-__device__ __forceinline__ void tma_load(void* dst, const TmaMap* map, int x, int y, uint64_t* bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
-               "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
-               : "memory");
-}
 // one thread of the warp, in a form that tells the compiler that a single one issues what follows (2048 prompt
 // rows: 39.8 and 75.4 us a launch of 128- and 256-row tiles with a lane test, 38.7 and 73.8 with elect.sync)
 __device__ __forceinline__ bool elect_one() {
@@ -73,20 +84,6 @@ __device__ __forceinline__ bool elect_one() {
 // K-major operand in 8-row x 128-byte swizzled atoms, 1024 bytes apart (descriptor version 1, swizzle mode 2)
 __device__ __forceinline__ uint64_t operand_desc(uint32_t saddr) {
   return (uint64_t)((saddr >> 4) & 0x3fffu) | (uint64_t)1 << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
-}
-// D = f32, A = B = bf16, both K-major, M = 128
-template <int BN>
-constexpr uint32_t kInstrDesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -122,173 +119,262 @@ struct GemmParams {
   int64_t tail_ld;
 };
 
-// DEEP: as many stages as one CTA per SM holds, for grids that give an SM no second CTA.  A stage's round trip (free ->
-// copy -> MMA) is over a microsecond, so the stages in flight set the rate.  Mean of 20 launches a prompt of 300 tokens,
-// 4096 / 14336 features: 57.6 -> 40.8 us; the two-matrix products of 200 tokens at 2048 / 8192: 38.9 -> 29.9 us.  A whole request
-// of these with 24 decoded steps, 29.6 and 13.0 ms, gains 1 to 3 %, little more than its runs differ
-template <int BN, bool GLU, bool DEEP>
+constexpr int kTileLd = 40;   // elements from row to row where bf16 outputs turn
+
+// one warp: 32 features x rows [c_begin, c_end) of accumulators -> y
+template <int BN, bool GLU>
+__device__ __forceinline__ void store_tile(const GemmParams& p, uint32_t tmem, int f0, int t0, int quarter, int lane, __nv_bfloat16* tile, int c_begin, int c_end) {
+  const int f = f0 + quarter * 32 + lane;
+  const bool live = f < p.M;
+  const float b0 = live && p.bias ? p.bias[f] : 0.0f, b1 = GLU && live && p.bias ? p.bias[p.M + f] : 0.0f;
+  const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
+  const bool sigm = p.act == ACT_SILU_SIGMOID, gelu = p.act == ACT_GLU_GELU, cap = p.act == ACT_SOFTCAP, tail = f >= p.tail;
+  // bf16 outputs turn in shared memory, 32 features x kCh rows of a warp at a time, and leave as 16-byte stores
+  constexpr int kCh = BN < 64 ? 16 : 32;
+  const int f_end = min(p.M, p.tail), fw = f0 + quarter * 32;
+  for (int c = c_begin; c < c_end && t0 + c < p.rows; c += kCh) {
+    uint32_t v[kCh], u[GLU ? kCh : 1];
+    tmem_ld(lane_base + c, v);
+    if constexpr (GLU) tmem_ld(lane_base + BN + c, u);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    float o[kCh];
+#pragma unroll
+    for (int j = 0; j < kCh; ++j) {
+      o[j] = __uint_as_float(v[j]) + b0;
+      if constexpr (GLU) {
+        o[j] = (gelu ? gelu_tanhf_(o[j]) : siluf_(o[j])) * (__uint_as_float(u[j]) + b1);
+      } else if (sigm) {
+        const float sg = sigmoidf_(o[j]);
+        o[j] = f < p.act_split ? o[j] * sg : sg;
+      } else if (cap) {
+        o[j] = softcapf_(o[j] * p.out_scale, p.softcap);
+      }
+    }
+    if (live && (tail || !p.yb)) {
+      float* y = tail ? p.tail_y + f - p.tail : p.y + f;
+      const int64_t ld = tail ? p.tail_ld : p.ldy;
+#pragma unroll
+      for (int j = 0; j < kCh; ++j)
+        if (t0 + c + j < p.rows) y[(int64_t)(t0 + c + j) * ld] = o[j];
+    }
+    if (!p.yb) continue;
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < kCh; ++j) tile[j * kTileLd + lane] = __float2bfloat16_rn(o[j]);
+    __syncwarp();
+#pragma unroll
+    for (int i = lane; i < 4 * kCh; i += 32) {
+      const int j = i / 4, q = 8 * (i % 4), n = f_end - fw - q;   // n features of this piece are stored
+      if (t0 + c + j >= p.rows || n <= 0) continue;
+      const __nv_bfloat16* src = tile + j * kTileLd + q;
+      __nv_bfloat16* dst = p.yb + (int64_t)(t0 + c + j) * p.ldy + fw + q;
+      if (n >= 8) {
+        *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
+      } else {
+        for (int e = 0; e < n; ++e) dst[e] = src[e];
+      }
+    }
+  }
+}
+
+// BN rows; SL slabs of 64 elements of K a stage
+template <int BN, bool GLU, int SL>
 struct Tile {
-  static constexpr int kStageBytes = (GLU ? 2 : 1) * kWeightTile + BN * kBK * 2;
-  static constexpr int kStages = DEEP ? 200 * 1024 / kStageBytes : kStageBytes > 40 * 1024 ? 2 : BN == 128 ? 3 : 4;   // two CTAs per SM: one computes while the other stores
-  static constexpr int kTmemCols = (GLU ? 2 : 1) * BN < 32 ? 32 : (GLU ? 2 : 1) * BN;
-  static constexpr int kBox = BN >= 128 ? 128 : kGemmTokenBox;   // rows per TMA copy of x
-  static constexpr int kSmem = kStages * kStageBytes + 1024 + 256;
+  static constexpr int kRows = BN / 2;                // rows of x of either CTA
+  static constexpr int kXTile = kRows * kBK * 2;
+  static constexpr int kSlabBytes = (GLU ? 2 : 1) * kWeightTile + kXTile;
+  static constexpr int kStageBytes = SL * kSlabBytes;
+  static constexpr int kAccCols = (GLU ? 2 : 1) * BN, kTmemCols = 2 * kAccCols;
+  static constexpr int kTurnBytes = kEpilogueWarps * 32 * kTileLd * 2;
+  static constexpr int kRest = kTurnBytes + 1024 + 512;   // beside the stages; 1024 to align these
+  static constexpr int kStages = std::min((226 * 1024 - kRest) / kStageBytes, 8);
+  static constexpr int kSmem = kStages * kStageBytes + kRest;
+  static_assert(kTmemCols <= 512 && kStages >= 2, "accumulators of two tiles");
 };
 
-template <int BN, bool GLU, bool DEEP>
-__global__ void __launch_bounds__(kThreads) gemm_bf16_kernel(const __grid_constant__ TmaMap wmap, const __grid_constant__ TmaMap xmap,
-                                                             const GemmParams p) {
-  using T = Tile<BN, GLU, DEEP>;
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the address of the first CTA's copy of a shared memory object
+__device__ __forceinline__ uint32_t in_first(const void* ptr) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(ptr)));
+  return a;
+}
+__device__ __forceinline__ void prefetch_map(const TmaMap* map) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+}
+// into this CTA's shared memory, counted on a barrier of the pair
+__device__ __forceinline__ void tma_load(void* dst, const TmaMap* map, int x, int y, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                   smem_u32(dst)),
+               "l"(map), "r"(x), "r"(y), "r"(bar)
+               : "memory");
+}
+// D = f32, A = B = bf16, both K-major, M = 256
+template <int BN>
+constexpr uint32_t kInstrDesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(2 * kBM >> 4) << 24);
+__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// arrives at both CTAs' barriers
+__device__ __forceinline__ void mma_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+               "h"((uint16_t)3)
+               : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive_at(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+template <int BN, bool GLU, int SL>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+    gemm_bf16_kernel(const __grid_constant__ TmaMap wmap, const __grid_constant__ TmaMap xmap, const GemmParams p) {
+  using T = Tile<BN, GLU, SL>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + T::kStages * T::kStageBytes);
-  uint64_t* empty = full + T::kStages;
-  uint64_t* done = empty + T::kStages;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  __nv_bfloat16* turn = reinterpret_cast<__nv_bfloat16*>(smem + T::kStages * T::kStageBytes);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + T::kStages * T::kStageBytes + T::kTurnBytes);   // of the first CTA: copies of both have landed
+  uint64_t* empty = full + T::kStages;       // of either: the MMAs are done with the stage
+  uint64_t* acc_full = empty + T::kStages;   // of either: a tile's accumulators stand
+  uint64_t* acc_empty = acc_full + 2;        // of the first CTA: both have read theirs
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t0 = blockIdx.x * BN, f0 = blockIdx.y * kBM;
-  const int nk = (p.K + kBK - 1) / kBK;
+  const uint32_t rank = cluster_rank();
+  const int slabs = (p.K + kBK - 1) / kBK, nk = (slabs + SL - 1) / SL;
+  const int nt = (p.rows + BN - 1) / BN, tiles = nt * ((p.M + 2 * kBM - 1) / (2 * kBM));
+  const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < T::kStages; ++s) {
       mbar_init(full + s, 1);
       mbar_init(empty + s, 1);
     }
-    mbar_init(done, 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(acc_full + b, 1);
+      mbar_init(acc_empty + b, 2 * kEpilogueWarps);
+    }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (warp == kMmaWarp) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(T::kTmemCols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(T::kTmemCols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  if (warp == kTmaWarp && lane == 0) {
+    prefetch_map(&wmap);
+    prefetch_map(&xmap);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
+  cluster_sync();            // the barriers and accumulators of both CTAs stand
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
 
-  if (warp == kTmaWarp && lane == 0) {
-    int issued = 0;
-    for (int i = 0; i < nk; ++i) {
-      const int s = i % T::kStages;
-      if (i >= T::kStages && !mbar_wait(empty + s, ((i / T::kStages) - 1) & 1, abort_flag)) break;
-      uint8_t* st = smem + s * T::kStageBytes;
-      mbar_arrive_expect_tx(full + s, T::kStageBytes);
-      tma_load(st, &wmap, i * kBK, f0, full + s);
-      if (GLU) tma_load(st + kWeightTile, &wmap, i * kBK, p.M + f0, full + s);
-      uint8_t* xt = st + (GLU ? 2 : 1) * kWeightTile;
+  if (warp == kTmaWarp) {
+    if (lane == 0) {
+      int s = 0, lap = 0;
+      bool ok = true;
+      for (int tile = first; ok && tile < tiles; tile += step) {
+        const int t0 = tile % nt * BN + (int)rank * T::kRows, f0 = (tile / nt * 2 + (int)rank) * kBM;
+        for (int i = 0; i < nk; ++i) {
+          if (lap > 0 && !(ok = mbar_wait(empty + s, (lap - 1) & 1, abort_flag))) break;
+          uint8_t* st = smem + s * T::kStageBytes;
+          const uint32_t bar = in_first(full + s);
+          if (rank == 0) mbar_arrive_expect_tx(full + s, 2 * T::kStageBytes);
 #pragma unroll
-      for (int b = 0; b < BN / T::kBox; ++b) tma_load(xt + b * T::kBox * kBK * 2, &xmap, i * kBK, t0 + b * T::kBox, full + s);
-      issued = i + 1;
-    }
-    // after a timeout: let the copies in flight land before the memory goes away
-    if (*abort_flag)
-      for (int i = issued > T::kStages ? issued - T::kStages : 0; i < issued; ++i)
-        for (int spin = 0; spin < 1 << 16 && !mbar_try_wait(full + i % T::kStages, (i / T::kStages) & 1); ++spin) {}
-  } else if (warp == kMmaWarp && elect_one()) {
-    for (int i = 0; i < nk; ++i) {
-      const int s = i % T::kStages;
-      if (!mbar_wait(full + s, (i / T::kStages) & 1, abort_flag)) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t st = smem_u32(smem + s * T::kStageBytes);
-      const uint32_t xt = st + (GLU ? 2 : 1) * kWeightTile;
-#pragma unroll
-      for (int k = 0; k < kBK / 16; ++k) {
-        const uint64_t db = operand_desc(xt + 32 * k);
-        mma_bf16(tmem, operand_desc(st + 32 * k), db, kInstrDesc<BN>, i > 0 || k > 0);
-        if (GLU) mma_bf16(tmem + BN, operand_desc(st + kWeightTile + 32 * k), db, kInstrDesc<BN>, i > 0 || k > 0);
+          for (int l = 0; l < SL; ++l) {
+            const int k = (i * SL + l) * kBK;
+            uint8_t* at = st + l * T::kSlabBytes;
+            tma_load(at, &wmap, k, f0, bar);
+            if (GLU) tma_load(at + kWeightTile, &wmap, k, p.M + f0, bar);
+            tma_load(at + (GLU ? 2 : 1) * kWeightTile, &xmap, k, t0, bar);
+          }
+          if (++s == T::kStages) s = 0, ++lap;
+        }
       }
-      mma_commit(empty + s);
+      // every commit to this CTA's barriers has arrived before it leaves
+      for (int e = 0; ok && e < T::kStages; ++e) {
+        const int uses = lap + (e < s);
+        if (uses > 0) ok = mbar_wait(empty + e, (uses - 1) & 1, abort_flag);
+      }
     }
-    mma_commit(done);
-    if (*abort_flag)   // after a timeout: let the MMAs in flight end before the accumulators are freed
-      for (int spin = 0; spin < 1 << 16 && !mbar_try_wait(done, 0); ++spin) {}
-  }
-  __syncwarp();
-  if (warp < 4) {
-    if (mbar_wait(done, 0, abort_flag) && !*abort_flag) {
+  } else if (warp == kMmaWarp) {
+    if (rank == 0 && elect_one()) {
+      int s = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int tile = first, n = 0; ok && tile < tiles; tile += step, ++n) {
+        const int b = n & 1;
+        if (n >= 2 && !mbar_wait(acc_empty + b, ((n >> 1) - 1) & 1, abort_flag)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t acc = tmem + b * T::kAccCols;
+        for (int i = 0; i < nk; ++i) {
+          if (!(ok = mbar_wait(full + s, phase, abort_flag))) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint64_t d0 = operand_desc(smem_u32(smem + s * T::kStageBytes));
+#pragma unroll
+          for (int l = 0; l < SL; ++l) {
+            if (SL > 1 && i * SL + l >= slabs) break;
+#pragma unroll
+            for (int k = 0; k < kBK / 16; ++k) {
+              const uint64_t da = d0 + ((l * T::kSlabBytes + 32 * k) >> 4), db = da + ((GLU ? 2 : 1) * kWeightTile >> 4);
+              mma_bf16(acc, da, db, kInstrDesc<BN>, i > 0 || l > 0 || k > 0);
+              if (GLU) mma_bf16(acc + BN, da + (kWeightTile >> 4), db, kInstrDesc<BN>, i > 0 || l > 0 || k > 0);
+            }
+          }
+          mma_commit(empty + s);
+          if (++s == T::kStages) s = 0, phase ^= 1;
+        }
+        mma_commit(acc_full + b);
+      }
+    }
+  } else {
+    const int quarter = warp & 3, half = warp >> 2;
+    for (int tile = first, n = 0; tile < tiles; tile += step, ++n) {
+      const int b = n & 1, t0 = tile % nt * BN, f0 = (tile / nt * 2 + (int)rank) * kBM;
+      if (!mbar_wait(acc_full + b, (n >> 1) & 1, abort_flag) || *abort_flag) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       __syncwarp();
-      const int f = f0 + warp * 32 + lane;
-      const bool live = f < p.M;
-      const float b0 = live && p.bias ? p.bias[f] : 0.0f, b1 = GLU && live && p.bias ? p.bias[p.M + f] : 0.0f;
-      const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-      const bool sigm = p.act == ACT_SILU_SIGMOID, gelu = p.act == ACT_GLU_GELU, cap = p.act == ACT_SOFTCAP, tail = f >= p.tail;
-      // bf16 outputs turn in shared memory (the stages are free: every copy has landed and been used), 32 features x kCh rows of
-      // a warp at a time, and leave as 16-byte stores
-      constexpr int kCh = BN < 32 ? BN : 32, kTileLd = 40;
-      __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(smem) + warp * 32 * kTileLd;
-      const int f_end = min(p.M, p.tail), fw = f0 + warp * 32;
-      for (int c = 0; c < BN && t0 + c < p.rows; c += kCh) {
-        uint32_t v[kCh], u[GLU ? kCh : 1];
-        tmem_ld(lane_base + c, v);
-        if constexpr (GLU) tmem_ld(lane_base + BN + c, u);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        float o[kCh];
-#pragma unroll
-        for (int j = 0; j < kCh; ++j) {
-          o[j] = __uint_as_float(v[j]) + b0;
-          if constexpr (GLU) {
-            o[j] = (gelu ? gelu_tanhf_(o[j]) : siluf_(o[j])) * (__uint_as_float(u[j]) + b1);
-          } else if (sigm) {
-            const float sg = sigmoidf_(o[j]);
-            o[j] = f < p.act_split ? o[j] * sg : sg;
-          } else if (cap) {
-            o[j] = softcapf_(o[j] * p.out_scale, p.softcap);
-          }
-        }
-        if (live && (tail || !p.yb)) {
-          float* y = tail ? p.tail_y + f - p.tail : p.y + f;
-          const int64_t ld = tail ? p.tail_ld : p.ldy;
-#pragma unroll
-          for (int j = 0; j < kCh; ++j)
-            if (t0 + c + j < p.rows) y[(int64_t)(t0 + c + j) * ld] = o[j];
-        }
-        if (!p.yb) continue;
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < kCh; ++j) tile[j * kTileLd + lane] = __float2bfloat16_rn(o[j]);
-        __syncwarp();
-#pragma unroll
-        for (int i = lane; i < 4 * kCh; i += 32) {
-          const int j = i / 4, q = 8 * (i % 4), n = f_end - fw - q;   // n features of this piece are stored
-          if (t0 + c + j >= p.rows || n <= 0) continue;
-          const __nv_bfloat16* src = tile + j * kTileLd + q;
-          __nv_bfloat16* dst = p.yb + (int64_t)(t0 + c + j) * p.ldy + fw + q;
-          if (n >= 8) {
-            *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
-          } else {
-            for (int e = 0; e < n; ++e) dst[e] = src[e];
-          }
-        }
-      }
+      store_tile<BN, GLU>(p, tmem + b * T::kAccCols, f0, t0, quarter, lane, turn + warp * 32 * kTileLd, half * (BN / 2), (half + 1) * (BN / 2));
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive_at(in_first(acc_empty + b));
     }
   }
+  __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
+  cluster_sync();            // neither frees what the other may still signal
   if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, 1);
   if (warp == kMmaWarp) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(T::kTmemCols) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(T::kTmemCols) : "memory");
   }
 }
 
-template <int BN, bool GLU, bool DEEP>
-cudaError_t launch_tile_stages(const TmaMap& wmap, const TmaMap& xmap, const GemmParams& p, cudaStream_t st) {
-  using T = Tile<BN, GLU, DEEP>;
-  const cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, GLU, DEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kSmem);
+int64_t tiles_of(const GemmParams& p, int bn) { return (int64_t)((p.M + 2 * kBM - 1) / (2 * kBM)) * ((p.rows + bn - 1) / bn); }
+
+template <int BN, bool GLU, int SL>
+cudaError_t launch_tiles(const TmaMap& wmap, const XMaps& x, const GemmParams& p, int pairs, cudaStream_t st) {
+  using T = Tile<BN, GLU, SL>;
+  constexpr int kBox = BN == 32 ? 0 : BN == 64 ? 1 : BN == 128 ? 2 : 3;   // of half of the rows
+  static_assert(kGemmTokenBox << kBox == T::kRows, "box");
+  const cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, GLU, SL>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kSmem);
   if (e != cudaSuccess) return e;
-  gemm_bf16_kernel<BN, GLU, DEEP><<<dim3((p.rows + BN - 1) / BN, (p.M + kBM - 1) / kBM), kThreads, T::kSmem, st>>>(wmap, xmap, p);
+  gemm_bf16_kernel<BN, GLU, SL><<<2 * (int)std::min<int64_t>(tiles_of(p, BN), pairs), kThreads, T::kSmem, st>>>(wmap, x.box[kBox], p);
   return cudaGetLastError();
-}
-
-int64_t tiles_of(const GemmParams& p, int bn) { return (int64_t)((p.M + kBM - 1) / kBM) * ((p.rows + bn - 1) / bn); }
-
-template <int BN, bool GLU>
-cudaError_t launch_tile(const TmaMap& wmap, const TmaMap& xmap, const GemmParams& p, int sm_count, cudaStream_t st) {
-  return tiles_of(p, BN) <= sm_count ? launch_tile_stages<BN, GLU, true>(wmap, xmap, p, st) : launch_tile_stages<BN, GLU, false>(wmap, xmap, p, st);
 }
 
 }  // namespace
@@ -313,23 +399,33 @@ bool encode_bf16_map(TmaMap* map, const __nv_bfloat16* base, int64_t rows, int64
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+bool encode_x_maps(XMaps* x, const __nv_bfloat16* base, int64_t rows, int64_t k, int64_t ld) {
+  for (int i = 0; i < 4; ++i)
+    if (!encode_bf16_map(x->box + i, base, rows, k, ld, kGemmTokenBox << i)) return false;
+  return true;
+}
+
 cudaError_t launch_gemm_bf16(const LinearArgs& a, const TmaMap& wmap, const XMaps& x, float* y, __nv_bfloat16* yb, int64_t ldy, int* status,
                              int sm_count, cudaStream_t st) {
   if (yb && (ldy % 8 != 0 || reinterpret_cast<uintptr_t>(yb) % 16 != 0)) return cudaErrorInvalidValue;
   const bool glu = is_glu(a.act);
   GemmParams p{glu ? a.w.M / 2 : a.w.M, a.w.K, a.rows, a.bias, a.act, a.act_split, y, yb, ldy, status,
                a.out_scale, a.softcap, a.tail, a.tail_y, a.tail_ld};
-  const int R = a.rows;
+  // The width with the least turns x time a turn.  Weights: us a turn of an SM pair at K = 2048 / 4096 / 8192 / 14336:
+  // 32 rows 10.6 / 16.6 / 26.8 / 42, 128 rows 12.6 / 18.6 / 29 / 48, 256 rows 18.7 / 27 / 45 / 72; two matrices at K = 2048: 32 rows 14.6, 64
+  // rows 18.7, 128 rows 22.  (64 rows of one matrix cost within 3 % of 128.)
+  const int pairs = std::max(sm_count / 2, 1);
+  const auto cost = [&](int bn, int weight) { return (tiles_of(p, bn) + pairs - 1) / pairs * weight; };
   if (glu) {
-    if (R <= 16) return launch_tile<16, true>(wmap, x.narrow, p, sm_count, st);
-    if (R <= 64 || tiles_of(p, 64) <= sm_count) return launch_tile<64, true>(wmap, x.narrow, p, sm_count, st);
-    return launch_tile<128, true>(wmap, x.wide, p, sm_count, st);
+    const int64_t c32 = cost(32, 7), c64 = cost(64, 9), c128 = cost(128, 11);
+    if (c32 <= c64 && c32 <= c128) return launch_tiles<32, true, 2>(wmap, x, p, pairs, st);
+    if (c64 < c128) return launch_tiles<64, true, 1>(wmap, x, p, pairs, st);
+    return launch_tiles<128, true, 1>(wmap, x, p, pairs, st);
   }
-  if (R <= 16) return launch_tile<16, false>(wmap, x.narrow, p, sm_count, st);
-  if (R <= 64 || tiles_of(p, 64) <= sm_count) return launch_tile<64, false>(wmap, x.narrow, p, sm_count, st);   // narrower tiles while every one has an SM
-  // 256-row tiles once there are more of them than SMs
-  if (tiles_of(p, 256) >= 180) return launch_tile_stages<256, false, false>(wmap, x.wide, p, st);
-  return launch_tile<128, false>(wmap, x.wide, p, sm_count, st);
+  const int64_t c32 = cost(32, 20), c128 = cost(128, 23), c256 = cost(256, 36);
+  if (c32 <= c128 && c32 <= c256) return launch_tiles<32, false, 2>(wmap, x, p, pairs, st);
+  if (c128 < c256) return launch_tiles<128, false, 2>(wmap, x, p, pairs, st);
+  return launch_tiles<256, false, 1>(wmap, x, p, pairs, st);
 }
 
 }  // namespace emelb

@@ -747,8 +747,7 @@ cudaError_t launch_latent_prompt(const LatentArgs& a, const TmaMap& upmap, const
   // keys and values of the visible positions
   const __nv_bfloat16* base = static_cast<const __nv_bfloat16*>(a.cache) + ((int64_t)rows.seq0 * a.capacity + key0) * a.width;
   XMaps x;
-  if (!encode_bf16_map(&x.narrow, base, keys, a.rank, a.width, kGemmTokenBox) || !encode_bf16_map(&x.wide, base, keys, a.rank, a.width, 128))
-    return cudaErrorInvalidValue;
+  if (!encode_x_maps(&x, base, keys, a.rank, a.width)) return cudaErrorInvalidValue;
   e = launch_gemm_bf16(LinearArgs{a.up, nullptr, ACT_NONE, 0, keys}, upmap, x, nullptr, a.kv, a.kv_ld, status, sm_count, st);
   if (e != cudaSuccess) return e;
   if (a.vdim <= 32) e = launch_prompt_tiles<4>(a, rows, key0, out, ldo, st);

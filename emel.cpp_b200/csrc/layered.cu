@@ -275,8 +275,7 @@ bool check(Layered* m, LayeredRun& r, cudaError_t e, int launches = 1) {
 }
 
 bool x_maps(XMaps* x, const void* base, int64_t rows, int64_t k, int64_t ld) {
-  const bf16* b = static_cast<const bf16*>(base);
-  return encode_bf16_map(&x->narrow, b, rows, k, ld, kGemmTokenBox) && encode_bf16_map(&x->wide, b, rows, k, ld, 128);
+  return encode_x_maps(x, static_cast<const bf16*>(base), rows, k, ld);
 }
 
 // y = act(x W^T + bias) over rows: bf16 operands on the tensor cores, or f32

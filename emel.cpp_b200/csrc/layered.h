@@ -85,7 +85,8 @@ struct TmaMap { alignas(64) unsigned char bytes[128]; };
 // {rows, K} row-major bf16 matrix as K-slabs of 64 elements x box_rows rows
 bool encode_bf16_map(TmaMap* map, const __nv_bfloat16* base, int64_t rows, int64_t k, int64_t ld, int box_rows);
 constexpr int kGemmWeightBox = 128, kGemmTokenBox = 16;
-struct XMaps { TmaMap narrow, wide; };   // the activations as boxes of kGemmTokenBox and of 128 rows
+struct XMaps { TmaMap box[4]; };   // the activations as boxes of kGemmTokenBox << i rows
+bool encode_x_maps(XMaps* x, const __nv_bfloat16* base, int64_t rows, int64_t k, int64_t ld);
 cudaError_t launch_gemm_bf16(const LinearArgs& a, const TmaMap& wmap, const XMaps& x, float* y, __nv_bfloat16* yb, int64_t ldy,
                              int* status, int sm_count, cudaStream_t st);
 

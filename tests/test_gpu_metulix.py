@@ -403,3 +403,20 @@ def test_long_prompts(be, tmp_path, f32):
     for sizes in ([1150], [700, 449, 1], [1, 600, 549], [511, 3, 636]):
         assert_close(mm.row_errors(feed(s, c.tokens, sizes), c.logits), f32, sizes)
     s.close()
+
+
+@pytest.fixture(scope="module")
+def ragged(tmp_path_factory):
+    """10 tiles of 256 gate and up features and of vocabulary, both with a ragged end; K of two and a bit slabs of 64."""
+    cfg = mm.model(136, 2531, [mm.attention(2, 1, 32, 32, 0.5, conv=3, rot=(16, 1000.0), window=50, keep=2, ff=2546)])
+    return Case(cfg, tmp_path_factory.mktemp("ragged"), 2000, 37)
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 100, 300, 1000, 2000])
+def test_products_of_every_tile_width(be, ragged, n):
+    """148 SMs: 32-row tiles to 100 rows, 64 (two matrices) and 128 rows at 300, 128 and 256 at 1000, 128 and more than two tiles
+    a pair of SMs at 2000."""
+    s = ragged.session(be, False, n_ctx=2048)
+    got = s.prefill_logits(ragged.tokens[:n], 0, range(n))
+    assert_close(mm.row_errors(got, ragged.logits[:n]), False, n)
+    s.close()
