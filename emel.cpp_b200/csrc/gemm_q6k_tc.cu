@@ -27,9 +27,12 @@
 // Registers are split by setmaxnreg: 640 threads x 96 at launch = 256 x 80 + 256 x 136 + 128 x 48.
 // Every mbarrier wait is bounded; on a timeout the CTA raises the status word, lets its copies land and frees its TMEM.
 //
-// What bounds it: the epilogue (two warps per scheduler) and the producers, each a chain of dependent steps of 2000 to
-// 2800 cycles a turn; the MMAs take 1040 (64 columns).  Measured, B200, kernel alone: 4096 x 11008 by 77 columns 62 us (the
-// mat-vec kernel that took every K before: 20.2 ms), 12 to 32 columns 96 us.
+// What bounds it: the producers, a chain of dependent steps of about 3,400 cycles a turn, of which the copies into the ring
+// (256 cp.async of a row each a turn) are a large part: as many as twice, for 16 producer warps with a quarter each, made the
+// turn 25 % longer, addresses that step from row to row instead of a product and a minimum per copy 8 % shorter; scales taken
+// apart two in a half2 and odd bytes by a permutation 4 %.  The MMAs take 1040 (64 columns).  Measured, B200, us a
+// call: 4096 x 11008 by 77 columns 66.3 -> 60.2 with the L2 cold before each call; one call behind the other 105 -> 93, 14336 x
+// 11008 by 200 414 -> 363, 11008 x 4096 by 77 82 -> 74, 14336 x 2816 by 16 35.5 -> 31.3.
 // Dispatch: K and rows that the streaming kernels and gemm_q6k_mma.cu do not take (their copies need rows of a multiple
 // of 16 bytes, K % 2048 == 0).  Where both work, many columns are about equal (14336 x 4096 by 2048 columns 944 + 10
 // against 1047 us, 4096 x 14336 by 333: 273 + 7 against 247) and few are faster there (4096 x 14336 by 32: 124 + 3
@@ -178,11 +181,22 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q6k_tc_kernel(const GemmArgs
         // blocks start at any even byte: a half needs up to 30 of the 53 aligned words that cover its block, one a lane
         const int word = lane < 17 ? 16 * n + lane : lane < 26 ? 32 + 8 * n + lane - 17 : lane < 29 ? 48 + 2 * n + lane - 26 : 52;
         if (lane < 30) {
+          // two rows a step: rows may start at odd halves of a word, every other one in the same way.  Rows past M repeat the
+          // last one or the one before; never stored
+          const int last = p.M - 1 - r0;
+          const uintptr_t first = reinterpret_cast<uintptr_t>(p.W) + (size_t)min(r0, p.M - 1) * p.row_bytes + (size_t)ikb * Q6_K_BYTES;
+          uintptr_t s0 = (first & ~uintptr_t(3)) + 4 * word, s1 = ((first + (last > 0 ? p.row_bytes : 0)) & ~uintptr_t(3)) + 4 * word;
+          const uint32_t d = smem_u32(dst) + 4 * lane;
 #pragma unroll 4
-          for (int rr = 0; rr < 32; ++rr) {                      // rows past M repeat the last one; never stored
-            const uintptr_t src = reinterpret_cast<uintptr_t>(p.W) + (size_t)min(r0 + rr, p.M - 1) * p.row_bytes + (size_t)ikb * Q6_K_BYTES;
-            const uint32_t d = smem_u32(dst + rr * kRawRow) + 4 * lane;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"((src & ~uintptr_t(3)) + 4 * word) : "memory");
+          for (int rr = 0; rr < 32; rr += 2) {
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + rr * kRawRow), "l"(s0) : "memory");
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + (rr + 1) * kRawRow), "l"(s1) : "memory");
+            if (rr + 3 <= last) {
+              s0 += 2 * p.row_bytes;
+              s1 += 2 * p.row_bytes;
+            } else if (rr + 2 <= last) {
+              s0 += 2 * p.row_bytes;
+            }
           }
         }
         if (++ikb == nkb) { ikb = 0; itile += gridDim.x; }
@@ -213,18 +227,18 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q6k_tc_kernel(const GemmArgs
       if (n == 0) *reinterpret_cast<uint32_t*>(rm) = sh ? bw[29] >> 16 : bw[29] & 0xffffu;
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
-        // weights 16q .. 16q+15 of each 32: scale 2f + q of the half for form f; sc = 16 hi + lo, both in -8 .. 8
-        __half2 sl[4], cl[4], sh2[4], ch[4];
+        // weights 16q .. 16q+15 of each 32: scale 2f + q of the half for form f, two forms in a half2.  sc + 136 = 16 (hi + 8) +
+        // (lo + 8), with 1024 in front each part is an f16
+        __half2 sl[2], cl[2], sh2[2], ch[2];
 #pragma unroll
-        for (int f = 0; f < 4; ++f) {
-          const int b = 2 * f + q;
-          const int sc = (int)(int8_t)(sw[b >> 2] >> (8 * (b & 3)));
-          const int hi = (sc + 8) >> 4, lo = sc - 16 * hi;
-          const __half2 l2 = __half2half2(__int2half_rn(lo)), h2v = __half2half2(__int2half_rn(hi));
-          sl[f] = __hmul2(l2, __float2half2_rn(1024.0f));
-          cl[f] = __hmul2(l2, __float2half2_rn(-0.001953125f));   // -32 * 2^-14
-          sh2[f] = __hmul2(h2v, __float2half2_rn(1024.0f));
-          ch[f] = __hmul2(h2v, __float2half2_rn(-0.001953125f));
+        for (int e = 0; e < 2; ++e) {
+          const uint32_t u = (((sw[e] >> (8 * q)) & 0x00ff00ffu) ^ 0x00800080u) + 0x00080008u;
+          const __half2 lo = __hsub2(bits_h2((u & 0x000f000fu) | 0x64006400u), __float2half2_rn(1032.0f));
+          const __half2 hi = __hsub2(bits_h2(((u >> 4) & 0x001f001fu) | 0x64006400u), __float2half2_rn(1032.0f));
+          sl[e] = __hmul2(lo, __float2half2_rn(1024.0f));
+          cl[e] = __hmul2(lo, __float2half2_rn(-0.001953125f));   // -32 * 2^-14
+          sh2[e] = __hmul2(hi, __float2half2_rn(1024.0f));
+          ch[e] = __hmul2(hi, __float2half2_rn(-0.001953125f));
         }
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
@@ -235,11 +249,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q6k_tc_kernel(const GemmArgs
                                  ((qa >> 4) & 0x0f0f0f0fu) | (qh & 0x30303030u), ((qb >> 4) & 0x0f0f0f0fu) | ((qh >> 2) & 0x30303030u)};
 #pragma unroll
           for (int f = 0; f < 4; ++f) {
-            const uint32_t e = v[f] & 0x00ff00ffu, d = (v[f] >> 8) & 0x00ff00ffu;
-            ol[2 * f] = expand2(e, sl[f], cl[f]);
-            ol[2 * f + 1] = expand2(d, sl[f], cl[f]);
-            oh[2 * f] = expand2(e, sh2[f], ch[f]);
-            oh[2 * f + 1] = expand2(d, sh2[f], ch[f]);
+            const uint32_t e = v[f] & 0x00ff00ffu, d = __byte_perm(v[f], 0, 0x4341);
+            const __half2 l = f & 1 ? __high2half2(sl[f >> 1]) : __low2half2(sl[f >> 1]), lc = f & 1 ? __high2half2(cl[f >> 1]) : __low2half2(cl[f >> 1]);
+            const __half2 h = f & 1 ? __high2half2(sh2[f >> 1]) : __low2half2(sh2[f >> 1]), hc = f & 1 ? __high2half2(ch[f >> 1]) : __low2half2(ch[f >> 1]);
+            ol[2 * f] = expand2(e, l, lc);
+            ol[2 * f + 1] = expand2(d, l, lc);
+            oh[2 * f] = expand2(e, h, hc);
+            oh[2 * f + 1] = expand2(d, h, hc);
           }
           tmem_st8(a_lane + 8u * i, ol);
           tmem_st8(a_lane + 128u + 8u * i, oh);
