@@ -31,7 +31,7 @@
 // (256 cp.async of a row each a turn) are a large part: as many as twice, for 16 producer warps with a quarter each, made the
 // turn 25 % longer, addresses that step from row to row instead of a product and a minimum per copy 8 % shorter; scales taken
 // apart two in a half2 and odd bytes by a permutation 4 %.  The MMAs take 1040 (64 columns).  Measured, B200, us a
-// call: 4096 x 11008 by 77 columns 66.3 -> 60.2 with the L2 cold before each call; one call behind the other 105 -> 93, 14336 x
+// call: 4096 x 11008 by 77 columns 66.3 -> 60.2 (a call by itself; one behind the other 105 -> 93), 14336 x
 // 11008 by 200 414 -> 363, 11008 x 4096 by 77 82 -> 74, 14336 x 2816 by 16 35.5 -> 31.3.
 // Dispatch: K and rows that the streaming kernels and gemm_q6k_mma.cu do not take (their copies need rows of a multiple
 // of 16 bytes, K % 2048 == 0).  Where both work, many columns are about equal (14336 x 4096 by 2048 columns 944 + 10
