@@ -34,6 +34,7 @@ SOURCES = {
     "gemm_q6k_wide.cu": [],
     "linear.cu": [],
     "gemm_bf16.cu": [],
+    "gemm_q8_tc.cu": [],
     "mixer_ops.cu": [],
     "mixed_attention.cu": [],
     "lightning.cu": [],

@@ -5,7 +5,7 @@
 // mma.sync.m16n8k32 (s8 x s8 -> s32) gives the 32-term integer sums of 16 rows x 8 columns, and the CUDA
 // cores apply the two scales and add the blocks up in ascending order with the reference's roundings — the
 // same bits as the mat-vec kernels — two columns per instruction on the packed f32x2 pipe.  The scaling, 4 float operations per product and block, bounds the
-// kernel, not the MMAs; a tcgen05 tile would only move the same scaling work behind a TMEM load.
+// kernel, not the MMAs.  Prompts with long sums run on tcgen05 (gemm_q8_tc.cu).
 //
 // One CTA = 128 (or, for small grids, 64) weight rows x 64 activation columns, one warp per 16 rows; K is walked in chunks of 8
 // blocks through a two-stage cp.async ring.  Weight rows are staged as they lie in memory (scale + quants,

@@ -8,7 +8,7 @@
 // This file holds the dispatch (launch_gemv), the generic kernel for shapes the
 // streaming kernels do not take (K not a multiple of 2048, unaligned rows) and the
 // argmax helpers; the streaming kernels are in gemv2.cu, the many-column
-// tensor-core kernels in gemm_tc.cu and gemm_q8_mma.cu.
+// tensor-core kernels in gemm_tc.cu, gemm_q8_tc.cu, gemm_q8_mma.cu and the gemm_q6k files.
 //
 // Float order, all kernels.  The integers of a block are exact whatever the order;
 // the f32 part follows the reference's x86 route literally: one value per block —
@@ -226,6 +226,8 @@ bool gemv_takes_tensor_core(int type, const GemvArgs& a, int ncols) {
 
 cudaError_t launch_gemv(int type, const GemvArgs& a, int ncols, bool argmax, int sm_count, cudaStream_t st,
                         int* launches) {
+  // prompts, Q8_0 / Q4_0: three tcgen05 instructions per 32-weight block (gemm_q8_tc.cu)
+  if (!argmax && gemm_q8_tc_supported(type, a, ncols, sm_count)) return launch_gemm_q8_tc(type, a, ncols, sm_count, st, launches);
   // many columns of Q8_0 / Q4_0: one tensor-core instruction per 32-weight block (gemm_q8_mma.cu)
   if (!argmax && gemm_q8_mma_supported(type, a, ncols)) {
     ++*launches;

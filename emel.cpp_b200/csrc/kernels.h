@@ -127,6 +127,10 @@ bool gemv_takes_tensor_core(int type, const GemvArgs& a, int ncols);
 bool gemm_q8_mma_supported(int type, const GemvArgs& a, int ncols);
 cudaError_t launch_gemm_q8_mma(int type, const GemvArgs& a, int ncols, int sm_count, cudaStream_t st);
 
+// gemm_q8_tc.cu: prompts, Q8_0 / Q4_0 weights on tcgen05; lays the planes out in the tensor-core workspace
+bool gemm_q8_tc_supported(int type, const GemvArgs& a, int ncols, int sm_count);
+cudaError_t launch_gemm_q8_tc(int type, const GemvArgs& a, int ncols, int sm_count, cudaStream_t st, int* launches);
+
 // gemm_q6k_mma.cu: nine and more columns of Q6_K weights, K % 2048 == 0 (mma.sync int8, one scale group per instruction)
 bool gemm_q6k_mma_supported(int type, const GemvArgs& a, int ncols);
 cudaError_t launch_gemm_q6k_mma(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st);
@@ -241,6 +245,7 @@ constexpr int kGemmTcMinCols = 32;
 constexpr int kGemmQ6kTcMinCols = 5;   // Q6_K rows that no streaming kernel takes: fewer columns run gemv_odd_kernel (and so do more of a small matrix: gemm_q6k_tc.cu)
 constexpr int kGemmMmaMinCols = 9;   // Q6_K: fewer columns run the CUDA-core mat-vec kernels (7 and 8: gemm_q6k_mma.cu)
 constexpr int kGemmQ4kMmaMinCols = 5; // Q4_K: 8 columns take 39 / 63 us through the mat-vec kernel, 23-28 / 35 us through the mma.sync one (4096x14336 / 14336x4096)
+constexpr int kGemmQ8TcMinCols = 33;   // Q8_0 / Q4_0 prompts; up to 32 columns gemm_q8_mma.cu has tiles of its own width
 constexpr int kGemmQ8MmaMinCols = 3; // Q8_0 / Q4_0: from three columns on the mma.sync kernel (21-24 us for up to 8 columns of 14336x4096) beats the mat-vec kernels (29 us at 4 columns)
 // activations of the tcgen05 kernels in the workspace: columns of f16 in swizzle atoms of 8 columns x 64 K, {dx, dx, mean, mean} a
 // column pair and, as f16, the 16 block sums a column

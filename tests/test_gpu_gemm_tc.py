@@ -250,3 +250,28 @@ def test_q4_k_columns_in_turns(port, monkeypatch):
         assert np.array_equal(dev_y.cpu().numpy().view(np.uint32), want.view(np.uint32))
     finally:
         b.close()
+
+
+@pytest.mark.parametrize("t", [eb.Q8_0, eb.Q4_0])
+@pytest.mark.parametrize("k,m,n,launches", [
+    (5376, 4801, 33, 3), (5120, 130, 1601, 3), (5120, 1300, 333, 3),      # one turn of tiles, ragged rows and columns
+    (2304, 2500, 900, 3),                                                  # several tiles a CTA, odd turns of K
+    (4096, 1300, 192, 2), (2304, 2500, 800, 2), (3840, 1300, 333, 2),      # on the other side of each line: mma.sync
+    (4096, 1300, 333, {eb.Q8_0: 3, eb.Q4_0: 2}),                           # tiles for two thirds of the SMs
+])
+def test_q8_0_and_q4_0_prompts(be, port, t, k, m, n, launches):
+    w = synth.random_blocks(t, m + n, m, k)
+    x = synth.activations_f32(m * n, k, n).reshape(k, n)
+    assert launches_of(be, lambda: check(be, port, t, w, k, m, x, n)) == (launches if isinstance(launches, int) else launches[t])      # quantizer, (operand layout,) product
+
+
+@pytest.mark.parametrize("t", [eb.Q8_0, eb.Q4_0])
+def test_q8_0_and_q4_0_prompts_largest_sums(be, port, t):
+    """Quants and activations at the ends of their range; scales from subnormal to large, of either sign."""
+    k, m, n = 5120, 1300, 260
+    b = np.zeros((m * k // 32, eb.BLOCK_BYTES[t]), np.uint8)
+    i = np.arange(len(b))
+    d = np.array([2.0 ** -24, -2.0 ** -14, 0.5, -8.0, 0.0], np.float16)[i % 5]
+    b[:, :2] = d.view(np.uint8).reshape(-1, 2)
+    b[:, 2:] = np.array([0x80, 0x7f, 0xff, 0x00, 0x88], np.uint8)[i // 5 % 5][:, None]
+    check(be, port, t, b.reshape(-1), k, m, one_sided(k, n), n)
