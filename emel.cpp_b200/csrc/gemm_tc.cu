@@ -24,8 +24,7 @@
 //               expands its row's half into TMEM, 64 weights at a time
 //   warps 8-15  epilogue: two warps per TMEM lane quarter, half of the columns each, a thread a row: the row's constants stay
 //               in registers, the float chain runs on packed f32x2 instructions
-//   warp  16    the MMAs of a super-block; TMEM allocation
-//   warp  17    the msum instructions
+//   warps 16, 17 MMA issue, msum included, half of the columns each; TMEM allocation
 //   warp  18    copies of the weights (TMA, 128 rows x 144 bytes) and of the activations, a quarter super-block each
 //   warp  19    copies of block sums, column scales and table
 // TMEM at TN = 128: two turns' accumulators (256 columns), msum of one turn (128, made and read in two parts, so that
@@ -43,7 +42,8 @@
 // before and now: 14336 x 4096 by 32 columns 47.7 -> 30.5, by 128 48.4 -> 44.6, by 512 159 -> 118; 4096 x 14336 by 32 134 -> 78,
 // by 333 136 -> 104, by 1900 517 -> 354; 1024 x 4096 by 333 47.6 -> 31.4.  What gave it: TMEM loads of whole lanes (32x32b, half
 // a cycle a register against two of 16x256b: 16 % of the product without its arithmetic), roles in few instructions (the
-// producers' loop not unrolled 374 -> 349), the table (233 -> 188 million instructions).  Without effect: tiles of 96 columns with
+// producers' loop not unrolled 374 -> 349), the table (233 -> 188 million instructions), the second MMA warp (a call, quantizer
+// included, 385 -> 372; the figures above are from before it).  Without effect: tiles of 96 columns with
 // msum double-buffered (400), 16 epilogue warps (355), copies or MMAs left out (the memories and the tensor core wait).
 #include <cuda.h>
 #include <cudaTypedefs.h>
