@@ -677,8 +677,10 @@ bool gemm_tc_supported(int type, int K, int ncols, const void* W, int64_t row_by
          row_bytes < (1 << 27) && planes_aligned(act);
 }
 
+namespace {
+
 // the weights as bytes {rows, K/256 * 144}, boxes of 128 rows x one block
-static bool encode_rows(CUtensorMap* map, const GemvArgs& a) {
+bool encode_rows(CUtensorMap* map, const GemvArgs& a) {
   static const PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
     void* fn = nullptr;
     cudaDriverEntryPointQueryResult q;
@@ -695,7 +697,7 @@ static bool encode_rows(CUtensorMap* map, const GemvArgs& a) {
 }
 
 template <int TN, bool kTable>
-static cudaError_t launch_tiles(const GemmArgs& g, const CUtensorMap& wmap, int sm_count, cudaStream_t st) {
+cudaError_t launch_tiles(const GemmArgs& g, const CUtensorMap& wmap, int sm_count, cudaStream_t st) {
   constexpr int kSmem = Cfg<TN, kTable>::kSmemBytes;
   // per host thread (one context, one lane per thread): no shared mutable state between lanes
   static thread_local unsigned configured = 0;  // one bit per device
@@ -713,13 +715,27 @@ static cudaError_t launch_tiles(const GemmArgs& g, const CUtensorMap& wmap, int 
 
 // Columns per tile: the fewest waves of CTAs, weighted with what a wave takes (4096 x 14336, one wave: 78, 88 and 97 us with
 // tiles of 32, 64 and 128 columns; 1024 x 4096: 31, 34.5 and 40).  Each is up to 1.4 times as fast as the others somewhere
-static int tile_columns(int M, int ncols, int sm_count, bool wide) {
+int tile_columns(int M, int ncols, int sm_count, bool wide) {
   const int mt = (M + BM - 1) / BM;
   auto waves = [&](int tn) { return (mt * ((ncols + tn - 1) / tn) + sm_count - 1) / sm_count; };
   const int c128 = 100 * waves(128), c64 = 90 * waves(64), c32 = 81 * waves(32);
   if (wide && ncols > 64 && c128 <= c64 && c128 <= c32) return 128;
   return c64 <= c32 ? 64 : 32;
 }
+
+size_t table_bytes(const GemvArgs& a) { return (size_t)((a.M + BM - 1) / BM) * (a.K / QK_K) * kTableBytes; }
+bool table_fits(const GemvArgs& a) { return table_bytes(a) + gemm_tc_workspace_bytes(a.K, 128) <= a.tc_ws_bytes; }
+
+// columns of a turn: what the workspace holds beside the rows' table, and a grid's y extent; ncols where one turn takes all
+int turn_columns(const GemvArgs& a, int ncols) {
+  const size_t group = gemm_tc_workspace_bytes(a.K, 128), groups = (table_fits(a) ? a.tc_ws_bytes - table_bytes(a) : a.tc_ws_bytes) / group;
+  const int fit = (int)(groups < 32767 ? groups : 32767) * 128;
+  return fit >= ncols || (ncols <= 64 && fit == 0) ? ncols : fit;   // a single group of 64 columns may fit where 128 do not
+}
+
+}  // namespace
+
+bool gemm_q4k_tc_one_turn(const GemvArgs& a, int ncols) { return turn_columns(a, ncols) == ncols; }
 
 // launches: the activation pre-pass (into the workspace), the pre-pass over the weights where several column tiles share
 // its results, and the product; the three again for columns whose operand the workspace does not hold beside the others'
@@ -731,14 +747,7 @@ cudaError_t launch_gemm_q4k_tc(const GemvArgs& a, int ncols, int sm_count, cudaS
   g.K = a.K;
   g.ldy = a.ldy;
   g.status = a.status;
-  const int nkb = a.K / QK_K, mt = (a.M + BM - 1) / BM;
-  const size_t table_bytes = (size_t)mt * nkb * kTableBytes;
-  // columns of a turn: what the workspace holds, and a grid's y extent
-  const size_t group = gemm_tc_workspace_bytes(a.K, 128);
-  auto columns = [&](size_t room) { return (int)(room / group < 32767 ? room / group : 32767) * 128; };
-  const bool table_fits = table_bytes + group <= a.tc_ws_bytes;
-  int fit = columns(table_fits ? a.tc_ws_bytes - table_bytes : a.tc_ws_bytes);
-  if (fit >= ncols || (ncols <= 64 && fit == 0)) fit = ncols;   // a single group of 64 columns may fit where 128 do not
+  const int nkb = a.K / QK_K, mt = (a.M + BM - 1) / BM, fit = turn_columns(a, ncols);
   CUtensorMap wmap;
   if (!encode_rows(&wmap, a)) return cudaErrorNotSupported;
   for (int c = 0; c < ncols; c += fit) {
@@ -757,7 +766,7 @@ cudaError_t launch_gemm_q4k_tc(const GemvArgs& a, int ncols, int sm_count, cudaS
       ++*launches;
       if (e != cudaSuccess) return e;
     }
-    const int tn = tile_columns(a.M, g.N, sm_count, table_fits && mt <= 65535);
+    const int tn = tile_columns(a.M, g.N, sm_count, table_fits(a) && mt <= 65535);
     if (tn == 128) {
       q4k_table_kernel<<<dim3(nkb, mt), BM, 0, st>>>(a.W, a.row_bytes, a.M, table);
       ++*launches;

@@ -103,7 +103,7 @@ struct GemvArgs {
   const JoinOut* join_out;   // device memory; null: none
   uint8_t* tc_ws;        // workspace of the many-column tensor-core kernel (null: that kernel is not used)
   size_t tc_ws_bytes;
-  int tc_ws_reuse;       // the previous many-column Q4_K product of this stream used the same planes, K, columns and col0
+  int tc_ws_reuse;       // tc_ws holds all columns of these planes in operand order: the Q4_K product before took them (same K, columns, col0) in one turn
   int* sched;            // {next task, finished blocks}: zero between launches (self-rearming)
   int* status;           // optional: set to 1 by a kernel whose bounded wait ran out
   int pdl;               // launch with programmatic stream serialization (kernels wait before dependent reads)
@@ -267,6 +267,9 @@ bool gemm_tc_supported(int type, int K, int ncols, const void* W, int64_t row_by
 // true when launch_gemv would run the kernel that honours GemvArgs::pro_x for this matrix
 bool gemv_prologue_supported(int type, const void* w, int64_t row_bytes, int K);
 size_t gemm_tc_workspace_bytes(int K, int ncols);
+// false: the columns go in turns, and only the last turn's operand stays in the workspace.  How many a turn takes depends on the
+// rows too, whose table shares the workspace
+bool gemm_q4k_tc_one_turn(const GemvArgs& a, int ncols);
 cudaError_t launch_gemm_q4k_tc(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st, int* launches);
 
 cudaError_t launch_argmax_pair_store(const float* best_val, const int* best_idx, int row_offset, int* pair, cudaStream_t st);

@@ -561,7 +561,7 @@ struct Enqueue {
     // Q4_K product of the same input
     const bool tc = gemv_takes_tensor_core(w.type, a, B);
     a.tc_ws_reuse = tc && batch_tc_tiled ? 1 : 0;
-    if (tc) batch_tc_tiled = true;
+    if (tc) batch_tc_tiled = gemm_q4k_tc_one_turn(a, B);   // else its last columns only
     else if (gemm_q6k_wide_supported(w.type, a, B, s->c->sm_count) || gemm_q6k_tc_supported(w.type, a, B)) batch_tc_tiled = false;   // lay their own copy over it
     a.sched = s->c->next_sched();
     a.status = s->c->status_word();

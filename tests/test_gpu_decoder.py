@@ -281,3 +281,39 @@ def test_batched_prompt_fills_the_context_to_the_last_row(be, port):
         assert np.array_equal(again.view(np.uint32), base.view(np.uint32))
     finally:
         sess.close()
+
+
+def test_batched_prompt_whose_query_product_takes_turns(port, monkeypatch):
+    """Width 16384 with a small workspace: 512 tokens of the query projection go in two turns (its table of 16384 rows leaves
+    room for 384 columns), those of the key and value projections in one.  Of the first turn nothing may be taken for theirs.
+    One layer, so bit-identical to batches of 128 tokens, which every product takes in one turn.  Weights of N(0, 0.005): scores of
+    a few tenths, so that every position counts."""
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("EMELB_ACT_MELEMS", "8")
+    b = eb.Backend(0)
+    cfg = el.config(1, 16384, 128, 8, 128, 256, 512, 576)
+    sess = el.Session(b, cfg)
+    keep = []
+    try:
+        ones = torch.ones(16384, device="cuda")
+        for layer, role in ((-1, el.TOKEN_EMBD), (-1, el.OUTPUT), (0, el.ATTN_Q), (0, el.ATTN_K), (0, el.ATTN_V), (0, el.ATTN_OUT), (0, el.FFN_GATE),
+                            (0, el.FFN_UP), (0, el.FFN_DOWN)):
+            k, m = el.matrix_shapes(cfg)[role]
+            values = synth.rng(40 + 7 * layer + role).standard_normal((997, 256), dtype=np.float32) * np.float32(1.0 if role == el.TOKEN_EMBD else 0.005)
+            w = torch.from_numpy(port.encode_rows(eb.Q4_K, values, 256, 997).reshape(997, -1)).cuda()
+            w = w[torch.arange(m * k // 256, device="cuda") * (2 * role + 5) % 997].contiguous().view(-1)
+            keep.append(w)
+            assert sess.bind_matrix(layer, role, w, eb.Q4_K), sess.last_error
+        for layer, role in ((-1, el.OUTPUT_NORM), (0, el.ATTN_NORM), (0, el.FFN_NORM)):
+            assert sess.bind_norm(layer, role, ones), sess.last_error
+        torch.cuda.synchronize()
+        prompt = synth.rng(43).integers(0, 512, size=513).tolist()
+        base = _prompt_then_logits(b, sess, prompt, [128] * 4)
+        assert sess.prefill(synth.rng(5).integers(0, 512, size=512).tolist(), 0)    # scrub
+        got = _prompt_then_logits(b, sess, prompt, [512])
+        assert b.sync()
+        assert np.isfinite(base).all() and base.std() > 0
+        assert np.array_equal(got.view(np.uint32), base.view(np.uint32)), _rel(got, base)
+    finally:
+        sess.close()
+        b.close()
