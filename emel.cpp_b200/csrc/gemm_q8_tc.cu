@@ -31,6 +31,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "q8_tc_order.h"
 #include "tc_common.cuh"
 
 namespace emelb {
@@ -39,7 +40,7 @@ namespace {
 using namespace tc;
 
 constexpr int BM = 128, TN = 64, kBlocks = 8, kTurnK = kBlocks * QK32;
-constexpr int kProducerWarps = 8, kEpilogueWarps = 16, kMmaWarp = 24, kMmaWarps = 3, kLoaderWarp = 27;
+constexpr int kProducerWarps = 8, kEpilogueWarps = 16, kMmaWarp = 24, kMmaWarps = q8tc::kMmaWarps, kLoaderWarp = 27;
 constexpr int kThreads = 28 * 32;
 constexpr int kProducerRegs = 96, kEpilogueRegs = 64, kOtherRegs = 48;
 static_assert(kProducerWarps * kProducerRegs + kEpilogueWarps * kEpilogueRegs + 4 * kOtherRegs <= 28 * 72, "register split");
@@ -246,8 +247,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q8_tc_kernel(const GemmArgs 
       uint32_t fresh = 1;              // parity of d_free
       for (int g = r; g < blocks; g += kMmaWarps) {
         const uint32_t pair = (uint32_t)(g >> 1) & 1u;
-        live = mbar_wait(x_full + 8 * xs, xphase, abort_flag) && mbar_wait(a_full + 8 * pair, (uint32_t)(g >> 2) & 1u, abort_flag) &&
-               mbar_wait(d_free + 8 * r, fresh, abort_flag);
+        live = q8tc::wait_for_block(g, xs, xphase, fresh, [&](q8tc::Barrier what, int index, uint32_t parity) {
+          return mbar_wait((what == q8tc::kXFull ? x_full : what == q8tc::kDFree ? d_free : a_full) + 8 * index, parity, abort_flag);
+        });
         if (!live) break;
         fence_after();
         const uint64_t x = x0 + (uint64_t)((xs * kXBytes + (b >> 1) * kChunkBytes + (b & 1) * 64) >> 4);
