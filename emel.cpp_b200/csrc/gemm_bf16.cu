@@ -19,7 +19,8 @@
 // stage where shared memory has room for enough of these).
 // Short sums: a cluster's start costs 1 to 2 us more than a CTA's, tiles of many rows win it back (K = 512: 2048 features, 1500 rows
 // 10.4 -> 12.4; 14336 features, 8 rows 6.3 -> 7.6, 2048 rows 47 -> 39).
-// Every wait is bounded; on a timeout the CTA raises the status word, lets its copies land and frees its TMEM.
+// Every wait is bounded; when one runs out both CTAs stop, let the copies and MMAs in flight end, raise the status word and free
+// their TMEM.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
@@ -30,9 +31,16 @@
 #include "common.cuh"
 #include "layered.h"
 
+// true: the wait of `role` of CTA `rank` in front of its use (or tile) `use` is taken to have run out.  Nothing but a test, which
+// compiles this file for itself, says so (tests/gemm_bf16_giveup_harness.cu)
+#ifndef EMELB_GIVE_UP
+#define EMELB_GIVE_UP(rank, role, use) false
+#endif
+
 namespace emelb {
 namespace {
 
+enum Role : int { kCopies, kMmas, kMmaTiles, kStores };
 constexpr int kEpilogueWarps = 8, kTmaWarp = 8, kMmaWarp = 9, kThreads = 320;
 constexpr int kBM = kGemmWeightBox, kBK = 64;
 constexpr int kWeightTile = kBM * kBK * 2;
@@ -206,6 +214,16 @@ __device__ __forceinline__ uint32_t in_first(const void* ptr) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(ptr)));
   return a;
 }
+// a word of the other CTA's shared memory, at the place that ptr has in this one's
+__device__ __forceinline__ void store_at(const volatile int* ptr, uint32_t rank, int v) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(const_cast<const int*>(ptr))), "r"(rank));
+  asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+// stands in for copies that nobody asked for
+__device__ __forceinline__ void mbar_complete_tx(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void prefetch_map(const TmaMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
@@ -238,6 +256,41 @@ __device__ __forceinline__ void mbar_arrive_at(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+// a wait of this CTA ran out: both are told
+__device__ __noinline__ void give_up(volatile int* abort_flag, uint32_t rank) {
+  *abort_flag = 1;
+  store_at(abort_flag, rank ^ 1u, 1);
+}
+
+// After a wait that ran out, when no role of either CTA issues any more: MMAs and copies in flight end, bounded.  All threads
+// of both CTAs call it.  (This and give_up are calls, and so out of the way: inlined they cost short products 0.3 to 1 us.)
+__device__ __noinline__ void end_in_flight(uint32_t rank, bool mma_warp, bool copier, bool leader, int issued, uint64_t* full, int stages,
+                                           uint32_t stage_bytes, uint64_t* drained, volatile int* second_issued) {
+  if (mma_warp) {
+    if (leader) mma_commit(drained);
+    if ((threadIdx.x & 31) == 0)
+      for (int spin = 0; spin < 1 << 16 && !mbar_try_wait(drained, 0); ++spin) {}
+  }
+  if (copier && rank == 1) store_at(second_issued, 0, issued);
+  __syncwarp();
+  cluster_sync();
+  if (copier && rank == 0) {
+    // The two may have stopped at different stages, at most `stages` apart (a stage comes free through MMAs that read both
+    // CTAs' copies); where one did not ask for copies, the first CTA stands in for its share of the barrier
+    const int other = *second_issued, both = min(issued, other), any = max(issued, other);
+    for (int i = max(0, any - stages); i < any; ++i) {
+      uint64_t* bar = full + i % stages;
+      if (i >= both) {
+        if (issued > other) mbar_complete_tx(bar, stage_bytes);
+        else mbar_arrive_expect_tx(bar, stage_bytes);
+      }
+      for (int spin = 0; spin < 1 << 16 && !mbar_try_wait(bar, (i / stages) & 1); ++spin) {}
+    }
+  }
+  __syncwarp();
+  cluster_sync();
+}
+
 template <int BN, bool GLU, int SL>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     gemm_bf16_kernel(const __grid_constant__ TmaMap wmap, const __grid_constant__ TmaMap xmap, const GemmParams p) {
@@ -249,8 +302,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   uint64_t* empty = full + T::kStages;       // of either: the MMAs are done with the stage
   uint64_t* acc_full = empty + T::kStages;   // of either: a tile's accumulators stand
   uint64_t* acc_empty = acc_full + 2;        // of the first CTA: both have read theirs
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint64_t* drained = acc_empty + 2;         // of either, only after a wait that ran out: all MMAs are done
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);   // set in both or in neither
+  volatile int* second_issued = abort_flag + 1;                                // of the first, after a wait that ran out
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
   const int slabs = (p.K + kBK - 1) / kBK, nk = (slabs + SL - 1) / SL;
@@ -266,6 +321,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       mbar_init(acc_full + b, 1);
       mbar_init(acc_empty + b, 2 * kEpilogueWarps);
     }
+    mbar_init(drained, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -282,6 +338,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   cluster_sync();            // the barriers and accumulators of both CTAs stand
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  const auto wait = [&](uint64_t* bar, uint32_t parity, Role role, int use) {
+    if (!EMELB_GIVE_UP(rank, role, use) && mbar_wait(bar, parity, abort_flag)) return true;
+    give_up(abort_flag, rank);
+    return false;
+  };
+  int issued = 0;         // stages that this CTA asked copies for (the copying thread)
+  bool leader = false;    // the thread that issues the pair's MMAs
 
   if (warp == kTmaWarp) {
     if (lane == 0) {
@@ -290,7 +353,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       for (int tile = first; ok && tile < tiles; tile += step) {
         const int t0 = tile % nt * BN + (int)rank * T::kRows, f0 = (tile / nt * 2 + (int)rank) * kBM;
         for (int i = 0; i < nk; ++i) {
-          if (lap > 0 && !(ok = mbar_wait(empty + s, (lap - 1) & 1, abort_flag))) break;
+          if ((lap > 0 || EMELB_GIVE_UP(rank, kCopies, s)) && !(ok = wait(empty + s, (lap - 1) & 1, kCopies, lap * T::kStages + s))) break;
           uint8_t* st = smem + s * T::kStageBytes;
           const uint32_t bar = in_first(full + s);
           if (rank == 0) mbar_arrive_expect_tx(full + s, 2 * T::kStageBytes);
@@ -305,24 +368,26 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           if (++s == T::kStages) s = 0, ++lap;
         }
       }
+      issued = lap * T::kStages + s;
       // every commit to this CTA's barriers has arrived before it leaves
       for (int e = 0; ok && e < T::kStages; ++e) {
         const int uses = lap + (e < s);
-        if (uses > 0) ok = mbar_wait(empty + e, (uses - 1) & 1, abort_flag);
+        if (uses > 0) ok = wait(empty + e, (uses - 1) & 1, kCopies, issued + e);
       }
     }
   } else if (warp == kMmaWarp) {
-    if (rank == 0 && elect_one()) {
-      int s = 0;
+    leader = rank == 0 && elect_one();
+    if (leader) {
+      int s = 0, use = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = first, n = 0; ok && tile < tiles; tile += step, ++n) {
+      for (int tile = first, n = 0; tile < tiles; tile += step, ++n) {
         const int b = n & 1;
-        if (n >= 2 && !mbar_wait(acc_empty + b, ((n >> 1) - 1) & 1, abort_flag)) break;
+        if (n >= 2 && !wait(acc_empty + b, ((n >> 1) - 1) & 1, kMmaTiles, n)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem + b * T::kAccCols;
-        for (int i = 0; i < nk; ++i) {
-          if (!(ok = mbar_wait(full + s, phase, abort_flag))) break;
+        for (int i = 0; i < nk; ++i, ++use) {
+          if (!(ok = wait(full + s, phase, kMmas, use))) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint64_t d0 = operand_desc(smem_u32(smem + s * T::kStageBytes));
 #pragma unroll
@@ -338,6 +403,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           mma_commit(empty + s);
           if (++s == T::kStages) s = 0, phase ^= 1;
         }
+        if (!ok) break;            // accumulators that are not whole are nobody's
         mma_commit(acc_full + b);
       }
     }
@@ -345,7 +411,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     const int quarter = warp & 3, half = warp >> 2;
     for (int tile = first, n = 0; tile < tiles; tile += step, ++n) {
       const int b = n & 1, t0 = tile % nt * BN, f0 = (tile / nt * 2 + (int)rank) * kBM;
-      if (!mbar_wait(acc_full + b, (n >> 1) & 1, abort_flag) || *abort_flag) break;
+      if (!__all_sync(0xffffffffu, wait(acc_full + b, (n >> 1) & 1, kStores, n))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       __syncwarp();
       store_tile<BN, GLU>(p, tmem + b * T::kAccCols, f0, t0, quarter, lane, turn + warp * 32 * kTileLd, half * (BN / 2), (half + 1) * (BN / 2));
@@ -357,6 +423,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   cluster_sync();            // neither frees what the other may still signal
+  if (__any_sync(0xffffffffu, *abort_flag)) {
+    end_in_flight(rank, warp == kMmaWarp, warp == kTmaWarp && lane == 0, leader, issued, full, T::kStages, T::kStageBytes, drained, second_issued);
+  }
   if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, 1);
   if (warp == kMmaWarp) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
