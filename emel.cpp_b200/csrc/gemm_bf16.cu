@@ -17,9 +17,9 @@
 // 200 rows 49 -> 27.  Bounds: large products the tensor cores, few rows the chain of a wait, the MMAs and a commit per stage
 // (about 290 cycles beside the MMAs' own, whether addresses are constants of an unrolled loop or not, hence two slabs of K a
 // stage where shared memory has room for enough of these).
-// Short sums: a cluster's start costs 1 to 2 us more than a CTA's, tiles of many rows win it back (K = 512: 2048 features, 1500 rows
-// 10.4 -> 12.4; 14336 features, 8 rows 6.3 -> 7.6, 2048 rows 47 -> 39).
-// Every wait is bounded; when one runs out both CTAs stop, let the copies and MMAs in flight end, raise the status word and free
+//
+// Short sums over few tiles run on single CTAs (gemm_bf16_one_kernel below): a cluster's start costs 1 to 2 us more than a CTA's.
+// Every wait is bounded; when one runs out the CTA, or both, stop, let the copies and MMAs in flight end, raise the status word and free
 // their TMEM.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -131,7 +131,7 @@ constexpr int kTileLd = 40;   // elements from row to row where bf16 outputs tur
 
 // one warp: 32 features x rows [c_begin, c_end) of accumulators -> y
 template <int BN, bool GLU>
-__device__ __forceinline__ void store_tile(const GemmParams& p, uint32_t tmem, int f0, int t0, int quarter, int lane, __nv_bfloat16* tile, int c_begin, int c_end) {
+__device__ __forceinline__ void store_tile(const GemmParams p, uint32_t tmem, int f0, int t0, int quarter, int lane, __nv_bfloat16* tile, int c_begin, int c_end) {
   const int f = f0 + quarter * 32 + lane;
   const bool live = f < p.M;
   const float b0 = live && p.bias ? p.bias[f] : 0.0f, b1 = GLU && live && p.bias ? p.bias[p.M + f] : 0.0f;
@@ -179,7 +179,10 @@ __device__ __forceinline__ void store_tile(const GemmParams& p, uint32_t tmem, i
       if (n >= 8) {
         *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
       } else {
-        for (int e = 0; e < n; ++e) dst[e] = src[e];
+        // no loop: as one it cost every piece of a ragged tile (136 features, 64 rows: 5.7 us, so 4.6)
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (e < n) dst[e] = src[e];
       }
     }
   }
@@ -433,6 +436,179 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   }
 }
 
+// ---- one CTA a tile of 128 features, no cluster: for sums so short that the start is a large part of the time.
+// 6 warps: 0-3 read the accumulators back, 4 issues the copies, 5 the MMAs.  Two CTAs an SM (one computes while the other
+// stores), or, where the grid leaves an SM no second one, DEEP: all the stages that an SM holds
+__device__ __forceinline__ void tma_load_one(void* dst, const TmaMap* map, int x, int y, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
+               "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+               : "memory");
+}
+template <int BN>
+constexpr uint32_t kInstrDescOne = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+__device__ __forceinline__ void mma_bf16_one(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void mma_commit_one(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+constexpr int kOneThreads = 192, kOneTmaWarp = 4, kOneMmaWarp = 5;
+
+template <int BN, bool GLU, bool DEEP>
+struct OneTile {
+  static constexpr int kStageBytes = (GLU ? 2 : 1) * kWeightTile + BN * kBK * 2;
+  static constexpr int kStages = DEEP ? 200 * 1024 / kStageBytes : BN == 256 ? 2 : BN == 128 ? 3 : 4;
+  // of x, a copy.  64 rows as two of 32: copies that reach far past the last row are slow (24576 features, K = 2048, 17 rows: 24.8 us, so 19.7)
+  static constexpr int kBoxRows = BN == 64 ? 32 : BN < 128 ? BN : 128, kBox = BN == 16 ? 0 : BN == 64 ? 1 : 3;
+  static_assert(kGemmTokenBox << kBox == kBoxRows, "box");
+  static constexpr int kTmemCols = (GLU ? 2 : 1) * BN < 32 ? 32 : (GLU ? 2 : 1) * BN;
+  static constexpr int kSmem = kStages * kStageBytes + 1024 + 256;
+  static_assert(4 * 32 * kTileLd * 2 <= kStages * kStageBytes, "bf16 outputs turn in the stages");
+};
+
+template <int BN, bool GLU, bool DEEP>
+__global__ void __launch_bounds__(kOneThreads) gemm_bf16_one_kernel(const __grid_constant__ TmaMap wmap, const __grid_constant__ TmaMap xmap,
+                                                                    const GemmParams p) {
+  using T = OneTile<BN, GLU, DEEP>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + T::kStages * T::kStageBytes);
+  uint64_t* empty = full + T::kStages;
+  uint64_t* done = empty + T::kStages;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t0 = blockIdx.x * BN, f0 = blockIdx.y * kBM;
+  const int nk = (p.K + kBK - 1) / kBK;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < T::kStages; ++s) {
+      mbar_init(full + s, 1);
+      mbar_init(empty + s, 1);
+    }
+    mbar_init(done, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == kOneMmaWarp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(T::kTmemCols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  const auto wait = [&](uint64_t* bar, uint32_t parity, Role role, int use) {
+    if (!EMELB_GIVE_UP(0, role, use) && mbar_wait(bar, parity, abort_flag)) return true;
+    *abort_flag = 1;
+    return false;
+  };
+
+  int issued = 0;
+  if (warp == kOneTmaWarp && lane == 0) {
+    for (int i = 0; i < nk; ++i) {
+      const int s = i % T::kStages;
+      if ((i >= T::kStages || EMELB_GIVE_UP(0, kCopies, i)) && !wait(empty + s, ((i / T::kStages) - 1) & 1, kCopies, i)) break;
+      uint8_t* st = smem + s * T::kStageBytes;
+      mbar_arrive_expect_tx(full + s, T::kStageBytes);
+      tma_load_one(st, &wmap, i * kBK, f0, full + s);
+      if (GLU) tma_load_one(st + kWeightTile, &wmap, i * kBK, p.M + f0, full + s);
+#pragma unroll
+      for (int b = 0; b < BN / T::kBoxRows; ++b)
+        tma_load_one(st + (GLU ? 2 : 1) * kWeightTile + b * T::kBoxRows * kBK * 2, &xmap, i * kBK, t0 + b * T::kBoxRows, full + s);
+      issued = i + 1;
+    }
+  } else if (warp == kOneMmaWarp && elect_one()) {
+    for (int i = 0; i < nk; ++i) {
+      const int s = i % T::kStages;
+      if (!wait(full + s, (i / T::kStages) & 1, kMmas, i)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t st = smem_u32(smem + s * T::kStageBytes), xt = st + (GLU ? 2 : 1) * kWeightTile;
+#pragma unroll
+      for (int k = 0; k < kBK / 16; ++k) {
+        const uint64_t db = operand_desc(xt + 32 * k);
+        mma_bf16_one(tmem, operand_desc(st + 32 * k), db, kInstrDescOne<BN>, i > 0 || k > 0);
+        if (GLU) mma_bf16_one(tmem + BN, operand_desc(st + kWeightTile + 32 * k), db, kInstrDescOne<BN>, i > 0 || k > 0);
+      }
+      mma_commit_one(empty + s);
+    }
+    mma_commit_one(done);
+  }
+  __syncwarp();
+  if (warp < 4) {
+    // `done` also follows MMAs that gave up: the flag, raised before, tells
+    const bool ok = wait(done, 0, kStores, 0) && !*abort_flag;
+    if (__all_sync(0xffffffffu, ok)) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // bf16 outputs turn in the stages, which are free: every copy has landed and been used
+      store_tile<BN, GLU>(p, tmem, f0, t0, warp, lane, reinterpret_cast<__nv_bfloat16*>(smem) + warp * 32 * kTileLd, 0, BN);
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (*abort_flag) {
+    // A wait ran out, and no role issues any more: the copies and MMAs in flight end (bounded) before their memory goes
+    if (warp == kOneTmaWarp && lane == 0)
+      for (int i = max(0, issued - T::kStages); i < issued; ++i)
+        for (int spin = 0; spin < 1 << 16 && !mbar_try_wait(full + i % T::kStages, (i / T::kStages) & 1); ++spin) {}
+    if (warp == kOneMmaWarp && lane == 0)
+      for (int spin = 0; spin < 1 << 16 && !mbar_try_wait(done, 0); ++spin) {}
+    __syncwarp();
+  }
+  if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, 1);
+  if (warp == kOneMmaWarp) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(T::kTmemCols) : "memory");
+  }
+}
+
+template <int BN, bool GLU, bool DEEP>
+cudaError_t launch_one_stages(const TmaMap& wmap, const XMaps& x, const GemmParams& p, cudaStream_t st) {
+  using T = OneTile<BN, GLU, DEEP>;
+  const cudaError_t e = cudaFuncSetAttribute(gemm_bf16_one_kernel<BN, GLU, DEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kSmem);
+  if (e != cudaSuccess) return e;
+  gemm_bf16_one_kernel<BN, GLU, DEEP><<<dim3((p.rows + BN - 1) / BN, (p.M + kBM - 1) / kBM), kOneThreads, T::kSmem, st>>>(wmap, x.box[T::kBox], p);
+  return cudaGetLastError();
+}
+
+int64_t one_tiles(const GemmParams& p, int bn) { return (int64_t)((p.M + kBM - 1) / kBM) * ((p.rows + bn - 1) / bn); }
+
+template <int BN, bool GLU>
+cudaError_t launch_one(const TmaMap& wmap, const XMaps& x, const GemmParams& p, int sm_count, cudaStream_t st) {
+  return one_tiles(p, BN) <= sm_count ? launch_one_stages<BN, GLU, true>(wmap, x, p, st) : launch_one_stages<BN, GLU, false>(wmap, x, p, st);
+}
+
+// rows of x a single CTA's tile: narrower ones while every one has an SM, the widest once there are more of them than SMs
+int one_rows(const GemmParams& p, int sm_count) {
+  if (p.rows <= 16) return 16;
+  if (p.rows <= 64 || one_tiles(p, 64) <= sm_count) return 64;
+  return 5 * one_tiles(p, 256) >= 6 * sm_count ? 256 : 128;
+}
+
+// Single CTAs or pairs, us there and here, one launch behind the other in a graph.
+// K to 256, to four tiles an SM: 4096 x 256 by 8 rows 3.5 / 4.5, by 200 4.5 / 6.4, by 2048 9.8 / 12.3, 136 x 136 by 100 4.5 / 5.2; beyond it the pairs' rate
+// wins (8192 x 256 by 1500 18.3 / 17.1).  K to 512 likewise (8192 x 512 by 8 5.3 / 5.8, by 128 6.2 / 7.6, by 333 8.8 / 10.0, by 1000 13.2 / 13.9, by 1500 23.2 /
+// 18.5), but with more than 32 rows in tiles for less than half of the SMs pairs are as fast or faster: 2048 x 512 by 100 5.3 / 5.0, by 333 5.4 / 6.7.
+// K to 1024, tiles for two thirds of the SMs to two an SM: 8192 x 1024 by 100 9.0 / 9.5, by 300 12.2 / 12.4, 2048 x 1024 by 1500 11.2 / 11.9; else 2048 x 1024 by 100
+// 8.3 / 6.7, 8192 x 1024 by 700 18.9 / 16.2.
+// Up to 64 rows of a matrix with one to two tiles an SM, which leaves most pairs idle in a last turn: 20480 x 2048 by 8 17.5 / 19.9, 32000 x 2048 by 64
+// 24.1 / 25.4, 24576 x 4096 by 64 39.4 / 42.2; 32000 x 4096 by 8 45.5 / 44.4, 14336 x 2048 by 32 13.8 / 13.2.
+// Two matrices and up to 16 rows: 512 x 2 x 256 by 16 5.1 / 5.7, 8192 x 2 x 2048 by 8 17.0 / 17.4; 14336 x 2 x 4096 by 8 41.7 / 41.9
+bool one_cta(const GemmParams& p, bool glu, int sm_count) {
+  if (glu) return p.rows <= 16 && p.K <= 2048;
+  const int64_t tiles = one_tiles(p, std::min(one_rows(p, sm_count), 128));
+  if (p.K <= 512) return tiles <= 4 * sm_count && (p.K <= 256 || p.rows <= 32 || 2 * tiles > sm_count);
+  if (p.K <= 1024) return 3 * tiles > 2 * sm_count && tiles <= 2 * sm_count;
+  return p.rows <= 64 && tiles > sm_count && (p.K <= 2048 ? tiles <= 2 * sm_count : p.K <= 4096 && 2 * tiles <= 3 * sm_count);
+}
+
 int64_t tiles_of(const GemmParams& p, int bn) { return (int64_t)((p.M + 2 * kBM - 1) / (2 * kBM)) * ((p.rows + bn - 1) / bn); }
 
 template <int BN, bool GLU, int SL>
@@ -480,6 +656,13 @@ cudaError_t launch_gemm_bf16(const LinearArgs& a, const TmaMap& wmap, const XMap
   const bool glu = is_glu(a.act);
   GemmParams p{glu ? a.w.M / 2 : a.w.M, a.w.K, a.rows, a.bias, a.act, a.act_split, y, yb, ldy, status,
                a.out_scale, a.softcap, a.tail, a.tail_y, a.tail_ld};
+  if (one_cta(p, glu, sm_count)) {
+    if (glu) return launch_one<16, true>(wmap, x, p, sm_count, st);
+    const int bn = one_rows(p, sm_count);
+    if (bn == 16) return launch_one<16, false>(wmap, x, p, sm_count, st);
+    if (bn == 64) return launch_one<64, false>(wmap, x, p, sm_count, st);
+    return bn == 128 ? launch_one<128, false>(wmap, x, p, sm_count, st) : launch_one_stages<256, false, false>(wmap, x, p, st);
+  }
   // The width with the least turns x time a turn.  Weights: us a turn of an SM pair at K = 2048 / 4096 / 8192 / 14336:
   // 32 rows 10.6 / 16.6 / 26.8 / 42, 128 rows 12.6 / 18.6 / 29 / 48, 256 rows 18.7 / 27 / 45 / 72; two matrices at K = 2048: 32 rows 14.6, 64
   // rows 18.7, 128 rows 22.  (64 rows of one matrix cost within 3 % of 128.)

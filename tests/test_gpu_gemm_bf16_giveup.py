@@ -1,4 +1,4 @@
-"""What the bf16 tile kernel does when a wait runs out: both CTAs of a pair stop, the copies and MMAs in flight end before the
+"""What the bf16 tile kernels do when a wait runs out: the CTA, or both of a pair, stop, the copies and MMAs in flight end before the
 memory goes to the next launch, and the status word says so.  The waits run out by a host program's choice (the kernel's source,
 compiled with a condition in front of them); nothing faults or hangs."""
 import os
