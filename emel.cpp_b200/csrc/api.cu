@@ -351,9 +351,9 @@ uint32_t emelb_create(int device, emelb_ctx** out) {
   ok = ok && cudaMalloc(&c->act_qs, c->act_capacity) == cudaSuccess;
   ok = ok && cudaMalloc(&c->act_d, c->act_capacity / 32 * sizeof(float)) == cudaSuccess;
   ok = ok && cudaMalloc(&c->act_bsums, c->act_capacity / 16 * sizeof(int16_t)) == cudaSuccess;
-  // operands of the tcgen05 kernels: 512 bytes of f16 for 256 K of a column, with Q4_K 40 of block sums, scale and mean and the
-  // weights' table beside them (56 a row for 256 K).  Columns that it does not hold are taken in turns: at the default size 2048
-  // columns of 14336 x 4096, 4096 x 14336 or 16384 x 16384 (rows x K) are one turn, of 18432 x 18432 or 8192 x 28672 two
+  // operands of the tcgen05 kernels: 512 bytes of f16 for 256 K of a column, with Q4_K 40 of block sums, scale and mean, and what is
+  // made of the weights once where it fits beside them.  Columns that it does not hold are taken in turns: at the default size
+  // 2048 columns are one turn up to K of 31,000
   c->tc_ws_bytes = c->act_capacity / 32768 * 35328 + (64u << 20);
   ok = ok && cudaMalloc(&c->tc_ws, c->tc_ws_bytes) == cudaSuccess;
   ok = ok && cudaMalloc(&c->gemv_sched, (2 * kSchedSlots + 2) * sizeof(int)) == cudaSuccess;

@@ -30,14 +30,14 @@
 // TMEM at TN = 128: two turns' accumulators (256 columns), msum of one turn (128, made and read in two parts, so that
 // the next turn's first part is made while the epilogue works on the second), the operand of one super-block (128, handed
 // over in quarters).  Narrower tiles keep two super-blocks of operand.
-// With several column tiles the mins' operand and {d, -dmin, T} of every row and super-block come from a table that a
-// pre-pass over the weights makes once (TN = 128); narrower tiles work them out while they expand.
+// Where it pays (TN = 128, many waves: plan_tiles) the mins' operand and {d, -dmin, T} of every row and super-block come from a
+// table that a pre-pass over the weights makes once; else the producers work them out while they expand.
 // Registers are split by setmaxnreg: 640 threads x 96 at launch = 256 x 80 + 256 x 136 + 128 x 48.
 // Every mbarrier wait is bounded; on a timeout the CTA raises the status word, lets its copies land and frees its TMEM.
 //
 // What bounds it: instruction issue, 60 % of the slots with some eight cycles between two instructions of a warp.  Per
 // 128 x 128 x 256: 6,600 warp instructions (1,536 packed float ones, 1,150 for the expansion), of 2,600 cycles the MMAs take
-// 1,090.  Measured, B200, 14336 x 4096 by 2048 columns: pre-passes and product 352 us, product alone 333 (340 and 722
+// 1,090.  Measured, B200, 14336 x 4096 by 2048 columns: pre-passes and product 352 us, product alone 333 (683 and 722
 // TFLOP/s); the int8 kernel before it (two operands of scale pieces, sums of mins on mma.sync) 439.  Whole calls on planes,
 // before and now: 14336 x 4096 by 32 columns 47.7 -> 30.5, by 128 48.4 -> 44.6, by 512 159 -> 118; 4096 x 14336 by 32 134 -> 78,
 // by 333 136 -> 104, by 1900 517 -> 354; 1024 x 4096 by 333 47.6 -> 31.4.  What gave it: TMEM loads of whole lanes (32x32b, half
@@ -106,8 +106,6 @@ __device__ __forceinline__ uint64_t plain_desc(uint32_t saddr, uint32_t chunk_st
 }
 
 struct GemmArgs {
-  const uint8_t* W;
-  int64_t row_bytes;
   int M, K, N;
   const uint8_t* x;       // [K/64][npad/8] swizzle atoms of 8 columns
   const uint8_t* sums;    // [K/256][2 chunks][npad][16 bytes]
@@ -118,6 +116,11 @@ struct GemmArgs {
   int64_t ldy;
   int* status;
 };
+
+// 16-byte pieces of the result's rows
+__host__ __device__ __forceinline__ bool rows_aligned(const GemmArgs& p) {
+  return ((p.ldy | (int64_t)(reinterpret_cast<uintptr_t>(p.y) >> 2)) & 3) == 0;
+}
 
 // pre-pass: the quantized activation planes of columns col0.. -> operand order.  K position 128 n + 16 w + 8 c + j of
 // a super-block holds element 128 n + 64 c + 32 (j / 4) + 4 w + {0, 2, 1, 3}[j % 4], which is what the producers'
@@ -534,6 +537,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q4k_tc_kernel(const GemmArgs
     // broadcasts.  (TMEM loads of whole lanes take half a cycle a register, those in the m16n8 fragment layout two.)
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kEpilogueRegs));
     constexpr int kMine = C::kPart / 2, kLoads = kMine / 8;        // columns of a part; loads of eight
+    static_assert(kLoads % 2 == 0, "rows leave 16 columns at a time");
     const int quarter = warp & 3, side = (warp - kEpilogueWarp0) >> 2;
     const uint32_t tb = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(kMine * side), lead = lane == 0;
     int ms = 0, rslot = 0, it = 0;
@@ -603,23 +607,31 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q4k_tc_kernel(const GemmArgs
       // of 32 rows an instruction took twice as long, and longer than the pairs of the fragment layout)
       const int tm = tile / nt, r0 = tm * BM + 32 * quarter, j = lane & 3;
       uint8_t* stage = smem + C::kOffStage + (warp - kEpilogueWarp0) * 32 * kStageRow;
-      const bool aligned = ((p.ldy | (int64_t)(reinterpret_cast<uintptr_t>(p.y) >> 2)) & 3) == 0;
+      const bool aligned = rows_aligned(p);
 #pragma unroll
       for (int s = 0; s < C::kParts; ++s)
 #pragma unroll
         for (int i = 0; i < kLoads; i += 2) {
-          const int n = kLoads > 1 ? 2 : 1;     // loads of this round
           __syncwarp();
 #pragma unroll
-          for (int e = 0; e < 2 * n; ++e)
+          for (int e = 0; e < 4; ++e)
             *reinterpret_cast<ulonglong2*>(stage + lane * kStageRow + 16 * e) = make_ulonglong2(acc[s][i + (e >> 1)][2 * (e & 1)], acc[s][i + (e >> 1)][2 * (e & 1) + 1]);
           __syncwarp();
           const int c = (tile - tm * nt) * TN + C::kPart * s + kMine * side + 8 * i + 4 * j;
+          // Other strides: single floats, 16 of a row side by side (four floats a lane: 14336 x 1024 by 333 52, so 48 us).  Not with
+          // the table, whose products are long: there the code in its way takes 0.6 % of 14336 x 4096 by 2048
+          if (!kTable && !aligned) {
+            const int cc = c - 4 * j + (lane & 15);
+            if (cc < p.N)
+#pragma unroll 1
+              for (int row = lane >> 4; row < 32 && r0 + row < p.M; row += 2) p.y[(size_t)(r0 + row) * p.ldy + cc] = *reinterpret_cast<const float*>(stage + row * kStageRow + 4 * (lane & 15));
+            continue;
+          }
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             const int row = r0 + 8 * k + (lane >> 2);
             const float4 v = *reinterpret_cast<const float4*>(stage + (8 * k + (lane >> 2)) * kStageRow + 16 * j);
-            if (row >= p.M || j >= 2 * n) continue;
+            if (row >= p.M) continue;
             float* yr = p.y + (size_t)row * p.ldy + c;
             if (aligned && c + 3 < p.N) {
               *reinterpret_cast<float4*>(yr) = v;
@@ -713,22 +725,33 @@ cudaError_t launch_tiles(const GemmArgs& g, const CUtensorMap& wmap, int sm_coun
   return cudaGetLastError();
 }
 
-// Columns per tile: the fewest waves of CTAs, weighted with what a wave takes (4096 x 14336, one wave: 78, 88 and 97 us with
-// tiles of 32, 64 and 128 columns; 1024 x 4096: 31, 34.5 and 40).  Each is up to 1.4 times as fast as the others somewhere
-int tile_columns(int M, int ncols, int sm_count, bool wide) {
-  const int mt = (M + BM - 1) / BM;
+// Columns per tile, and whether a table of the rows is made first: what takes the least time by a model of hundredths of a us.  A
+// wave of CTAs takes a start and a time per super-block; the table is a launch and a pass over the weights, and saves a part
+// of every wave and super-block.  Fitted to 190 calls of 3000 to 32000 rows, K of 256 to 4096 and 32 to 1900 columns, of which it takes
+// six 3 to 8 % longer than the best does.  us, tiles of 32, 64, 128 without and 128 with table: 14336 x 256 by 160 columns 24.3, 24.5, 26.5,
+// 29.4; 6500 x 768 by 256 30.7, 27.9, 25.6, 29.7; 4096 x 1024 by 512 39.9, 31.7, 27.6, 31.8; 14336 x 2048 by 333 109, 78.9, 68.7, 70.7, by 1900 472, 280,
+// 199, 191; 4096 x 14336, one wave, 78, 88 and (table) 97
+struct Plan {
+  int columns;
+  bool table;
+};
+Plan plan_tiles(int M, int K, int ncols, int call_columns, int sm_count, bool table_fits, bool aligned) {
+  const int64_t mt = (M + BM - 1) / BM, nkb = K / QK_K;
   auto waves = [&](int tn) { return (mt * ((ncols + tn - 1) / tn) + sm_count - 1) / sm_count; };
-  const int c128 = 100 * waves(128), c64 = 90 * waves(64), c32 = 81 * waves(32);
-  if (wide && ncols > 64 && c128 <= c64 && c128 <= c32) return 128;
-  return c64 <= c32 ? 64 : 32;
+  const int64_t c32 = waves(32) * (45 + 119 * nkb), c64 = waves(64) * (90 + 132 * nkb);
+  const int64_t saved = waves(128) * (18 + 12 * nkb) - 320 - mt * nkb * 26 / 100;
+  // calls of 1024 column tiles and more make the table either way, in each of their turns: its launches are 2 % of them at most
+  if (table_fits && call_columns > 1023 * 128 && ncols > 64) return Plan{128, true};
+  // strides of no 16 bytes: the kernels without table store them better (14336 x 256 by 1901 83, with table 96)
+  const bool table = table_fits && saved > 0 && (aligned || nkb > 4);
+  const int64_t c128 = waves(128) * (190 + 162 * nkb) - (table ? saved : 0);
+  if (ncols > 64 && c128 <= c64 && c128 <= c32) return Plan{128, table};
+  return Plan{c64 <= c32 ? 64 : 32, false};
 }
 
-size_t table_bytes(const GemvArgs& a) { return (size_t)((a.M + BM - 1) / BM) * (a.K / QK_K) * kTableBytes; }
-bool table_fits(const GemvArgs& a) { return table_bytes(a) + gemm_tc_workspace_bytes(a.K, 128) <= a.tc_ws_bytes; }
-
-// columns of a turn: what the workspace holds beside the rows' table, and a grid's y extent; ncols where one turn takes all
+// columns of a turn: what the workspace holds, and a grid's y extent; ncols where one turn takes all
 int turn_columns(const GemvArgs& a, int ncols) {
-  const size_t group = gemm_tc_workspace_bytes(a.K, 128), groups = (table_fits(a) ? a.tc_ws_bytes - table_bytes(a) : a.tc_ws_bytes) / group;
+  const size_t groups = a.tc_ws_bytes / gemm_tc_workspace_bytes(a.K, 128);
   const int fit = (int)(groups < 32767 ? groups : 32767) * 128;
   return fit >= ncols || (ncols <= 64 && fit == 0) ? ncols : fit;   // a single group of 64 columns may fit where 128 do not
 }
@@ -737,12 +760,12 @@ int turn_columns(const GemvArgs& a, int ncols) {
 
 bool gemm_q4k_tc_one_turn(const GemvArgs& a, int ncols) { return turn_columns(a, ncols) == ncols; }
 
-// launches: the activation pre-pass (into the workspace), the pre-pass over the weights where several column tiles share
-// its results, and the product; the three again for columns whose operand the workspace does not hold beside the others'
+// launches: the activation pre-pass (into the workspace), the pre-pass over the weights where it pays and its results fit beside
+// the columns, and the product; the three again for columns whose operand the workspace does not hold beside the others'.  (A
+// table never sends columns to another turn: what a turn holds follows from K and the columns alone, for every matrix of an
+// input.)
 cudaError_t launch_gemm_q4k_tc(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st, int* launches) {
   GemmArgs g{};
-  g.W = a.W;
-  g.row_bytes = a.row_bytes;
   g.M = a.M;
   g.K = a.K;
   g.ldy = a.ldy;
@@ -755,7 +778,8 @@ cudaError_t launch_gemm_q4k_tc(const GemvArgs& a, int ncols, int sm_count, cudaS
     g.npad = padded_columns(g.N);
     g.y = a.y + a.col0 + c;
     const OperandLayout x = operand_layout(a.tc_ws, a.K, g.npad);
-    uint8_t* table = a.tc_ws + operand_layout_bytes(a.K, g.npad);
+    const size_t used = operand_layout_bytes(a.K, g.npad);
+    uint8_t* table = a.tc_ws + used;
     g.x = x.x;
     g.sums = x.sums;
     g.pairs = x.pairs;
@@ -766,15 +790,16 @@ cudaError_t launch_gemm_q4k_tc(const GemvArgs& a, int ncols, int sm_count, cudaS
       ++*launches;
       if (e != cudaSuccess) return e;
     }
-    const int tn = tile_columns(a.M, g.N, sm_count, table_fits(a) && mt <= 65535);
-    if (tn == 128) {
+    const Plan plan = plan_tiles(a.M, a.K, g.N, ncols, sm_count, used + (size_t)mt * nkb * kTableBytes <= a.tc_ws_bytes && mt <= 65535, rows_aligned(g));
+    if (plan.table) {
       q4k_table_kernel<<<dim3(nkb, mt), BM, 0, st>>>(a.W, a.row_bytes, a.M, table);
       ++*launches;
       e = cudaGetLastError();
       if (e != cudaSuccess) return e;
       e = launch_tiles<128, true>(g, wmap, sm_count, st);
     } else {
-      e = tn == 64 ? launch_tiles<64, false>(g, wmap, sm_count, st) : launch_tiles<32, false>(g, wmap, sm_count, st);
+      e = plan.columns == 128 ? launch_tiles<128, false>(g, wmap, sm_count, st)
+          : plan.columns == 64 ? launch_tiles<64, false>(g, wmap, sm_count, st) : launch_tiles<32, false>(g, wmap, sm_count, st);
     }
     ++*launches;
     if (e != cudaSuccess) return e;

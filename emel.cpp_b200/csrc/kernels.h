@@ -267,8 +267,7 @@ bool gemm_tc_supported(int type, int K, int ncols, const void* W, int64_t row_by
 // true when launch_gemv would run the kernel that honours GemvArgs::pro_x for this matrix
 bool gemv_prologue_supported(int type, const void* w, int64_t row_bytes, int K);
 size_t gemm_tc_workspace_bytes(int K, int ncols);
-// false: the columns go in turns, and only the last turn's operand stays in the workspace.  How many a turn takes depends on the
-// rows too, whose table shares the workspace
+// false: the columns go in turns, and only the last turn's operand stays in the workspace
 bool gemm_q4k_tc_one_turn(const GemvArgs& a, int ncols);
 cudaError_t launch_gemm_q4k_tc(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st, int* launches);
 

@@ -283,10 +283,10 @@ def test_batched_prompt_fills_the_context_to_the_last_row(be, port):
         sess.close()
 
 
-def test_batched_prompt_whose_query_product_takes_turns(port, monkeypatch):
-    """Width 16384 with a small workspace: 512 tokens of the query projection go in two turns (its table of 16384 rows leaves
-    room for 384 columns), those of the key and value projections in one.  Of the first turn nothing may be taken for theirs.
-    One layer, so bit-identical to batches of 128 tokens, which every product takes in one turn.  Weights of N(0, 0.005): scores of
+def test_batched_prompt_whose_query_table_is_larger_than_the_workspace(port, monkeypatch):
+    """Width 16384 with a small workspace, which does not hold 512 columns beside a table of the query projection's 16384 rows,
+    but beside one of the key and value projections': whatever that product does (it once took turns), what it leaves may be
+    taken for theirs only if it is all of the columns.  One layer, so bit-identical to batches of 128 tokens.  Weights of N(0, 0.005): scores of
     a few tenths, so that every position counts."""
     torch = pytest.importorskip("torch")
     monkeypatch.setenv("EMELB_ACT_MELEMS", "8")

@@ -275,3 +275,40 @@ def test_q8_0_and_q4_0_prompts_largest_sums(be, port, t):
     b[:, :2] = d.view(np.uint8).reshape(-1, 2)
     b[:, 2:] = np.array([0x80, 0x7f, 0xff, 0x00, 0x88], np.uint8)[i // 5 % 5][:, None]
     check(be, port, t, b.reshape(-1), k, m, one_sided(k, n), n)
+
+
+@pytest.mark.parametrize("k,m,n", [(256, 3100, 513), (512, 4100, 515), (768, 6500, 162), (1024, 4096, 333), (1024, 14300, 97), (2048, 5700, 130)])
+@pytest.mark.parametrize("extreme", [False, True])
+def test_q4_k_short_sums(be, port, k, m, n, extreme):
+    """Tiles of 64 (K = 256) and 128 columns without a table of the rows: two launches behind the quantizer.  Odd and even strides."""
+    w = extreme_blocks(eb.Q4_K, m, k) if extreme else synth.random_blocks(eb.Q4_K, m + n, m, k)
+    x = one_sided(k, n) if extreme else synth.activations_f32(m * n, k, n).reshape(k, n)
+    assert launches_of(be, lambda: check(be, port, eb.Q4_K, w, k, m, x, n)) == 3
+
+
+def tiled_rows(torch, t, seed, m, k):
+    """Rows 7 i % 997 of 997 random ones, on the device."""
+    few = torch.from_numpy(synth.random_blocks(t, seed, 997, k).reshape(997, -1)).cuda()
+    return few, few[torch.arange(m, device="cuda") * 7 % 997].contiguous()
+
+
+def test_q4_k_table_larger_than_the_workspace(monkeypatch):
+    """Rows whose table does not fit beside the activations: all columns in one turn, without it."""
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("EMELB_ACT_MELEMS", "8")
+    b = eb.Backend(0)
+    try:
+        k, m, n = 4096, 83001, 2047
+        few, w = tiled_rows(torch, eb.Q4_K, 9, m, k)
+        x = torch.from_numpy(synth.activations_f32(10, k, n).reshape(k, n)).cuda()
+        y, want = torch.zeros((m, n), device="cuda"), torch.zeros((997, n), device="cuda")
+        torch.cuda.synchronize()
+
+        def call():
+            assert b.mul_mat(eb.mul_mat_op(w, eb.Q4_K, k, m, x, n, y)), b.last_error
+        assert launches_of(b, call) == 3      # quantizer, operand layout, product
+        assert b.mul_mat(eb.mul_mat_op(few, eb.Q4_K, k, 997, x, n, want)), b.last_error
+        assert b.sync()
+        assert torch.equal(y.view(torch.int32), want[torch.arange(m, device="cuda") * 7 % 997].view(torch.int32))
+    finally:
+        b.close()
