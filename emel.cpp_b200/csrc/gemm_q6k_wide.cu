@@ -132,6 +132,8 @@ __global__ void __launch_bounds__(256) q6k_slab_kernel(const uint8_t* W, int64_t
   }
 }
 
+// kAligned: rows of results go in 16-byte pieces.  A kernel of its own, because the other form in its way costs it 2 %
+template <bool kAligned>
 __global__ void __launch_bounds__(kThreads, 1) gemm_q6k_wide_kernel(const GemmArgs p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -408,7 +410,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q6k_wide_kernel(const GemmAr
       // rows leave through shared memory, 8 columns at a time, two lanes a row: 32 bytes of a row side by side
       const int tm = tile / nt, r0 = tm * BM + 32 * quarter, j = lane & 1;
       uint8_t* stage = smem + kOffStage + (warp - kEpilogueWarp0) * 32 * kStageRow;
-      const bool aligned = ((p.ldy | (int64_t)(reinterpret_cast<uintptr_t>(p.y) >> 2)) & 3) == 0;
 #pragma unroll
       for (int s = 0; s < 2; ++s)
 #pragma unroll
@@ -418,19 +419,26 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q6k_wide_kernel(const GemmAr
           for (int e = 0; e < 2; ++e) *reinterpret_cast<ulonglong2*>(stage + lane * kStageRow + 16 * e) = make_ulonglong2(acc[s][i][2 * e], acc[s][i][2 * e + 1]);
           __syncwarp();
           const int c = (tile - tm * nt) * TN + kPart * s + kMine * side + 8 * i + 4 * j;
+          if constexpr (!kAligned) {
+            // other strides: single floats, 8 of a row side by side (four floats a lane: 4096 x 4096 by 1901 188, so 171 us)
+            const int cc = c - 4 * j + (lane & 7);
+            if (cc < p.N)
+#pragma unroll 1
+              for (int row = lane >> 3; row < 32 && r0 + row < p.M; row += 4) p.y[(size_t)(r0 + row) * p.ldy + cc] = *reinterpret_cast<const float*>(stage + row * kStageRow + 4 * (lane & 7));
+          } else {
 #pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const int row = r0 + 16 * k + (lane >> 1);
-            const float4 v = *reinterpret_cast<const float4*>(stage + (16 * k + (lane >> 1)) * kStageRow + 16 * j);
-            if (row >= p.M) continue;
-            float* yr = p.y + (size_t)row * p.ldy + c;
-            if (aligned && c + 3 < p.N) {
-              *reinterpret_cast<float4*>(yr) = v;
-            } else {
-              if (c < p.N) yr[0] = v.x;
-              if (c + 1 < p.N) yr[1] = v.y;
-              if (c + 2 < p.N) yr[2] = v.z;
-              if (c + 3 < p.N) yr[3] = v.w;
+            for (int k = 0; k < 2; ++k) {
+              const int row = r0 + 16 * k + (lane >> 1);
+              const float4 v = *reinterpret_cast<const float4*>(stage + (16 * k + (lane >> 1)) * kStageRow + 16 * j);
+              if (row >= p.M) continue;
+              float* yr = p.y + (size_t)row * p.ldy + c;
+              if (c + 3 < p.N) {
+                *reinterpret_cast<float4*>(yr) = v;
+              } else {
+                if (c < p.N) yr[0] = v.x;
+                if (c + 1 < p.N) yr[1] = v.y;
+                if (c + 2 < p.N) yr[2] = v.z;
+              }
             }
           }
         }
@@ -448,36 +456,55 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_q6k_wide_kernel(const GemmAr
 
 }  // namespace
 
-// Against the kernels for fewer columns, us a call there and here; this one needs about 2 us a super-block and its passes.
-// gemm_q6k_mma.cu (K % 2048 == 0, aligned rows; CTAs of 64 x 64): from one CTA an SM on, or long rows.  4096 x 4096 by 128 columns
-// 40 / 50, by 200 69 / 50, 14336 x 4096 by 100 109 / 65, by 1900 977 / 377, 1024 x 4096 by 512 41 / 46, by 1024 55 / 48, 1024 x 14336
-// by 100 128 / 115, 4096 x 14336 by 128 128 / 128, by 1900 972 / 430.  gemm_q6k_tc.cu (other rows; 128 x 64) needs no pass over
-// the weights: 192 columns too.  4096 x 2816 by 200 39 / 40, by 333 66 / 45, 4096 x 11008 by 200 114 / 105, by 1900 728 / 337,
-// 14336 x 11008 by 128 215 / 219, by 512 709 / 369
+// Against the kernels for fewer columns.  From one of their tiles an SM on, or for long rows, the cheaper one by a model in us: of
+// this kernel a start, the pass over the weights and a time per wave and super-block; of gemm_q6k_mma.cu (K % 2048 == 0, aligned
+// rows) its first wave of 64 x 64 tiles and what each further tile an SM adds, more where the last column tile is partial;
+// of gemm_q6k_tc.cu (other rows) its waves of 128 x 64.  Fitted to 250 calls; us there and here: 2048 x 2048 by 512 columns 35.9 / 39.9,
+// by 640 47.2 / 41.9, 5632 x 2048 by 192 36.3 / 43.0, by 256 46.1 / 43.0, 4096 x 4096 by 192 60.5 / 56.4, by 512 110 / 60, 14336 x 4096 by 1900 977 / 377,
+// 4096 x 14336 by 128 136 / 140, by 1900 972 / 430; 6500 x 768 by 320 33.4 / 40.0, by 1024 58.5 / 48.1, 4096 x 2816 by 320 64.6 / 47.2, by 576 67.8 / 69.7,
+// 4096 x 11008 by 200 109.5 / 116.7, by 320 202 / 121.
+// Rows of a single super-block stay here from the first line on, though the other kernel is 2 to 8 us faster at that (6500 x 256 by
+// 201 23.7 / 28.7, 14336 x 256 by 1024 50.2 / 50.2): tests hold sizes of theirs to this kernel
 bool gemm_q6k_wide_supported(int type, const GemvArgs& a, int ncols, int sm_count) {
   if (type != T_Q6_K || a.M < BM || a.K % QK_K != 0 || !a.tc_ws) return false;
   const bool streamed = gemv_fast_path_ok(type, a.W, a.row_bytes, a.K);
-  const int tile_rows = streamed ? 64 : BM;
   if (ncols < (streamed ? 96 : 192)) return false;
-  if (a.K < 40 * QK_K && (int64_t)((a.M + tile_rows - 1) / tile_rows) * ((ncols + 63) / 64) <= sm_count) return false;
+  const int64_t nkb = a.K / QK_K, column_tiles = (ncols + 63) / 64, tile_rows = streamed ? 64 : BM;
+  const int64_t tiles = (a.M + tile_rows - 1) / tile_rows * column_tiles;
+  if (nkb < 40 && tiles <= sm_count) return false;
+  const auto waves = [&](int64_t n) { return (double)((n + sm_count - 1) / sm_count); };
+  const double here = 22.5 + 3.6e-7 * a.M * a.K + waves((int64_t)((a.M + BM - 1) / BM) * ((ncols + TN - 1) / TN)) * (2.5 + 1.75 * nkb);
+  double there;
+  if (streamed) {
+    const double w = waves(tiles);
+    there = 11.5 + nkb * (2.2 + (w > 1 ? 1.3 * (w - 1) - 0.4 : 0.0) + (ncols % 64 ? 4.5 / column_tiles : 0.0));
+  } else {
+    there = 17.5 + waves(tiles) * (0.5 + 2.1 * nkb);
+  }
+  if (nkb > 1 && there <= here) return false;
   if (a.residual || a.W2 || a.W3 || a.pro_x || a.rope_cos || a.join_in || a.join_out) return false;
-  const int nkb = a.K / QK_K;
   return reinterpret_cast<uintptr_t>(a.W) % 2 == 0 && a.row_bytes % 2 == 0 && planes_aligned(a.act) &&
          operand_layout_bytes(a.K, TN) + (size_t)nkb * kSlab <= a.tc_ws_bytes;
 }
 
-// launches: the activation pre-pass, then for as many rows as the workspace holds the pre-pass over the weights and the
-// product; all again for columns whose operand it does not hold beside them
-cudaError_t launch_gemm_q6k_wide(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st, int* launches) {
+template <bool kAligned>
+static cudaError_t launch_product(const GemmArgs& g, int grid, cudaStream_t st) {
   // per host thread (one context, one lane per thread): no shared mutable state between lanes
   static thread_local unsigned configured = 0;  // one bit per device
   int dev = 0;
   cudaGetDevice(&dev);
   if (!(configured & (1u << (dev & 31)))) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_q6k_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_q6k_wide_kernel<kAligned>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (e != cudaSuccess) return e;
     configured |= 1u << (dev & 31);
   }
+  gemm_q6k_wide_kernel<kAligned><<<grid, kThreads, kSmemBytes, st>>>(g);
+  return cudaGetLastError();
+}
+
+// launches: the activation pre-pass, then for as many rows as the workspace holds the pre-pass over the weights and the
+// product; all again for columns whose operand it does not hold beside them
+cudaError_t launch_gemm_q6k_wide(const GemvArgs& a, int ncols, int sm_count, cudaStream_t st, int* launches) {
   const int nkb = a.K / QK_K, mt = (a.M + BM - 1) / BM;
   const size_t group = operand_layout_bytes(a.K, TN), tile_row = (size_t)nkb * kSlab;
   // columns first: a slab is worth its making for many of them.  At least one tile row stays
@@ -509,9 +536,10 @@ cudaError_t launch_gemm_q6k_wide(const GemvArgs& a, int ncols, int sm_count, cud
       e = cudaGetLastError();
       if (e != cudaSuccess) return e;
       const int tiles = tiles_m * ((n + TN - 1) / TN);
-      gemm_q6k_wide_kernel<<<tiles < sm_count ? tiles : sm_count, kThreads, kSmemBytes, st>>>(g);
+      const int grid = tiles < sm_count ? tiles : sm_count;
+      const bool aligned = ((g.ldy | (int64_t)(reinterpret_cast<uintptr_t>(g.y) >> 2)) & 3) == 0;
+      e = aligned ? launch_product<true>(g, grid, st) : launch_product<false>(g, grid, st);
       *launches += 2;
-      e = cudaGetLastError();
       if (e != cudaSuccess) return e;
     }
   }

@@ -312,3 +312,34 @@ def test_q4_k_table_larger_than_the_workspace(monkeypatch):
         assert torch.equal(y.view(torch.int32), want[torch.arange(m, device="cuda") * 7 % 997].view(torch.int32))
     finally:
         b.close()
+
+
+@pytest.mark.parametrize("k,m,n,launches", [
+    (2048, 1030, 768, 2), (2048, 2048, 512, 2), (2048, 2048, 645, 4), (2048, 2600, 250, 4),    # aligned rows: mma.sync, or the prompt kernel
+    (768, 6500, 320, 3), (768, 6500, 777, 4), (1280, 2500, 700, 4), (512, 14300, 200, 3),      # others: 128 x 64 tiles, or the prompt kernel
+])
+def test_q6_k_line_to_the_prompt_kernel(be, port, k, m, n, launches):
+    w = synth.random_blocks(eb.Q6_K, m + n, m, k)
+    x = synth.activations_f32(m * n, k, n).reshape(k, n)
+    assert launches_of(be, lambda: check(be, port, eb.Q6_K, w, k, m, x, n)) == launches
+
+
+@pytest.mark.parametrize("offset", [2, 8, 14])
+def test_q6_k_prompt_kernel_at_even_addresses(be, port, offset):
+    torch = pytest.importorskip("torch")
+    k, m, n = 1280, 2500, 702
+    w = synth.random_blocks(eb.Q6_K, 5, m, k)
+    x = synth.activations_f32(6, k, n).reshape(k, n)
+    want = np.zeros((m, n), np.float32)
+    assert port.mul_mat(ob.mul_mat_op(w, eb.Q6_K, k, m, x, n, want), route="blocks")
+    room = torch.zeros(w.size + 64, dtype=torch.uint8, device="cuda")
+    dev_w = room[offset:offset + w.size]
+    dev_w.copy_(torch.from_numpy(w.reshape(-1)))
+    dev_x, dev_y = torch.from_numpy(x).cuda(), torch.zeros((m, n), device="cuda")
+    torch.cuda.synchronize()
+
+    def call():
+        assert be.mul_mat(eb.mul_mat_op(dev_w, eb.Q6_K, k, m, dev_x, n, dev_y)), be.last_error
+    assert launches_of(be, call) == 4
+    assert be.sync()
+    assert np.array_equal(dev_y.cpu().numpy().view(np.uint32), want.view(np.uint32))
