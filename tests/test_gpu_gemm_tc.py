@@ -343,3 +343,55 @@ def test_q6_k_prompt_kernel_at_even_addresses(be, port, offset):
     assert launches_of(be, call) == 4
     assert be.sync()
     assert np.array_equal(dev_y.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("t", [eb.Q8_0, eb.Q4_0])
+def test_q8_0_and_q4_0_prompt_columns_in_turns(monkeypatch, t):
+    """More columns than the workspace holds (9088): layout and product once per turn.  Columns at the turns' and tiles' ends and
+    between them equal those of the mma.sync kernel."""
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("EMELB_ACT_MELEMS", "40")
+    b = eb.Backend(0)
+    try:
+        k, m, n = 4096, 130, 10001
+        w = torch.from_numpy(synth.random_blocks(t, 9, m, k)).cuda()
+        x = torch.randn((k, n), device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+        at = torch.tensor([0, 1, 63, 64, 4000, 4001, 9023, 9086, 9087, 9088, 9089, 9151, 9152, 9900, 9983, 9984, 9999, 10000], device="cuda")
+        some = x[:, at].contiguous()
+        y, want = torch.zeros((m, n), device="cuda"), torch.zeros((m, len(at)), device="cuda")
+        torch.cuda.synchronize()
+
+        def call():
+            assert b.mul_mat(eb.mul_mat_op(w, t, k, m, x, n, y)), b.last_error
+        assert launches_of(b, call) == 5      # quantizer, and two turns
+        assert launches_of(b, lambda: b.mul_mat(eb.mul_mat_op(w, t, k, m, some, len(at), want))) == 2
+        assert b.sync()
+        assert torch.equal(y[:, at].contiguous().view(torch.int32), want.view(torch.int32)) and bool(want.any())
+    finally:
+        b.close()
+
+
+def test_q6_k_prompt_columns_and_rows_in_turns(monkeypatch):
+    """Columns that fill the workspace but for one tile row of unpacked weights: three turns of rows, then the other columns with
+    all rows at once.  Columns at the turns' and tiles' ends equal those of the kernels for few columns."""
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("EMELB_ACT_MELEMS", "72")
+    b = eb.Backend(0)
+    try:
+        k, m = 256, 300
+        n = (72 << 20) // k - 5               # 268928 columns and 25979
+        w = torch.from_numpy(synth.random_blocks(eb.Q6_K, 9, m, k)).cuda()
+        x = torch.randn((k, n), device="cuda", generator=torch.Generator("cuda").manual_seed(4))
+        at = torch.tensor([0, 63, 64, 127, 128, 100000, 268863, 268927, 268928, 268929, 269055, 269056, n - 2, n - 1], device="cuda")
+        some = x[:, at].contiguous()
+        y, want = torch.zeros((m, n), device="cuda"), torch.zeros((m, len(at)), device="cuda")
+        torch.cuda.synchronize()
+
+        def call():
+            assert b.mul_mat(eb.mul_mat_op(w, eb.Q6_K, k, m, x, n, y)), b.last_error
+        assert launches_of(b, call) == 1 + (1 + 2 * 3) + (1 + 2)      # quantizer; layout, and slabs and product of each turn of rows
+        assert b.mul_mat(eb.mul_mat_op(w, eb.Q6_K, k, m, some, len(at), want)), b.last_error
+        assert b.sync()
+        assert torch.equal(y[:, at].contiguous().view(torch.int32), want.view(torch.int32)) and bool(want.any())
+    finally:
+        b.close()
