@@ -34,8 +34,8 @@
 // call: 4096 x 11008 by 77 columns 66.3 -> 60.2 (a call by itself; one behind the other 105 -> 93), 14336 x
 // 11008 by 200 414 -> 363, 11008 x 4096 by 77 82 -> 74, 14336 x 2816 by 16 35.5 -> 31.3.
 // Dispatch: K and rows that the streaming kernels and gemm_q6k_mma.cu do not take (their copies need rows of a multiple
-// of 16 bytes, K % 2048 == 0).  Where both work, many columns are about equal (14336 x 4096 by 2048 columns 944 + 10
-// against 1047 us, 4096 x 14336 by 333: 273 + 7 against 247) and few are faster there (4096 x 14336 by 32: 124 + 3
+// of 16 bytes, K % 2048 == 0), up to the columns where gemm_q6k_wide.cu, which unpacks the blocks once for all column tiles,
+// is the cheaper one (its line is there).  Rows that both take are faster there with few columns (4096 x 14336 by 32: 124 + 3
 // against 99; by 8 127 against the mat-vec kernels' 60, by 5 127 against 49), so those kernels keep their sizes.
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -24,8 +24,8 @@
 // Registers are split by setmaxnreg: 896 threads x 72 at launch = 512 x 64 + 256 x 104 + 128 x 40.
 // Every mbarrier wait is bounded; on a timeout the CTA raises the status word, lets its copies land and frees its TMEM.
 //
-// What bounds it: the chain through one operand buffer, MMAs of either part (2,090 cycles a turn, both) -> expansion -> MMAs, 3,600
-// cycles a turn.  Measured, B200, 14336 x 4096 by 1900 columns: 377 us a call on planes (layout 12, slabs 18, product 340:
+// What bounds it: the chain through one operand buffer, MMAs of either part (2,050 cycles a turn, both) -> expansion -> MMAs, 3,370
+// cycles a turn (14336 x 4096 by 512 columns: tensor pipe 61 %, issue slots 52 %).  Measured, B200, 14336 x 4096 by 1900 columns: 377 us a call on planes (layout 12, slabs 18, product 340:
 // 656 TFLOP/s), mma.sync kernel 977; 4096 x 14336: 430, 972.  One warp for all MMAs took 541 (its waits stood in the way of
 // its instructions), two with the loop over quarters rolled 428, four 384.  The slabs' loads all in flight: 33 -> 18 us.
 #include <cuda_runtime.h>

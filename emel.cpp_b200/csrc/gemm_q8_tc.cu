@@ -20,9 +20,10 @@
 // Registers are split by setmaxnreg: 896 threads x 72 at launch = 256 x 96 + 512 x 64 + 128 x 48.
 // Every mbarrier wait is bounded; on a timeout the CTA raises the status word, lets its copies land and frees its TMEM.
 //
-// What bounds it: the round of an accumulator, MMAs -> epilogue -> MMAs, about 350 cycles a block with three on their way.
-// Measured, B200, us a call, mma.sync kernel and here: Q8_0 5632 x 5632 by 1024 columns 297 -> 214, 2048 x 5632 by 333 79 -> 56; Q4_0 257
-// -> 214, 68 -> 56.  With the product of the scales on the CUDA cores (three packed operations, the columns' scales from
+// What bounds it: instruction issue, 77 % of the slots (1,270 warp instructions and 416 cycles a block of a tile, MMAs 96), behind
+// it the round of an accumulator, MMAs -> epilogue -> MMAs, with three on their way.
+// Measured, B200, us a call on planes, mma.sync kernel and here: Q8_0 5632 x 5632 by 1024 columns 296 -> 216, 2048 x 5632 by 333 79 -> 56;
+// Q4_0 255 -> 215, 69 -> 56.  With the product of the scales on the CUDA cores (three packed operations, the columns' scales from
 // shared memory, whose 16-byte loads took more than half of the time) 248 and 62.
 #include <cuda.h>
 #include <cudaTypedefs.h>

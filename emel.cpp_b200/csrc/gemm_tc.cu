@@ -35,11 +35,11 @@
 // Registers are split by setmaxnreg: 640 threads x 96 at launch = 256 x 80 + 256 x 136 + 128 x 48.
 // Every mbarrier wait is bounded; on a timeout the CTA raises the status word, lets its copies land and frees its TMEM.
 //
-// What bounds it: instruction issue, 60 % of the slots with some eight cycles between two instructions of a warp.  Per
-// 128 x 128 x 256: 6,600 warp instructions (1,536 packed float ones, 1,150 for the expansion), of 2,600 cycles the MMAs take
+// What bounds it: instruction issue, 61 % of the slots with some eight cycles between two instructions of a warp.  Per
+// 128 x 128 x 256: 6,700 warp instructions (1,536 packed float ones, 1,150 for the expansion), of 2,760 cycles the MMAs take
 // 1,090.  Measured, B200, 14336 x 4096 by 2048 columns: pre-passes and product 352 us, product alone 333 (683 and 722
 // TFLOP/s); the int8 kernel before it (two operands of scale pieces, sums of mins on mma.sync) 439.  Whole calls on planes,
-// before and now: 14336 x 4096 by 32 columns 47.7 -> 30.5, by 128 48.4 -> 44.6, by 512 159 -> 118; 4096 x 14336 by 32 134 -> 78,
+// before and now: 14336 x 4096 by 32 columns 47.7 -> 30.5, by 128 48.4 -> 39.9, by 512 159 -> 118; 4096 x 14336 by 32 134 -> 78,
 // by 333 136 -> 104, by 1900 517 -> 354; 1024 x 4096 by 333 47.6 -> 31.4.  What gave it: TMEM loads of whole lanes (32x32b, half
 // a cycle a register against two of 16x256b: 16 % of the product without its arithmetic), roles in few instructions (the
 // producers' loop not unrolled 374 -> 349), the table (233 -> 188 million instructions), the second MMA warp (a call, quantizer

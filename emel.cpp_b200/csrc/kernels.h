@@ -123,7 +123,7 @@ cudaError_t launch_gemv_odd(int type, const GemvArgs& a, int ncols, int sm_count
 // whether launch_gemv (without argmax) hands this product to the tcgen05 kernel
 bool gemv_takes_tensor_core(int type, const GemvArgs& a, int ncols);
 
-// gemm_q8_mma.cu: 32 and more columns of Q8_0 / Q4_0 weights (mma.sync int8, one block per instruction)
+// gemm_q8_mma.cu: three and more columns of Q8_0 / Q4_0 weights, up to gemm_q8_tc.cu's (mma.sync int8, one block per instruction)
 bool gemm_q8_mma_supported(int type, const GemvArgs& a, int ncols);
 cudaError_t launch_gemm_q8_mma(int type, const GemvArgs& a, int ncols, int sm_count, cudaStream_t st);
 

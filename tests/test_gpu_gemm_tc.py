@@ -78,8 +78,8 @@ def one_sided(k, n):
 @pytest.mark.parametrize("m,n", [(136, 32), (300, 33), (2400, 128), (14300, 130), (12700, 131), (2500, 1154)])
 @pytest.mark.parametrize("extreme", [False, True])
 def test_q4_k_tiles_of_every_width(be, port, m, n, extreme):
-    """Tiles of 32, 64 (2400 rows: one wave) and 128 columns (the last three: fewer waves), whole and ragged, with and without
-    8-byte rows of results."""
+    """Tiles of 32 and, the last three, 128 columns, whole and ragged, with and without 16-byte rows of results.  (64: see
+    test_q4_k_short_sums; 128 with a table of the rows: test_q4_k_columns_in_turns and the benchmarked shapes.)"""
     k = 512
     w = extreme_blocks(eb.Q4_K, m, k) if extreme else synth.random_blocks(eb.Q4_K, m + n, m, k)
     x = one_sided(k, n) if extreme else synth.activations_f32(m * n, k, n).reshape(k, n)
@@ -277,10 +277,11 @@ def test_q8_0_and_q4_0_prompts_largest_sums(be, port, t):
     check(be, port, t, b.reshape(-1), k, m, one_sided(k, n), n)
 
 
-@pytest.mark.parametrize("k,m,n", [(256, 3100, 513), (512, 4100, 515), (768, 6500, 162), (1024, 4096, 333), (1024, 14300, 97), (2048, 5700, 130)])
+@pytest.mark.parametrize("k,m,n", [(256, 3100, 513), (512, 4100, 515), (768, 6500, 162), (1024, 4096, 333), (1024, 14300, 97), (2048, 5700, 130), (512, 2500, 250), (768, 14300, 63)])
 @pytest.mark.parametrize("extreme", [False, True])
 def test_q4_k_short_sums(be, port, k, m, n, extreme):
-    """Tiles of 64 (K = 256) and 128 columns without a table of the rows: two launches behind the quantizer.  Odd and even strides."""
+    """Tiles of 128 and, the last three, 64 columns without a table of the rows: two launches behind the quantizer.  Odd and even
+    strides."""
     w = extreme_blocks(eb.Q4_K, m, k) if extreme else synth.random_blocks(eb.Q4_K, m + n, m, k)
     x = one_sided(k, n) if extreme else synth.activations_f32(m * n, k, n).reshape(k, n)
     assert launches_of(be, lambda: check(be, port, eb.Q4_K, w, k, m, x, n)) == 3
