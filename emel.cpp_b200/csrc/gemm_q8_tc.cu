@@ -423,12 +423,15 @@ cudaError_t launch_product(const GemmArgs& g, const CUtensorMap& wmap, int sm_co
 // here: 2048 x 2048 by 333 columns 32 / 31, 5632 x 2048 by 64 23 / 26, by 333 54 / 52, by 1024 115 / 91; 2048 x 5632 by 333 79 / 56,
 // 5632 x 5632 by 64 56 / 50.  Where 64 x 64 tiles leave half of the SMs idle that kernel takes narrow ones (2048 x 5632 by 64
 // 29 / 50), so those stay there; and Q4_0, half the bytes, needs longer sums or more tiles (1024 x 4096 by 333 41.8 / 43.6, 4096 x
-// 4096 by 128 37.6 / 38.9; 14336 x 4096 by 64 49.9 / 39.7, 2048 x 5632 by 333 68.5 / 55.7)
+// 4096 by 128 37.6 / 38.9; 14336 x 4096 by 64 49.9 / 39.7, 2048 x 5632 by 333 68.5 / 55.7).  A thread stores a row's columns, which
+// without 16-byte pieces takes a tenth more (5632 x 2048 by 1900 171, by 1901 211): for Q4_0 and short sums that is the
+// advantage and more (2750 x 2048 by 1440 95.4 / 92.0, by 1441 97.4 / 104.4, 4096 x 3072 by 1441 168.8 / 166.7)
 bool gemm_q8_tc_supported(int type, const GemvArgs& a, int ncols, int sm_count) {
   const int64_t columns = (ncols + TN - 1) / TN, tiles = (a.M + BM - 1) / BM * columns;
   if (2 * ((a.M + 63) / 64) * columns <= sm_count) return false;
   if (a.K < 4096 && (a.K < 2048 || tiles < 2 * sm_count)) return false;
   if (type == T_Q4_0 && a.K < 5120 && 3 * tiles < 2 * sm_count) return false;
+  if (type == T_Q4_0 && a.K < 3072 && ((a.ldy | a.col0 | (int64_t)(reinterpret_cast<uintptr_t>(a.y) >> 2)) & 3) != 0) return false;
   if ((type != T_Q8_0 && type != T_Q4_0) || ncols < kGemmQ8TcMinCols || a.K % kTurnK != 0 || !a.tc_ws) return false;
   if (a.residual || a.W2 || a.W3 || a.pro_x || a.rope_cos || a.join_in || a.join_out) return false;
   return reinterpret_cast<uintptr_t>(a.W) % 16 == 0 && a.row_bytes % 16 == 0 && a.row_bytes < (1 << 27) && reinterpret_cast<uintptr_t>(a.act.qs) % 16 == 0 &&

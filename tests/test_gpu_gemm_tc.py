@@ -396,3 +396,13 @@ def test_q6_k_prompt_columns_and_rows_in_turns(monkeypatch):
         assert torch.equal(y[:, at].contiguous().view(torch.int32), want.view(torch.int32)) and bool(want.any())
     finally:
         b.close()
+
+
+@pytest.mark.parametrize("t,k,n,launches", [(eb.Q8_0, 2304, 901, 3), (eb.Q4_0, 2304, 901, 2), (eb.Q4_0, 2304, 902, 2), (eb.Q4_0, 2304, 904, 3),
+                                            (eb.Q4_0, 3072, 901, 3)])
+def test_q8_0_and_q4_0_prompts_of_other_strides(be, port, t, k, n, launches):
+    """Rows of results that are no multiple of 16 bytes: short Q4_0 sums stay on mma.sync."""
+    m = 2500
+    w = synth.random_blocks(t, m + n, m, k)
+    x = synth.activations_f32(m * n, k, n).reshape(k, n)
+    assert launches_of(be, lambda: check(be, port, t, w, k, m, x, n)) == launches
