@@ -18,7 +18,8 @@
 // (about 290 cycles beside the MMAs' own, whether addresses are constants of an unrolled loop or not, hence two slabs of K a
 // stage where shared memory has room for enough of these).
 //
-// Short sums over few tiles run on single CTAs (gemm_bf16_one_kernel below): a cluster's start costs 1 to 2 us more than a CTA's.
+// Short sums over few tiles run on single CTAs (gemm_bf16_one_kernel below), because a cluster's start costs 1 to 2 us more than a
+// CTA's, and so do sizes that leave most pairs idle in a last turn, but not the SMs (one_cta).
 // Every wait is bounded; when one runs out the CTA, or both, stop, let the copies and MMAs in flight end, raise the status word and free
 // their TMEM.
 #include <cuda.h>
@@ -592,24 +593,36 @@ int one_rows(const GemmParams& p, int sm_count) {
   return 5 * one_tiles(p, 256) >= 6 * sm_count ? 256 : 128;
 }
 
+int64_t tiles_of(const GemmParams& p, int bn) { return (int64_t)((p.M + 2 * kBM - 1) / (2 * kBM)) * ((p.rows + bn - 1) / bn); }
+
+// Turns x time a turn of one matrix.  Weights: us a turn of an SM pair at K = 2048 / 4096 / 8192 / 14336: 32 rows 10.6 / 16.6 / 26.8 / 42, 128 rows
+// 12.6 / 18.6 / 29 / 48, 256 rows 18.7 / 27 / 45 / 72.  (64 rows cost within 3 % of 128.)
+template <int BN>
+int64_t turns_cost(const GemmParams& p, int pairs) {
+  return (tiles_of(p, BN) + pairs - 1) / pairs * (BN == 32 ? 20 : BN == 128 ? 23 : 36);
+}
+int64_t pairs_cost(const GemmParams& p, int pairs) { return std::min({turns_cost<32>(p, pairs), turns_cost<128>(p, pairs), turns_cost<256>(p, pairs)}); }
+
 // Single CTAs or pairs, us there and here, one launch behind the other in a graph.
 // K to 256, to four tiles an SM: 4096 x 256 by 8 rows 3.5 / 4.5, by 200 4.5 / 6.4, by 2048 9.8 / 12.3, 136 x 136 by 100 4.5 / 5.2; beyond it the pairs' rate
 // wins (8192 x 256 by 1500 18.3 / 17.1).  K to 512 likewise (8192 x 512 by 8 5.3 / 5.8, by 128 6.2 / 7.6, by 333 8.8 / 10.0, by 1000 13.2 / 13.9, by 1500 23.2 /
 // 18.5), but with more than 32 rows in tiles for less than half of the SMs pairs are as fast or faster: 2048 x 512 by 100 5.3 / 5.0, by 333 5.4 / 6.7.
-// K to 1024, tiles for two thirds of the SMs to two an SM: 8192 x 1024 by 100 9.0 / 9.5, by 300 12.2 / 12.4, 2048 x 1024 by 1500 11.2 / 11.9; else 2048 x 1024 by 100
-// 8.3 / 6.7, 8192 x 1024 by 700 18.9 / 16.2.
+// K to 1024, tiles for half of the SMs to two an SM: 8192 x 1024 by 100 9.0 / 9.5, by 300 12.2 / 12.4, 2048 x 1024 by 300 8.3 / 8.8, by 1500 11.2 / 11.9; else 2048 x
+// 1024 by 100 8.3 / 6.7, 8192 x 1024 by 700 18.9 / 16.2.
 // Up to 64 rows of a matrix with one to two tiles an SM, which leaves most pairs idle in a last turn: 20480 x 2048 by 8 17.5 / 19.9, 32000 x 2048 by 64
-// 24.1 / 25.4, 24576 x 4096 by 64 39.4 / 42.2; 32000 x 4096 by 8 45.5 / 44.4, 14336 x 2048 by 32 13.8 / 13.2.
+// 24.1 / 25.4, 24576 x 4096 by 64 39.4 / 42.2, 23736 x 9320 by 6 76.6 / 88.9; 32000 x 4096 by 8 45.5 / 44.4, 14336 x 2048 by 32 13.8 / 13.2.
+// More rows where an odd number of 128-feature tiles fills the SMs, but half of it, rounded up, not the pairs: 6256 x 8720 by 374 39.2 / 48.7, 6256 x 9616 by 1523
+// 124 / 140.
 // Two matrices and up to 16 rows: 512 x 2 x 256 by 16 5.1 / 5.7, 8192 x 2 x 2048 by 8 17.0 / 17.4; 14336 x 2 x 4096 by 8 41.7 / 41.9
 bool one_cta(const GemmParams& p, bool glu, int sm_count) {
   if (glu) return p.rows <= 16 && p.K <= 2048;
   const int64_t tiles = one_tiles(p, std::min(one_rows(p, sm_count), 128));
   if (p.K <= 512) return tiles <= 4 * sm_count && (p.K <= 256 || p.rows <= 32 || 2 * tiles > sm_count);
-  if (p.K <= 1024) return 3 * tiles > 2 * sm_count && tiles <= 2 * sm_count;
-  return p.rows <= 64 && tiles > sm_count && (p.K <= 2048 ? tiles <= 2 * sm_count : p.K <= 4096 && 2 * tiles <= 3 * sm_count);
+  if (p.K <= 1024) return 2 * tiles > sm_count && tiles <= 2 * sm_count;
+  if (p.rows <= 64) return tiles > sm_count && 2 * tiles <= (p.K <= 2048 ? 4 : 3) * sm_count;
+  if (one_rows(p, sm_count) == 256) return 42 * ((one_tiles(p, 256) + sm_count - 1) / sm_count) < pairs_cost(p, std::max(sm_count / 2, 1));
+  return tiles <= sm_count && 30 < pairs_cost(p, std::max(sm_count / 2, 1));
 }
-
-int64_t tiles_of(const GemmParams& p, int bn) { return (int64_t)((p.M + 2 * kBM - 1) / (2 * kBM)) * ((p.rows + bn - 1) / bn); }
 
 template <int BN, bool GLU, int SL>
 cudaError_t launch_tiles(const TmaMap& wmap, const XMaps& x, const GemmParams& p, int pairs, cudaStream_t st) {
@@ -663,18 +676,16 @@ cudaError_t launch_gemm_bf16(const LinearArgs& a, const TmaMap& wmap, const XMap
     if (bn == 64) return launch_one<64, false>(wmap, x, p, sm_count, st);
     return bn == 128 ? launch_one<128, false>(wmap, x, p, sm_count, st) : launch_one_stages<256, false, false>(wmap, x, p, st);
   }
-  // The width with the least turns x time a turn.  Weights: us a turn of an SM pair at K = 2048 / 4096 / 8192 / 14336:
-  // 32 rows 10.6 / 16.6 / 26.8 / 42, 128 rows 12.6 / 18.6 / 29 / 48, 256 rows 18.7 / 27 / 45 / 72; two matrices at K = 2048: 32 rows 14.6, 64
-  // rows 18.7, 128 rows 22.  (64 rows of one matrix cost within 3 % of 128.)
+  // the width with the least turns x time a turn: us a turn of two matrices at K = 2048 32 rows 14.6, 64 rows 18.7, 128 rows 22
   const int pairs = std::max(sm_count / 2, 1);
-  const auto cost = [&](int bn, int weight) { return (tiles_of(p, bn) + pairs - 1) / pairs * weight; };
   if (glu) {
+    const auto cost = [&](int bn, int weight) { return (tiles_of(p, bn) + pairs - 1) / pairs * weight; };
     const int64_t c32 = cost(32, 7), c64 = cost(64, 9), c128 = cost(128, 11);
     if (c32 <= c64 && c32 <= c128) return launch_tiles<32, true, 2>(wmap, x, p, pairs, st);
     if (c64 < c128) return launch_tiles<64, true, 1>(wmap, x, p, pairs, st);
     return launch_tiles<128, true, 1>(wmap, x, p, pairs, st);
   }
-  const int64_t c32 = cost(32, 20), c128 = cost(128, 23), c256 = cost(256, 36);
+  const int64_t c32 = turns_cost<32>(p, pairs), c128 = turns_cost<128>(p, pairs), c256 = turns_cost<256>(p, pairs);
   if (c32 <= c128 && c32 <= c256) return launch_tiles<32, false, 2>(wmap, x, p, pairs, st);
   if (c128 < c256) return launch_tiles<128, false, 2>(wmap, x, p, pairs, st);
   return launch_tiles<256, false, 1>(wmap, x, p, pairs, st);

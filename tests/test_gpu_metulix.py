@@ -420,3 +420,18 @@ def test_products_of_every_tile_width(be, ragged, n):
     got = s.prefill_logits(ragged.tokens[:n], 0, range(n))
     assert_close(mm.row_errors(got, ragged.logits[:n]), False, n)
     s.close()
+
+
+@pytest.mark.parametrize("width,ff,vocab,n", [
+    (136, 1100, 2531, 2), (136, 1100, 2531, 17), (136, 1100, 2531, 140), (136, 1100, 2531, 700),      # K to 256; gate and up of up to 16 rows
+    (520, 2546, 2531, 16), (520, 2546, 2531, 33), (520, 2546, 9000, 40), (520, 2546, 2531, 1400),     # K to 1024
+    (1032, 72, 20000, 3), (1032, 72, 20000, 18), (1032, 72, 20000, 40),                               # one to two tiles an SM by up to 64 rows
+    (6272, 1032, 101, 300),                                                                           # 147 tiles of 128 features, 75 of 256
+])
+def test_products_of_single_ctas(be, tmp_path, width, ff, vocab, n):
+    """Sizes at which a cluster's start or idle pairs of SMs would cost more than the pairs give."""
+    c = Case(mm.model(width, vocab, [mm.attention(2, 1, 32, 32, 0.5, conv=3, rot=(16, 1000.0), window=50, keep=2, ff=ff)]), tmp_path, n, 41)
+    s = c.session(be, False, n_ctx=1536)
+    want = range(max(0, n - 64), n)
+    assert_close(mm.row_errors(s.prefill_logits(c.tokens, 0, want), c.logits[want.start:]), False, width, n)
+    s.close()
